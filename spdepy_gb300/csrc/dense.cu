@@ -662,277 +662,245 @@ __device__ __forceinline__ float df_rsqrt(DF d) {
   return fmaf(0.5f * y, e, y);
 }
 
-// Blocked double-float factorisation of one diagonal block A = L L^T
-// (w <= 64), in 16-column sub-blocks s with the trailing Schur updates written
-// as A_ik -= (a_ic / d_c) a_kc, so that the pivots d_c and the columns a_ic
-// (at the time column c is eliminated) stay in double-float and L_ic =
-// a_ic / sqrt(d_c) is rounded to FP32 once, at the end.  Per sub-block:
-//   (1) warp 0 eliminates the 16 x 16 diagonal sub-block column by column
-//       (warp-synchronous, each lane holding up to five of its 136 entries);
-//   (2) four threads per row below it eliminate that row's 16 columns and
-//       record S_ic = a_ic / d_c;
-//   (3) the whole CTA applies the rank-16 update S a^T to the trailing lower
-//       triangle, 2 x 2 entries per thread.
-// Then L^-1 (FP32) by sub-blocks: the four 16 x 16 diagonal inverses (one warp
-// each, one lane per column), then the off-diagonal blocks by distance from the
-// diagonal, X_ij = -X_ii (sum_{i > k >= j} L_ik X_kj).  About 20 CTA barriers
-// in all instead of one per column.
+// Double-float factorisation of one diagonal block A = L L^T (w <= 64) and its
+// inverse, one CTA per block.
+//
+// The elimination is written A_ik -= (a_ic / d_c) a_kc, so that the pivots d_c
+// and the columns a_ic (at the time column c is eliminated) stay in double-float
+// and L_ic = a_ic / sqrt(d_c) is rounded to FP32 once, at the end.  Every entry
+// takes its updates in the order of c, so the result does not depend on how the
+// work is split over threads.
+//
+// Bound: latency.  The blocks of a front's top levels are a serial chain with
+// one block per launch, so the kernel is built around the chain from pivot to
+// pivot.  It goes by 16-column panels.  A panel is eliminated by one warp per 16
+// rows below its diagonal block: lanes 0-15 hold the diagonal block's rows (the
+// same in every warp), lanes 16-31 the warp's own rows, one row per lane in
+// registers, so that pivots and multipliers travel by shuffle and no warp waits for
+// another inside a panel.  The trailing rank-16 update is spread over all 256
+// threads, each holding the entries (ty + 16 m, tx + 16 n), n <= m, in registers.
+// Then L^-1 (FP32) by 16-column sub-blocks: the four diagonal inverses (a warp
+// each, one lane per column, right-looking so that the partial sums of all rows
+// advance together) beside the pivot logarithms on a fifth warp, then the
+// off-diagonal blocks by distance from the diagonal, X_ij = -X_ii (sum_{i > k >= j}
+// L_ik X_kj), the factor's entries read four at a time.
+// Measured (CUDA events, 64 x 64 blocks): one block 32 us (67 for the same sweep with
+// the columns exchanged through shared memory and the inverse by rows), 608
+// blocks 78 us (102), 1,280 blocks 124 us (239).  Three CTAs per SM: at two the
+// panel has more registers (30 us for one block) but 1,280 blocks take 143.
 constexpr int kDfSub = 16;
+constexpr int kDfLd = kMaxNbk + 4;          // row stride of L and L^-1 in shared memory (16-byte rows)
+constexpr int kDfPan = kDfSub + 2;          // row stride (double-floats) of a panel in shared memory
 
-__device__ __forceinline__ int tri_row(int q) {  // largest r with r (r + 1) / 2 <= q
-  int r = int((sqrtf(8.0f * float(q) + 1.0f) - 1.0f) * 0.5f);
-  while (r * (r + 1) / 2 > q) --r;
-  while ((r + 1) * (r + 2) / 2 <= q) ++r;
-  return r;
-}
+template <int N>
+struct IntC {
+  static constexpr int value = N;
+};
 
-__global__ void __launch_bounds__(256) potrf_df_kernel(const DiagTask* __restrict__ tasks, float* __restrict__ L,
-                                                       float* __restrict__ dinv, double* __restrict__ logpiv,
-                                                       int* __restrict__ err) {
-  // Ah/Al: the double-float working matrix (lower triangle); after the
-  // factorisation Al holds L (FP32, zero above the diagonal) and Ah holds L^-1.
-  __shared__ float Ah[kMaxNbk][kMaxNbk + 1], Al[kMaxNbk][kMaxNbk + 1];
-  // S_ic of the current sub-block (double-float); later the inverse's products
-  __shared__ float Sh[kMaxNbk][kDfSub + 1], Sl[kMaxNbk][kDfSub + 1];
+__global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __restrict__ tasks, float* __restrict__ L,
+                                                          float* __restrict__ dinv, double* __restrict__ logpiv,
+                                                          int* __restrict__ err) {
+  // L and L^-1; before that, two panel buffers and the panel's multipliers
+  __shared__ __align__(16) float smem[2 * kMaxNbk * kDfLd];
+  __shared__ float Tb[3 * kDfSub * kDfSub];
   __shared__ float dph[kMaxNbk], dpl[kMaxNbk], rsq[kMaxNbk];
-  __shared__ float dvh[kDfSub], dvl[kDfSub];
   __shared__ int bad;
+  static_assert(2 * kMaxNbk * kDfLd >= 3 * 2 * kMaxNbk * kDfPan, "panel buffers fit");
+  float (*Ls)[kDfLd] = reinterpret_cast<float (*)[kDfLd]>(smem);
+  float (*Xs)[kDfLd] = Ls + kMaxNbk;
+  float2 (*pan0)[kDfPan] = reinterpret_cast<float2 (*)[kDfPan]>(smem);
+  float2 (*mul)[kDfPan] = pan0 + 2 * kMaxNbk;  // S_ic = a_ic / d_c
   const DiagTask tk = tasks[blockIdx.x];
   const int w = tk.w;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ty = tid >> 4, tx = tid & 15;
   float* blk = L + tk.a;
-  for (int e = tid; e < w * w; e += 256) {
-    const int i = e / w, k = e - i * w;
-    if (k <= i) {
-      Ah[i][k] = blk[int64_t(i) * tk.lda + k];
-      Al[i][k] = 0.0f;
+  DF r[4][4];                               // n <= m used
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int n = 0; n <= m; ++n) {
+      const int i = ty + 16 * m, k = tx + 16 * n;
+      r[m][n] = DF{(k <= i && i < w) ? blk[int64_t(i) * tk.lda + k] : 0.0f, 0.0f};
     }
-  }
   if (tid == 0) bad = 0;
-  // entries of the 16 x 16 lower triangle held by this lane in (1): e = lane + 32 t
-  int eii[5], ekk[5];
+  for (int jb = 0; 16 * jb < w; ++jb) {
+    float2 (*pan)[kDfPan] = pan0 + (jb & 1) * kMaxNbk;
+    const int c0 = 16 * jb, cw = min(kDfSub, w - c0);
+    // block column jb to shared memory (the register indices are compile-time constants)
 #pragma unroll
-  for (int t = 0; t < 5; ++t) {
-    const int e = lane + 32 * t;
-    const int r = tri_row(e < 136 ? e : 0);
-    eii[t] = e < 136 ? r : kDfSub;  // kDfSub: no entry
-    ekk[t] = e < 136 ? e - r * (r + 1) / 2 : 0;
-  }
-  __syncthreads();
-  const int nsb = (w + kDfSub - 1) / kDfSub;
-  for (int sb = 0; sb < nsb; ++sb) {
-    const int c0 = sb * kDfSub, cw = min(kDfSub, w - c0);
-    // ---- (1) diagonal sub-block, warp 0; inactive entries are masked, not
-    // branched around, so that the five updates of a lane overlap
-    if (warp == 0) {
-      DF v[5];
+    for (int n = 0; n < 4; ++n)
+      if (n == jb) {
 #pragma unroll
-      for (int t = 0; t < 5; ++t)
-        v[t] = eii[t] < cw ? DF{Ah[c0 + eii[t]][c0 + ekk[t]], Al[c0 + eii[t]][c0 + ekk[t]]} : DF{0.0f, 0.0f};
-      for (int j = 0; j < cw; ++j) {
-        // publish column j (its entries are final from here on)
+        for (int m = n; m < 4; ++m) pan[ty + 16 * m][tx] = make_float2(r[m][n].hi, r[m][n].lo);
+      }
+    __syncthreads();
+    if (warp == 0 || c0 + 16 * (warp + 1) < w) {
+      const int row = lane < 16 ? c0 + lane : min(c0 + 16 * (warp + 1) + lane - 16, kMaxNbk - 1);
+      DF x[16];
 #pragma unroll
-        for (int t = 0; t < 5; ++t)
-          if (eii[t] < cw && ekk[t] == j) {
-            Ah[c0 + eii[t]][c0 + j] = v[t].hi;
-            Al[c0 + eii[t]][c0 + j] = v[t].lo;
-          }
-        __syncwarp();
-        DF d{Ah[c0 + j][c0 + j], Al[c0 + j][c0 + j]};
+      for (int k = 0; k < 16; ++k) {
+        const float2 v = pan[row][k];
+        x[k] = DF{v.x, v.y};
+      }
+      __syncwarp();
+      const bool own = lane >= 16 ? c0 + 16 * (warp + 1) < w : warp == 0;  // this lane's row is written by this warp
+      float piv_h = 1.0f, piv_l = 0.0f;
+      bool failed = false;
+      // columns >= cw are zero: their pivot counts as 1 and they change nothing
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        DF d{__shfl_sync(0xffffffffu, x[j].hi, j), __shfl_sync(0xffffffffu, x[j].lo, j)};
         const bool nonpos = !(d.hi > 0.0f) || !isfinite(d.hi);
         if (nonpos) d = DF{1.0f, 0.0f};
-        const DF dv = df_rcp(d);
-        if (lane == 0) {
-          if (nonpos) bad = 1;
-          dph[c0 + j] = d.hi;
-          dpl[c0 + j] = d.lo;
-          dvh[j] = dv.hi;
-          dvl[j] = dv.lo;
+        const DF sj = df_mul(x[j], df_rcp(d));
+        piv_h = lane == j ? d.hi : piv_h;
+        piv_l = lane == j ? d.lo : piv_l;
+        failed |= nonpos && j < cw;
+        if (own) {
+          pan[row][j] = make_float2(x[j].hi, x[j].lo);
+          mul[row][j] = make_float2(sj.hi, sj.lo);
         }
 #pragma unroll
-        for (int t = 0; t < 5; ++t) {
-          const bool act = eii[t] < cw && ekk[t] > j;
-          const int ri = c0 + (act ? eii[t] : j), rk = c0 + (act ? ekk[t] : j);  // (j, j) when masked
-          DF ci = df_mul(DF{Ah[ri][c0 + j], Al[ri][c0 + j]}, dv);
-          DF ck{Ah[rk][c0 + j], Al[rk][c0 + j]};
-          if (!act) ci = ck = DF{0.0f, 0.0f};
-          v[t] = df_fms(v[t], ci, ck);
+        for (int k = j + 1; k < 16; ++k) {
+          const DF a{__shfl_sync(0xffffffffu, x[j].hi, k), __shfl_sync(0xffffffffu, x[j].lo, k)};
+          x[k] = df_fms(x[k], sj, a);
         }
+      }
+      if (warp == 0 && lane < cw) {
+        dph[c0 + lane] = piv_h;
+        dpl[c0 + lane] = piv_l;
+        if (failed) bad = 1;
       }
     }
     __syncthreads();
-    const int b0 = c0 + cw, mt = w - b0;  // rows below the sub-block
-    if (mt <= 0) break;
-    // ---- (2) panel rows, four threads per row: thread q holds the row's
-    // entries in columns q, q + 4, q + 8, q + 12 of the sub-block; the owner of
-    // column j forms S_ij and passes it to the other three by shuffle
-    const unsigned pmask = __ballot_sync(0xffffffffu, tid < 4 * mt);
-    if (tid < 4 * mt) {
-      const int i = b0 + (tid >> 2), q = tid & 3;
-      DF x[4];
+    auto trailing = [&](auto block) {
+      constexpr int n = decltype(block)::value;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = q + 4 * u;
-        x[u] = c < cw ? DF{Ah[i][c0 + c], Al[i][c0 + c]} : DF{0.0f, 0.0f};
+      for (int m = n; m < 4; ++m) {  // the panel's final entries
+        const float2 v = pan[ty + 16 * m][tx];
+        r[m][n] = DF{v.x, v.y};
       }
-      for (int j = 0; j < cw; ++j) {
-        const int uj = j >> 2, qj = j & 3;
-        DF xj = x[0];
-        if (uj == 1) xj = x[1];
-        if (uj == 2) xj = x[2];
-        if (uj == 3) xj = x[3];
-        DF sj = df_mul(xj, DF{dvh[j], dvl[j]});
-        const int src = (lane & ~3) | qj;
-        sj.hi = __shfl_sync(pmask, sj.hi, src);
-        sj.lo = __shfl_sync(pmask, sj.lo, src);
-        if (q == qj) {
-          Sh[i][j] = sj.hi;
-          Sl[i][j] = sj.lo;
-          Ah[i][c0 + j] = xj.hi;
-          Al[i][c0 + j] = xj.lo;
-        }
+      if (c0 + 16 < w) {
+#pragma unroll 4
+        for (int c = 0; c < kDfSub; c += 2) {
+          float4 sv[4], av[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = q + 4 * u;
-          const bool act = c > j && c < cw;
-          const int r = c0 + (act ? c : j);  // (j, j) when masked
-          const DF nx = df_fms(x[u], sj, DF{Ah[r][c0 + j], Al[r][c0 + j]});
-          if (act) x[u] = nx;
-        }
-      }
-    }
-    __syncthreads();
-    // ---- (3) trailing update A_ik -= sum_c S_ic a_kc, 2 x 2 entries per thread
-    const int nb2 = (mt + 1) >> 1, nq = nb2 * (nb2 + 1) / 2;
-    for (int q = tid; q < nq; q += 256) {
-      const int bi = tri_row(q), bk = q - bi * (bi + 1) / 2;
-      const int i0 = b0 + 2 * bi, k0 = b0 + 2 * bk;
-      const bool i1ok = i0 + 1 < w, k1ok = k0 + 1 < w;
-      DF acc[2][2];
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int i = i0 + r, k = k0 + u;
-          const bool ok = (r == 0 || i1ok) && (u == 0 || k1ok) && k <= i;
-          acc[r][u] = ok ? DF{Ah[i][k], Al[i][k]} : DF{0.0f, 0.0f};
-        }
-      for (int c = 0; c < cw; ++c) {
-        const DF s0{Sh[i0][c], Sl[i0][c]};
-        const DF s1 = i1ok ? DF{Sh[i0 + 1][c], Sl[i0 + 1][c]} : DF{0.0f, 0.0f};
-        const DF a0{Ah[k0][c0 + c], Al[k0][c0 + c]};
-        const DF a1 = k1ok ? DF{Ah[k0 + 1][c0 + c], Al[k0 + 1][c0 + c]} : DF{0.0f, 0.0f};
-        acc[0][0] = df_fms(acc[0][0], s0, a0);
-        acc[1][0] = df_fms(acc[1][0], s1, a0);
-        acc[1][1] = df_fms(acc[1][1], s1, a1);
-        if (bi != bk) acc[0][1] = df_fms(acc[0][1], s0, a1);
-      }
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int i = i0 + r, k = k0 + u;
-          if ((r == 0 || i1ok) && (u == 0 || k1ok) && k <= i) {
-            Ah[i][k] = acc[r][u].hi;
-            Al[i][k] = acc[r][u].lo;
+          for (int m = n + 1; m < 4; ++m) {
+            sv[m] = *reinterpret_cast<const float4*>(&mul[ty + 16 * m][c]);
+            av[m] = *reinterpret_cast<const float4*>(&pan[tx + 16 * m][c]);
           }
+#pragma unroll
+          for (int m = n + 1; m < 4; ++m)
+#pragma unroll
+            for (int q = n + 1; q <= m; ++q) {
+              r[m][q] = df_fms(r[m][q], DF{sv[m].x, sv[m].y}, DF{av[q].x, av[q].y});
+              r[m][q] = df_fms(r[m][q], DF{sv[m].z, sv[m].w}, DF{av[q].z, av[q].w});
+            }
         }
+      }
+    };
+    switch (jb) {
+      case 0: trailing(IntC<0>{}); break;
+      case 1: trailing(IntC<1>{}); break;
+      case 2: trailing(IntC<2>{}); break;
+      default: trailing(IntC<3>{}); break;
     }
-    __syncthreads();
   }
-  // ---- L = a_ik / sqrt(d_k) (FP32) into Al and the block: thread (i, q)
-  // holds row i, columns 16 q .. 16 q + 15
+  __syncthreads();
   if (tid < w) rsq[tid] = df_rsqrt(DF{dph[tid], dpl[tid]});
   __syncthreads();
-  {
-    const int i = tid >> 2, kq = (tid & 3) * kDfSub;
-    float lv[kDfSub];
+  // L = a_ik / sqrt(d_k) (FP32), zero above the diagonal
 #pragma unroll
-    for (int u = 0; u < kDfSub; ++u) {
-      const int k = kq + u;
-      float v = 0.0f;
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int i = ty + 16 * m, k = tx + 16 * n;
       if (i < w && k < w) {
-        if (k < i) v = (Ah[i][k] + Al[i][k]) * rsq[k];
-        else if (k == i) v = 1.0f / rsq[k];
-      }
-      lv[u] = v;
-    }
-    __syncthreads();
-    if (i < w) {
-#pragma unroll
-      for (int u = 0; u < kDfSub; ++u) {
-        const int k = kq + u;
-        if (k < w) {
-          Al[i][k] = lv[u];
-          blk[int64_t(i) * tk.lda + k] = lv[u];
-        }
-      }
-    }
-  }
-  __syncthreads();
-  // ---- L^-1 into Ah: diagonal 16 x 16 inverses, warp s, lane = column
-  if (warp < nsb && lane < kDfSub) {
-    const int c0 = warp * kDfSub, cw = min(kDfSub, w - c0), c = lane;
-    if (c < cw) {
-      float x[kDfSub];
-#pragma unroll
-      for (int ii = 0; ii < kDfSub; ++ii) {
         float v = 0.0f;
-        if (ii == c) v = rsq[c0 + c];
-        else if (ii > c && ii < cw) {
-          float sum = 0.0f;
-#pragma unroll
-          for (int k = 0; k < ii; ++k) sum = fmaf(Al[c0 + ii][c0 + k], x[k], sum);
-          v = -sum * rsq[c0 + ii];
+        if (n <= m) {
+          if (k < i) v = (r[m][n].hi + r[m][n].lo) * rsq[k];
+          else if (k == i) v = 1.0f / rsq[k];
         }
-        x[ii] = v;
+        Ls[i][k] = v;
+        blk[int64_t(i) * tk.lda + k] = v;
       }
+    }
+  __syncthreads();
+  const int nsb = (w + kDfSub - 1) / kDfSub;
+  if (warp < nsb) {
+    // diagonal 16 x 16 inverse of sub-block `warp`, lane = column: x_ii = -(sum_{k < ii} L_(ii,k) x_k) / L_(ii,ii)
+    if (lane < kDfSub) {
+      const int c0 = warp * kDfSub, cw = min(kDfSub, w - c0), c = lane;
+      float sum[kDfSub];
 #pragma unroll
-      for (int ii = 0; ii < kDfSub; ++ii)
-        if (ii < cw) Ah[c0 + ii][c0 + c] = x[ii];
+      for (int ii = 0; ii < kDfSub; ++ii) sum[ii] = 0.0f;
+#pragma unroll
+      for (int k = 0; k < kDfSub; ++k) {
+        if (k >= cw) break;
+        float x = 0.0f;
+        if (k == c) x = rsq[c0 + k];
+        else if (k > c) x = -sum[k] * rsq[c0 + k];
+        Xs[c0 + k][c0 + c] = x;
+#pragma unroll
+        for (int ii = k + 1; ii < kDfSub; ++ii)
+          if (ii < cw) sum[ii] = fmaf(Ls[c0 + ii][c0 + k], x, sum[ii]);
+      }
+    }
+  } else if (warp == 7) {
+    double s = 0.0;
+    for (int j = lane; j < w; j += 32) s += 0.5 * log(double(dph[j]) + double(dpl[j]));
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      logpiv[blockIdx.x] = s;
+      if (bad) atomicCAS(err, -1, tk.front);
     }
   }
   __syncthreads();
   // off-diagonal blocks by distance dd: T = sum_k L_(bi,k) X_(k,bj), then X_(bi,bj) = -X_(bi,bi) T
-  float* Tb = &Sh[0][0];  // up to 3 x 256 products
-  for (int dd = 1; dd < nsb; ++dd) {
-    const int np = nsb - dd;
-    for (int e = tid; e < np * 256; e += 256) {
-      const int pidx = e >> 8, r = (e >> 4) & 15, c = e & 15;
-      const int bi = dd + pidx, bj = pidx;
-      const int i = bi * kDfSub + r;
-      float sum = 0.0f;
-      if (i < w)
-        for (int k = bj * kDfSub; k < bi * kDfSub; ++k) sum = fmaf(Al[i][k], Ah[k][bj * kDfSub + c], sum);
-      Tb[e] = sum;
-    }
-    __syncthreads();
-    for (int e = tid; e < np * 256; e += 256) {
-      const int pidx = e >> 8, r = (e >> 4) & 15, c = e & 15;
-      const int bi = dd + pidx, bj = pidx;
-      const int i = bi * kDfSub + r;
-      if (i < w) {
-        float sum = 0.0f;
-        for (int rr = 0; rr <= r; ++rr) sum = fmaf(Ah[i][bi * kDfSub + rr], Tb[(pidx << 8) + (rr << 4) + c], sum);
-        Ah[i][bj * kDfSub + c] = -sum;
+#pragma unroll
+  for (int dd = 1; dd < 4; ++dd) {
+    if (dd >= nsb) break;
+#pragma unroll
+    for (int pi = 0; pi < 4 - dd; ++pi) {
+      const int i = (dd + pi) * kDfSub + ty;  // rows >= w compute values that nothing reads
+      float s = 0.0f;
+#pragma unroll
+      for (int k4 = 4 * pi; k4 < 4 * (pi + dd); ++k4) {
+        const float4 l = *reinterpret_cast<const float4*>(&Ls[i][4 * k4]);
+        s = fmaf(l.x, Xs[4 * k4 + 0][pi * kDfSub + tx], s);
+        s = fmaf(l.y, Xs[4 * k4 + 1][pi * kDfSub + tx], s);
+        s = fmaf(l.z, Xs[4 * k4 + 2][pi * kDfSub + tx], s);
+        s = fmaf(l.w, Xs[4 * k4 + 3][pi * kDfSub + tx], s);
       }
+      Tb[(pi << 8) + tid] = s;
     }
     __syncthreads();
-  }
-  if (tid < 32) {
-    double sum = 0.0;
-    for (int j = tid; j < w; j += 32) sum += 0.5 * log(double(dph[j]) + double(dpl[j]));
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-    if (tid == 0) {
-      logpiv[blockIdx.x] = sum;
-      if (bad) atomicCAS(err, -1, tk.front);
+#pragma unroll
+    for (int pi = 0; pi < 4 - dd; ++pi) {
+      const int bi = dd + pi, i = bi * kDfSub + ty;
+      float s = 0.0f;
+#pragma unroll
+      for (int r4 = 0; r4 < kDfSub / 4; ++r4) {
+        const float4 xi = *reinterpret_cast<const float4*>(&Xs[i][bi * kDfSub + 4 * r4]);
+        const float xr[4] = {xi.x, xi.y, xi.z, xi.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float nx = fmaf(xr[e], Tb[(pi << 8) + ((4 * r4 + e) << 4) + tx], s);
+          if (4 * r4 + e <= ty) s = nx;
+        }
+      }
+      Xs[i][pi * kDfSub + tx] = -s;
     }
+    __syncthreads();
   }
   float* dvp = dinv + tk.dinv;
-  for (int e = tid; e < w * w; e += 256) {
-    const int i = e / w, c = e - i * w;
-    dvp[int64_t(i) * kMaxNbk + c] = c <= i ? Ah[i][c] : 0.0f;
-  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const int i = ty + 16 * m, c = tx + 16 * n;
+      if (i < w && c < w) dvp[int64_t(i) * kMaxNbk + c] = c <= i ? Xs[i][c] : 0.0f;
+    }
 }
 
 template <typename T>
