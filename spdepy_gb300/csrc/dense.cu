@@ -285,75 +285,126 @@ __global__ void __launch_bounds__(256) gemv_kernel(const GemmTask* __restrict__ 
 
 // ------------------------------------------------------ panel solve (FP32)
 // X = A Linv^T for one 64-column diagonal block: tasks with m <= 128 rows,
-// n <= 64 columns and k <= 64, both operands in row layout.  The CTA stages its
-// whole A tile and the block inverse in shared memory once (no K loop), then
-// each thread computes an 8 x 4 block of the output; A may alias C (in-place
-// panel solve): every read happens before the first write.
-constexpr int kPanelLdA = 129, kPanelLdB = 65;
-constexpr int kPanelSmem = (64 * kPanelLdA + 64 * kPanelLdB) * int(sizeof(float));
+// n <= 64 columns and k <= 64, both operands in row layout.  A CTA takes ROWS rows
+// of a task; it stages them and the block inverse in shared memory as they lie (no
+// K loop, one 16-byte load per four values where the rows are aligned), then
+// thread (ty, tx) computes the entries (ty + 16 r, tx + 16 c), reading both
+// operands four k values at a time without bank conflicts.  A may alias C
+// (in-place panel solve; the rows of a task's CTAs are their own): every read
+// happens before the first write.  Bound: latency, the launch being one of a
+// serial chain per 64 columns.
+constexpr int kPanelLd = 68;  // row stride of the staged tiles: 16-byte rows, 4 banks apart
+constexpr int panel_smem(int rows) { return (rows + 64) * kPanelLd * int(sizeof(float)); }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) panel64_kernel(const GemmTask* __restrict__ tasks, const float* Ab,
-                                                      const float* Bb, float* Cb) {
-  extern __shared__ float psm[];
-  float* As = psm;                     // As[k * kPanelLdA + i] = A(i, k)
-  float* Bs = psm + 64 * kPanelLdA;    // Bs[k * kPanelLdB + j] = B(j, k)
-  const GemmTask tk = tasks[blockIdx.x];
-  const float* A = Ab + tk.a;
-  const float* B = Bb + tk.b;
-  float* C = Cb + tk.c;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < 128 * 64; e += 256) {
-    const int i = e >> 6, k = e & 63;
-    As[k * kPanelLdA + i] = (i < tk.m && k < tk.k) ? A[int64_t(i) * tk.lda + k] : 0.f;
-  }
-  for (int e = tid; e < 64 * 64; e += 256) {
-    const int j = e >> 6, k = e & 63;
-    Bs[k * kPanelLdB + j] = (j < tk.n && k < tk.k) ? B[int64_t(j) * tk.ldb + k] : 0.f;
-  }
-  __syncthreads();
-  const int ty = tid >> 4, tx = tid & 15;  // rows 8 ty .. + 7, columns 4 tx .. + 3
-  float acc[8][4];
+// rows x 64 values of X (zero outside m x k) into shared memory, NT threads
+template <int ROWS>
+__device__ __forceinline__ void panel_stage(const float* X, int ldx, int m, int k, float* sh, int tid) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(X) & 15) == 0) && (ldx & 3) == 0;
+  float4 v[ROWS / 16];
 #pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
-  for (int kk = 0; kk < tk.k; ++kk) {
-    float a[8], b[4];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) a[r] = As[kk * kPanelLdA + ty * 8 + r];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) b[c] = Bs[kk * kPanelLdB + tx * 4 + c];
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
-  }
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int i = ty * 8 + r;
-    if (i >= tk.m) continue;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int j = tx * 4 + c;
-      if (j >= tk.n) continue;
-      float* dst = C + int64_t(i) * tk.ldc + j;
-      if (MODE == kSub) *dst -= acc[r][c];
-      else if (MODE == kStore) *dst = acc[r][c];
-      else if (MODE == kNegStore) *dst = -acc[r][c];
-      else *dst += acc[r][c];
+  for (int u = 0; u < ROWS / 16; ++u) {
+    const int i = (tid >> 4) + 16 * u, c = 4 * (tid & 15);
+    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < m) {
+      const float* x = X + int64_t(i) * ldx + c;
+      if (vec && c + 4 <= k) {
+        v[u] = *reinterpret_cast<const float4*>(x);
+      } else {
+        if (c + 0 < k) v[u].x = x[0];
+        if (c + 1 < k) v[u].y = x[1];
+        if (c + 2 < k) v[u].z = x[2];
+        if (c + 3 < k) v[u].w = x[3];
+      }
     }
   }
+#pragma unroll
+  for (int u = 0; u < ROWS / 16; ++u)
+    *reinterpret_cast<float4*>(sh + ((tid >> 4) + 16 * u) * kPanelLd + 4 * (tid & 15)) = v[u];
 }
 
-template <int MODE>
-static void panel64_launch(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st) {
+template <int MODE, int ROWS>
+__global__ void __launch_bounds__(256) panel64_kernel(const GemmTask* __restrict__ tasks, const float* Ab,
+                                                      const float* Bb, float* Cb) {
+  extern __shared__ __align__(16) float psm[];
+  constexpr int kSplit = 128 / ROWS, R = ROWS / 16;
+  float* As = psm;                     // As[i * kPanelLd + k] = A(i, k)
+  float* Bs = psm + ROWS * kPanelLd;   // Bs[j * kPanelLd + k] = B(j, k)
+  const GemmTask tk = tasks[blockIdx.x / kSplit];
+  const int row0 = int(blockIdx.x % kSplit) * ROWS, m = min(ROWS, tk.m - row0);
+  if (m <= 0) return;
+  float* C = Cb + tk.c + int64_t(row0) * tk.ldc;
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  panel_stage<ROWS>(Ab + tk.a + int64_t(row0) * tk.lda, tk.lda, m, tk.k, As, tid);
+  panel_stage<64>(Bb + tk.b, tk.ldb, tk.n, tk.k, Bs, tid);
+  float old[R][4];
+  if (MODE == kSub || MODE == kAdd) {  // in flight with the operands
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int i = ty + 16 * r, j = tx + 16 * c;
+        old[r][c] = (i < m && j < tk.n) ? C[int64_t(i) * tk.ldc + j] : 0.f;
+      }
+  }
+  __syncthreads();
+  float acc[R][4];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
+#pragma unroll 2
+  for (int kk = 0; kk < tk.k; kk += 4) {
+    float4 a[R], b[4];
+#pragma unroll
+    for (int r = 0; r < R; ++r) a[r] = *reinterpret_cast<const float4*>(As + (ty + 16 * r) * kPanelLd + kk);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(Bs + (tx + 16 * c) * kPanelLd + kk);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r].x, b[c].x, acc[r][c]);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r].y, b[c].y, acc[r][c]);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r].z, b[c].z, acc[r][c]);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r].w, b[c].w, acc[r][c]);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = ty + 16 * r, j = tx + 16 * c;
+      if (i >= m || j >= tk.n) continue;
+      float* dst = C + int64_t(i) * tk.ldc + j;
+      if (MODE == kSub) *dst = old[r][c] - acc[r][c];
+      else if (MODE == kStore) *dst = acc[r][c];
+      else if (MODE == kNegStore) *dst = -acc[r][c];
+      else *dst = old[r][c] + acc[r][c];
+    }
+}
+
+// Fewer rows per CTA while the launch leaves SMs idle: 32 rows up to 152 tasks, 64 up to 304.
+template <int MODE, int ROWS>
+static void panel64_rows(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st) {
   static const bool attr = [] {  // once, thread-safely (two pipelines launch from two host threads)
-    cudaFuncSetAttribute(panel64_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
+    cudaFuncSetAttribute(panel64_kernel<MODE, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem(ROWS));
     return true;
   }();
   (void)attr;
-  panel64_kernel<MODE><<<n, 256, kPanelSmem, st>>>(t, A, B, C);
+  panel64_kernel<MODE, ROWS><<<n * (128 / ROWS), 256, panel_smem(ROWS), st>>>(t, A, B, C);
+}
+template <int MODE>
+static void panel64_launch(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st) {
+  if (n <= 152) panel64_rows<MODE, 32>(t, n, A, B, C, st);
+  else if (n <= 304) panel64_rows<MODE, 64>(t, n, A, B, C, st);
+  else panel64_rows<MODE, 128>(t, n, A, B, C, st);
 }
 
 template <typename T, int MODE>
