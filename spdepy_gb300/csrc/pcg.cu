@@ -492,21 +492,51 @@ __global__ void obs32_kernel(const double* __restrict__ obs, double tau, float* 
   if (k < n) o32[k] = float(tau * obs[k]);
 }
 
-// row-major FP64 (n x nrhs) -> column-major FP32, and x += xc back (xc = 0)
-__global__ void to32cm_kernel(const double* __restrict__ v, float* __restrict__ o, int64_t n, int nrhs) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= n * nrhs) return;
-  const int64_t k = e / nrhs;
-  o[(e - k * nrhs) * n + k] = float(v[e]);
+template <int V>
+struct IntC {
+  static constexpr int value = V;
+};
+
+// FP32 vectors of the solver hold their columns in groups of four (four values per
+// node side by side, one 16-byte access), then a group of two and single
+// columns; `packed` false keeps every column by itself (IC(0)).  Column c of
+// node k lies at lead n + width k + (c - lead) for the group [lead, lead + width).
+struct ColGroup {
+  int lead, width;
+};
+__host__ __device__ __forceinline__ ColGroup col_group(int c, int nrhs, int packed) {
+  if (!packed) return {c, 1};
+  const int n4 = nrhs & ~3;
+  if (c < n4) return {c & ~3, 4};
+  if ((nrhs & 2) && c < n4 + 2) return {n4, 2};
+  return {c, 1};
 }
-__global__ void acc64cm_kernel(double* __restrict__ x, float* __restrict__ xc, int64_t n, int nrhs) {
+__device__ __forceinline__ int64_t col_elem(int c, int64_t k, int64_t n, int nrhs, int packed) {
+  const ColGroup g = col_group(c, nrhs, packed);
+  return g.lead * n + g.width * k + (c - g.lead);
+}
+
+// row-major FP64 (n x nrhs) -> grouped FP32, and x += xc back (xc = 0)
+__global__ void to32cm_kernel(const double* __restrict__ v, float* __restrict__ o, int64_t n, int nrhs, int packed) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= n * nrhs) return;
   const int64_t k = e / nrhs;
-  const int64_t f = (e - k * nrhs) * n + k;
+  o[col_elem(int(e - k * nrhs), k, n, nrhs, packed)] = float(v[e]);
+}
+__global__ void acc64cm_kernel(double* __restrict__ x, float* __restrict__ xc, int64_t n, int nrhs, int packed) {
+  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e >= n * nrhs) return;
+  const int64_t k = e / nrhs;
+  const int64_t f = col_elem(int(e - k * nrhs), k, n, nrhs, packed);
   x[e] += double(xc[f]);
   xc[f] = 0.f;
 }
+
+// V values of one node (V = 1, 2 or 4 columns of a group)
+template <int V>
+struct alignas(4 * V) Cols {
+  float v[V];
+};
 
 // Fixed-order block sum of one float per thread into part[] (thread 0 writes)
 __device__ __forceinline__ double block_sum(float v, float* red) {
@@ -521,70 +551,132 @@ __device__ __forceinline__ double block_sum(float v, float* red) {
   return s;
 }
 
-// ap = A p in FP32 for column blockIdx.y, one thread per node (the cell's
-// coefficients, shared by all its time steps, come from L1 / L2), and the
-// block's partial sum of p . ap into part[col gridDim.x + block].  Node and
-// coefficient offsets fit in 32 bits (checked by the caller).
-__global__ void __launch_bounds__(256, 4) spmv32n_kernel(int Mx, int Ny, int T, int sep, float qe, float qm,
-                                                         float qo, const float* __restrict__ cf,
-                                                         const float* __restrict__ o32, const float* __restrict__ pv,
-                                                         float* __restrict__ apv, double* __restrict__ part) {
-  __shared__ float red[8];
-  const int Ns = Mx * Ny, n = Ns * T;
-  const int col = blockIdx.y;
-  const float* x = pv + int64_t(col) * n;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  float dot = 0.f;
-  if (k < n) {
-    const int t = k / Ns, c = k - t * Ns;
-    const int cy = c / Mx, cx = c - cy * Mx;
-    // bit (dx + 2) of vx: cx + dx inside the grid; likewise vy
-    const uint32_t vx = (cx >= 2 ? 1u : 0u) | (cx >= 1 ? 2u : 0u) | 4u | (cx + 1 < Mx ? 8u : 0u) | (cx + 2 < Mx ? 16u : 0u);
-    const uint32_t vy = (cy >= 2 ? 1u : 0u) | (cy >= 1 ? 2u : 0u) | 4u | (cy + 1 < Ny ? 8u : 0u) | (cy + 2 < Ny ? 16u : 0u);
-    const float* cc = cf + c;
-    const float* xt = x + k;
-    const int sb = (t == 0 && T > 1 && !sep) ? 0 : 25;
-    auto block25 = [&](const float* xs) {
-      float acc = 0.f;
+// The per-node kernels (stencil product, G, G^T) work on 32-node warps: warp group g
+// holds the nodes 32 g .. 32 g + 31 in node order, and the partial sums of the dot
+// products are those of a group (summed eight at a time by the scalar kernel).
+// A CTA's eight warps take groups R = round(Mx / 32) apart, i.e. nearly the same
+// columns of eight consecutive grid rows, and walk `steps` time steps with them in
+// strides of P = round(Ns / 32) groups, at most 16 nodes off the same cells: the
+// neighbours' vector values and the cells' coefficients (or rows of G) that a step
+// needs are then mostly in L1, from another warp or from the step before.
+struct Walk {
+  int R, P, steps, ngroups;  // groups per grid row and per time step, steps per CTA, groups in all
+  int rows8, bx;             // eight-row tiles and CTAs per time step
+};
+__device__ __forceinline__ int walk_group(const Walk& wk, int j) {
+  const int by = int(blockIdx.x) / wk.bx, cta = int(blockIdx.x) - by * wk.bx;
+  const int ry = cta / wk.R;
+  const int a1 = 8 * ry + int(threadIdx.x >> 5), a = (cta - ry * wk.R) + wk.R * a1;
+  const int64_t g = a + int64_t(by * wk.steps + j) * wk.P;
+  return a < wk.P && g < wk.ngroups ? int(g) : -1;
+}
+__device__ __forceinline__ float warp_sum(float v) {
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+
+// ap = A p in FP32 for the columns [lead + V y, + V), one thread per node and V
+// columns, and the warp groups' sums of p . ap into part[col gpad + group].  Node
+// and coefficient offsets fit in 32 bits (checked by the caller).
+// Bound: L1 / L2 loads (43 coefficients and 43 V vector values per node).  Four
+// columns per thread share the coefficients' loads and the index arithmetic.
+// Measured at 200 x 200 x 24: 16 columns 155 us (417 with one column per thread), at
+// 400 x 400 x 48 one column 178 us (228); with a branch per neighbour instead of
+// a zero coefficient 356 us for the 16 columns.
+template <int V, int SEP>
+__global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, float qe, float qm, float qo,
+                                                        Walk wk, int lead, int gpad, const float* __restrict__ cf,
+                                                        const float* __restrict__ o32, const float* __restrict__ pv,
+                                                        float* __restrict__ apv, float* __restrict__ part) {
+  const int Ns = Mx * Ny, n = Ns * T, lane = threadIdx.x & 31;
+  const int c0 = lead + V * int(blockIdx.y);
+  const Cols<V>* x = reinterpret_cast<const Cols<V>*>(pv + int64_t(c0) * n);
+  Cols<V>* out = reinterpret_cast<Cols<V>*>(apv + int64_t(c0) * n);
+  for (int j = 0; j < wk.steps; ++j) {
+    const int g = walk_group(wk, j);
+    if (g < 0) continue;
+    const int k = 32 * g + lane;
+    float dot[V];
 #pragma unroll
-      for (int s = 0; s < 25; ++s) {
-        const int dx = s % 5 - 2, dy = s / 5 - 2;
-        if ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u) acc = fmaf(cc[(sb + s) * Ns], xs[dy * Mx + dx], acc);
-      }
-      return acc;
-    };
-    float acc;
-    if (sep) {
-      // Q = Qt (x) Qs: Qt_tt (Qs x_t) + Qt_off (Qs x_(t-1) + Qs x_(t+1))
-      acc = (t == 0 || t == T - 1 ? qe : qm) * block25(xt);
-      if (t > 0) acc = fmaf(qo, block25(xt - Ns), acc);
-      if (t + 1 < T) acc = fmaf(qo, block25(xt + Ns), acc);
-    } else {
-      acc = block25(xt);
-      if (T > 1) {
-        if (t < T - 1) acc = fmaf(cc[68 * Ns], xt[0], acc);
-        if (t + 1 < T) {
+    for (int v = 0; v < V; ++v) dot[v] = 0.f;
+    if (k < n) {
+      const int t = k / Ns, c = k - t * Ns;
+      const int cy = c / Mx, cx = c - cy * Mx;
+      // bit (dx + 2) of vx: cx + dx inside the grid; likewise vy
+      const uint32_t vx = (cx >= 2 ? 1u : 0u) | (cx >= 1 ? 2u : 0u) | 4u | (cx + 1 < Mx ? 8u : 0u) | (cx + 2 < Mx ? 16u : 0u);
+      const uint32_t vy = (cy >= 2 ? 1u : 0u) | (cy >= 1 ? 2u : 0u) | 4u | (cy + 1 < Ny ? 8u : 0u) | (cy + 2 < Ny ? 16u : 0u);
+      const uint32_t vt = (t > 0 ? 1u : 0u) | 2u | (t + 1 < T ? 4u : 0u);
+      const float* cc = cf + c;
+      const Cols<V>* xt = x + k;
+      float acc[V];
+      // a neighbour outside the grid counts with coefficient zero (on the node's own
+      // value): no branches, so that the loads of a node overlap
+      auto add = [&](int slot, int dx, int dy, int dt, bool in) {
+        const float q = in ? cc[slot * Ns] : 0.f;
+        const Cols<V> xv = xt[in ? dt * Ns + dy * Mx + dx : 0];
 #pragma unroll
-          for (int s = 0; s < 9; ++s) {
-            const int dx = s % 3 - 1, dy = s / 3 - 1;
-            if ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u) acc = fmaf(cc[(50 + s) * Ns], xt[Ns + dy * Mx + dx], acc);
-          }
+        for (int v = 0; v < V; ++v) acc[v] = fmaf(q, xv.v[v], acc[v]);
+      };
+      auto block25 = [&](int sb, int dt) {
+        const bool vd = (vt >> (dt + 1)) & 1u;
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = 0.f;
+#pragma unroll
+        for (int s = 0; s < 25; ++s) {
+          const int dx = s % 5 - 2, dy = s / 5 - 2;
+          add(sb + s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
         }
-        if (t > 0) {
+      };
+      auto block9 = [&](int s0, int dt) {
+        const bool vd = (vt >> (dt + 1)) & 1u;
 #pragma unroll
-          for (int s = 0; s < 9; ++s) {
-            const int dx = s % 3 - 1, dy = s / 3 - 1;
-            if ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u) acc = fmaf(cc[(59 + s) * Ns], xt[-Ns + dy * Mx + dx], acc);
-          }
+        for (int s = 0; s < 9; ++s) {
+          const int dx = s % 3 - 1, dy = s / 3 - 1;
+          add(s0 + s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
+        }
+      };
+      if (SEP) {
+        // Q = Qt (x) Qs: Qt_tt (Qs x_t) + Qt_off (Qs x_(t-1) + Qs x_(t+1))
+        float s[V];
+        block25(25, 0);
+#pragma unroll
+        for (int v = 0; v < V; ++v) s[v] = (t == 0 || t == T - 1 ? qe : qm) * acc[v];
+#pragma unroll
+        for (int dt = -1; dt <= 1; dt += 2) {
+          block25(25, dt);
+#pragma unroll
+          for (int v = 0; v < V; ++v) s[v] = fmaf(qo, acc[v], s[v]);
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = s[v];
+      } else {
+        block25(t == 0 && T > 1 ? 0 : 25, 0);
+        add(68, 0, 0, 0, T > 1 && t < T - 1);
+        if (T > 1) {
+          block9(50, 1);
+          block9(59, -1);
         }
       }
+      const Cols<V> x0 = xt[0];
+      if (o32) {
+        const float q = o32[k];
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = fmaf(q, x0.v[v], acc[v]);
+      }
+      Cols<V> r;
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        r.v[v] = acc[v];
+        dot[v] = x0.v[v] * acc[v];
+      }
+      out[k] = r;
     }
-    if (o32) acc = fmaf(o32[k], xt[0], acc);
-    apv[int64_t(col) * n + k] = acc;
-    dot = xt[0] * acc;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const float w = warp_sum(dot[v]);
+      if (lane == 0) part[int64_t(c0 + v) * gpad + g] = w;
+    }
   }
-  const double bs = block_sum(dot, red);
-  if (threadIdx.x == 0) part[int64_t(col) * gridDim.x + blockIdx.x] = bs;
 }
 
 // Diagonal of A at node (cell c, time t) from the FP32 coefficients
@@ -601,41 +693,70 @@ __device__ __forceinline__ float diag32(const float* __restrict__ cf, int Ns, in
 //   mode 0: z = r;  mode 1: z = r / A_pp;  mode 2: z left to the G^T G kernel
 // and the block's partial sums of r . z (mode < 2) into partA[col G + b] and of
 // r . r into partB[col G + b].
+// The sums are those of kElemBlocks blocks per column; the launch leaves out the blocks
+// past the last node (G = gridDim.x of them run).
 constexpr int kElemBlocks = 1216;  // 8 per SM
-__global__ void __launch_bounds__(256) update32c_kernel(int Ns, int T, int sep, float qe, float qm, int mode,
-                                                        const float* __restrict__ cf, const float* __restrict__ o32,
-                                                        float* __restrict__ xc, float* __restrict__ rv,
-                                                        const float* __restrict__ pv, const float* __restrict__ apv,
-                                                        float* __restrict__ zv, const float* __restrict__ alpha,
-                                                        double* __restrict__ partA, double* __restrict__ partB) {
+template <int V>
+__global__ void __launch_bounds__(256, V == 1 ? 8 : 4) update32_kernel(int Ns, int T, int sep, float qe, float qm, int mode, int lead,
+                                                       const float* __restrict__ cf, const float* __restrict__ o32,
+                                                       float* __restrict__ xcv, float* __restrict__ rv,
+                                                       const float* __restrict__ pv, const float* __restrict__ apv,
+                                                       float* __restrict__ zv, const float* __restrict__ alpha,
+                                                       double* __restrict__ partA, double* __restrict__ partB) {
   __shared__ float red[8];
   const int64_t n = int64_t(Ns) * T;
-  const int col = blockIdx.y;
-  const float a = alpha[col];
-  float* r = rv + col * n;
-  float srz = 0.f, srr = 0.f;
-  for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x) {
-    float rk = r[k];
-    if (a != 0.f) {
-      xc[col * n + k] = fmaf(a, pv[col * n + k], xc[col * n + k]);
-      rk = fmaf(-a, apv[col * n + k], rk);
+  const int c0 = lead + V * int(blockIdx.y);
+  float a[V], srz[V], srr[V];
+  bool step = false;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    a[v] = alpha[c0 + v];
+    step |= a[v] != 0.f;
+    srz[v] = srr[v] = 0.f;
+  }
+  Cols<V>* r = reinterpret_cast<Cols<V>*>(rv + c0 * n);
+  Cols<V>* xc = reinterpret_cast<Cols<V>*>(xcv + c0 * n);
+  Cols<V>* z = reinterpret_cast<Cols<V>*>(zv + c0 * n);
+  const Cols<V>* p = reinterpret_cast<const Cols<V>*>(pv + c0 * n);
+  const Cols<V>* ap = reinterpret_cast<const Cols<V>*>(apv + c0 * n);
+  for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += int64_t(kElemBlocks) * blockDim.x) {
+    Cols<V> rk = r[k];
+    if (step) {
+      Cols<V> xk = xc[k];
+      const Cols<V> pk = p[k], ak = ap[k];
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (a[v] != 0.f) {
+          xk.v[v] = fmaf(a[v], pk.v[v], xk.v[v]);
+          rk.v[v] = fmaf(-a[v], ak.v[v], rk.v[v]);
+        }
+      xc[k] = xk;
       r[k] = rk;
     }
-    srr = fmaf(rk, rk, srr);
+#pragma unroll
+    for (int v = 0; v < V; ++v) srr[v] = fmaf(rk.v[v], rk.v[v], srr[v]);
     if (mode < 2) {
-      float zk = rk;
+      Cols<V> zk = rk;
       if (mode == 1) {
         const int t = int(k) / Ns, c = int(k) - t * Ns;  // node indices fit in 32 bits
-        zk = __fdividef(rk, diag32(cf, Ns, T, sep, qe, qm, c, t) + (o32 ? o32[k] : 0.f));
+        const float d = diag32(cf, Ns, T, sep, qe, qm, c, t) + (o32 ? o32[k] : 0.f);
+#pragma unroll
+        for (int v = 0; v < V; ++v) zk.v[v] = __fdividef(rk.v[v], d);
       }
-      zv[col * n + k] = zk;
-      srz = fmaf(rk, zk, srz);
+      z[k] = zk;
+#pragma unroll
+      for (int v = 0; v < V; ++v) srz[v] = fmaf(rk.v[v], zk.v[v], srz[v]);
     }
   }
-  const double b1 = block_sum(srz, red);
-  if (threadIdx.x == 0 && mode < 2) partA[int64_t(col) * gridDim.x + blockIdx.x] = b1;
-  const double b2 = block_sum(srr, red);
-  if (threadIdx.x == 0) partB[int64_t(col) * gridDim.x + blockIdx.x] = b2;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    if (mode < 2) {
+      const double b1 = block_sum(srz[v], red);
+      if (threadIdx.x == 0) partA[int64_t(c0 + v) * gridDim.x + blockIdx.x] = b1;
+    }
+    const double b2 = block_sum(srr[v], red);
+    if (threadIdx.x == 0) partB[int64_t(c0 + v) * gridDim.x + blockIdx.x] = b2;
+  }
 }
 
 // Weights of G: compact (rows per cell and time class, observed rows through
@@ -644,8 +765,14 @@ struct GWeights {
   const float* w;
   const uint32_t* mask;  // compact, with observations: observed nodes have their own rows
   const int* rank;
-  const uint32_t* near;  // with mask: bit p set when one of the 27 nodes p - d is observed
   int nob, Ns, T, compact;
+  // with mask: the nodes p whose row of G^T gathers from an observed node (bit p of
+  // near, number of bits before each word in nrank) have that row written out,
+  // near_w[o ncap + index]
+  const uint32_t* near;
+  const int* nrank;
+  const float* near_w;
+  int ncap;
 };
 
 // Bits of the nodes whose G^T row gathers from an observed node: p = q + d for
@@ -665,92 +792,149 @@ __global__ void near_obs_kernel(const int* __restrict__ nodes, int nob, int Mx, 
   }
 }
 
-// u = G r (TRANS 0) or z = G^T u with the block's partial sum of r . z
-// (TRANS 1) for column blockIdx.y, one thread per node; the rows of G come
-// from the compact (COMPACT 1) or per-node weights through L1 / L2.  Offsets
-// fit in 32 bits (checked by the caller).
-template <int TRANS, int COMPACT>
-__global__ void __launch_bounds__(256, 4) g32n_kernel(int Mx, int Ny, int T, GWeights gw,
-                                                      const float* __restrict__ xv, float* __restrict__ outv,
-                                                      const float* __restrict__ rv, double* __restrict__ part) {
-  __shared__ float red[8];
+// rank[w] = number of set bits before word w (one block of 1024 threads)
+__global__ void __launch_bounds__(1024) bit_rank_kernel(const uint32_t* __restrict__ bits, int nwords,
+                                                        int* __restrict__ rank) {
+  __shared__ int sums[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int base = 0;
+  for (int w0 = 0; w0 < nwords; w0 += 1024) {
+    const int i = w0 + tid, c = i < nwords ? __popc(bits[i]) : 0;
+    int v = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= d) v += u;
+    }
+    if (lane == 31) sums[warp] = v;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int q = 0; q < 32; ++q) {
+      if (q < warp) before += sums[q];
+      all += sums[q];
+    }
+    if (i < nwords) rank[i] = base + before + v - c;
+    base += all;
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ int time_class(int t, int T) { return t == 0 ? 0 : (t == T - 1 ? 2 : 1); }
+
+// The rows of G^T next to observed nodes: near_w[o ncap + i] = weight with which
+// node p gathers from q = p - d_o, 0 outside the grid
+__global__ void near_rows_kernel(int Mx, int Ny, int T, GWeights gw, float* __restrict__ near_w) {
   const int Ns = Mx * Ny, n = Ns * T;
-  const int col = blockIdx.y;
-  const float* x = xv + int64_t(col) * n;
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  float dot = 0.f;
-  if (p < n) {
-    const int t = p / Ns, c = p - t * Ns;
-    const int y = c / Mx, xx = c - y * Mx;
-    // bit (d + 1) set: the neighbour at +-d (sign of the direction used) is inside
-    const int sg = TRANS ? -1 : 1;
-    auto bits = [](int v, int lim, int sgn) {
-      return (v - sgn >= 0 && v - sgn < lim ? 1u : 0u) | 2u | (v + sgn >= 0 && v + sgn < lim ? 4u : 0u);
-    };
-    const uint32_t bx = bits(xx, Mx, sg), by = bits(y, Ny, sg), bt = bits(t, T, sg);
-    const float* w = gw.w;
-    // the weight row of node q (time tq, cell cq) for offset o
-    auto wrow = [&](int q, int tq, int cq, int o) -> float {
-      if (!COMPACT) return w[o * n + q];
-      if (gw.mask) {
-        const uint32_t m = gw.mask[q >> 5], bit = 1u << (q & 31);
-        if (m & bit) return w[3 * kOff * Ns + o * gw.nob + gw.rank[q >> 5] + __popc(m & (bit - 1u))];
-      }
-      const int kc = tq == 0 ? 0 : (tq == T - 1 ? 2 : 1);
-      return w[(kc * kOff + o) * Ns + cq];
-    };
-    float acc = 0.f;
-    // interior node (all 27 neighbours exist and, for G^T, lie in the interior
-    // time class): no validity tests, rows found without per-offset lookups
-    const bool inner = xx >= 1 && xx + 1 < Mx && y >= 1 && y + 1 < Ny && t >= 1 + TRANS && t + 1 + TRANS < T &&
-                       (!TRANS || !COMPACT || !gw.mask || !((gw.near[p >> 5] >> (p & 31)) & 1u));
-    if (inner && !TRANS) {
-      const float* wr;
-      int stride;
+  if (p >= n) return;
+  const uint32_t word = gw.near[p >> 5], bit = 1u << (p & 31);
+  if (!(word & bit)) return;
+  const int i = gw.nrank[p >> 5] + __popc(word & (bit - 1u));
+  const int t = p / Ns, c = p - t * Ns, y = c / Mx, x = c - y * Mx;
+  for (int o = 0; o < kOff; ++o) {
+    const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dt = o / 9 - 1;
+    const int xq = x - dx, yq = y - dy, tq = t - dt;
+    float v = 0.f;
+    if (xq >= 0 && xq < Mx && yq >= 0 && yq < Ny && tq >= 0 && tq < T) {
+      const int cq = yq * Mx + xq, q = tq * Ns + cq;
+      const uint32_t m = gw.mask[q >> 5], b = 1u << (q & 31);
+      if (m & b) v = gw.w[3 * kOff * Ns + o * gw.nob + gw.rank[q >> 5] + __popc(m & (b - 1u))];
+      else v = gw.w[(time_class(tq, T) * kOff + o) * Ns + cq];
+    }
+    near_w[int64_t(o) * gw.ncap + i] = v;
+  }
+}
+
+// u = G r (TRANS 0) or z = G^T u with the warp groups' sums of r . z (TRANS 1) for
+// the columns [lead + V y, + V), one thread per node and V columns; the rows of G
+// come from the compact (COMPACT 1) or per-node weights through L1 / L2.  Every
+// row is one base, stride and neighbour shift per time offset, so that observed
+// nodes, their neighbours and the boundary differ from the interior by a
+// predicate per offset and not by another path (a warp holds several kinds).
+// Offsets fit in 32 bits (checked by the caller).  Bound: L1 / L2 loads.
+// Measured at 200 x 200 x 24 with 1 % observed, 16 columns: G 101 us (413 with one
+// column per thread), G^T 150 us (1,026: near an observed node, which is in nearly
+// every warp, each of 27 weights was looked up through bitmask and rank).
+template <int V, int TRANS, int COMPACT>
+__global__ void __launch_bounds__(256, V == 1 ? 4 : 3) g32_kernel(int Mx, int Ny, int T, Walk wk, int lead, int gpad, GWeights gw,
+                                                     const float* __restrict__ xv, float* __restrict__ outv,
+                                                     const float* __restrict__ rv, float* __restrict__ part) {
+  const int Ns = Mx * Ny, n = Ns * T, lane = threadIdx.x & 31;
+  const int c0 = lead + V * int(blockIdx.y);
+  const Cols<V>* x = reinterpret_cast<const Cols<V>*>(xv + int64_t(c0) * n);
+  const Cols<V>* r = reinterpret_cast<const Cols<V>*>(rv + (TRANS ? int64_t(c0) * n : 0));
+  Cols<V>* out = reinterpret_cast<Cols<V>*>(outv + int64_t(c0) * n);
+  for (int j = 0; j < wk.steps; ++j) {
+    const int g = walk_group(wk, j);
+    if (g < 0) continue;
+    const int p = 32 * g + lane;
+    float dot[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) dot[v] = 0.f;
+    if (p < n) {
+      const int t = p / Ns, c = p - t * Ns;
+      const int y = c / Mx, xx = c - y * Mx;
+      // bit (d + 1) set: the neighbour at +d (G) or -d (G^T) is inside
+      const int sg = TRANS ? -1 : 1;
+      auto bits = [](int v, int lim, int sgn) {
+        return (v - sgn >= 0 && v - sgn < lim ? 1u : 0u) | 2u | (v + sgn >= 0 && v + sgn < lim ? 4u : 0u);
+      };
+      const uint32_t bx = bits(xx, Mx, sg), by = bits(y, Ny, sg), bt = bits(t, T, sg);
+      // weight of offset o: row[dt + 1][o stride - dy shift_y - dx shift_x]
+      const float* row[3];
+      int stride, shift_y = 0, shift_x = 0;
       if (!COMPACT) {
-        wr = w + p;
         stride = n;
+        shift_y = TRANS ? Mx : 0;
+        shift_x = TRANS ? 1 : 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) row[d] = gw.w + p - (TRANS ? (d - 1) * Ns : 0);
       } else {
-        wr = w + kOff * Ns + c;
-        stride = Ns;
-        if (gw.mask) {
-          const uint32_t m = gw.mask[p >> 5], bit = 1u << (p & 31);
-          if (m & bit) {
-            wr = w + 3 * kOff * Ns + gw.rank[p >> 5] + __popc(m & (bit - 1u));
-            stride = gw.nob;
-          }
+        const uint32_t* own = TRANS ? gw.near : gw.mask;  // nodes with a row of their own
+        const uint32_t word = own ? own[p >> 5] : 0u, bit = 1u << (p & 31);
+        if (word & bit) {
+          const int i = (TRANS ? gw.nrank : gw.rank)[p >> 5] + __popc(word & (bit - 1u));
+          stride = TRANS ? gw.ncap : gw.nob;
+          row[0] = row[1] = row[2] = (TRANS ? gw.near_w : gw.w + 3 * kOff * Ns) + i;
+        } else {
+          stride = Ns;
+          shift_y = TRANS ? Mx : 0;
+          shift_x = TRANS ? 1 : 0;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) row[d] = gw.w + time_class(TRANS ? t - (d - 1) : t, T) * kOff * Ns + c;
         }
       }
+      float acc[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) acc[v] = 0.f;
 #pragma unroll
       for (int o = 0; o < kOff; ++o) {
         const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dt = o / 9 - 1;
-        acc = fmaf(wr[o * stride], x[p + dt * Ns + dy * Mx + dx], acc);
+        // a neighbour outside the grid counts with weight zero (on the node's own value)
+        const bool in = (bx >> (dx + 1)) & (by >> (dy + 1)) & (bt >> (dt + 1)) & 1u;
+        const float wv = in ? row[dt + 1][o * stride - dy * shift_y - dx * shift_x] : 0.f;
+        const int d = in ? dt * Ns + dy * Mx + dx : 0;
+        const Cols<V> xq = x[TRANS ? p - d : p + d];
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = fmaf(wv, xq.v[v], acc[v]);
       }
-    } else if (inner) {
+      Cols<V> res;
 #pragma unroll
-      for (int o = 0; o < kOff; ++o) {
-        const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dt = o / 9 - 1;
-        const int d = dt * Ns + dy * Mx + dx;
-        const float wv = COMPACT ? w[(kOff + o) * Ns + c - dy * Mx - dx] : w[o * n + p - d];
-        acc = fmaf(wv, x[p - d], acc);
-      }
-    } else {
+      for (int v = 0; v < V; ++v) res.v[v] = acc[v];
+      out[p] = res;
+      if (TRANS) {
+        const Cols<V> rp = r[p];
 #pragma unroll
-      for (int o = 0; o < kOff; ++o) {
-        const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dt = o / 9 - 1;
-        if (!((bx >> (dx + 1)) & (by >> (dy + 1)) & (bt >> (dt + 1)) & 1u)) continue;
-        const int d = dt * Ns + dy * Mx + dx;
-        const int q = TRANS ? p - d : p + d;
-        const float wv = TRANS ? wrow(q, t - dt, c - dy * Mx - dx, o) : wrow(p, t, c, o);
-        acc = fmaf(wv, x[q], acc);
+        for (int v = 0; v < V; ++v) dot[v] = rp.v[v] * acc[v];
       }
     }
-    outv[int64_t(col) * n + p] = acc;
-    if (TRANS) dot = rv[int64_t(col) * n + p] * acc;
-  }
-  if (TRANS) {
-    const double bs = block_sum(dot, red);
-    if (threadIdx.x == 0) part[int64_t(col) * gridDim.x + blockIdx.x] = bs;
+    if (TRANS) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const float w = warp_sum(dot[v]);
+        if (lane == 0) part[int64_t(c0 + v) * gpad + g] = w;
+      }
+    }
   }
 }
 
@@ -895,31 +1079,75 @@ __global__ void __launch_bounds__(256) dot32c_kernel(const float* __restrict__ a
   if (threadIdx.x == 0) part[int64_t(blockIdx.y) * gridDim.x + blockIdx.x] = bs;
 }
 
-// Per-column scalars from block partials (one block per column, fixed order):
-//   mode 0: pap = sum partA;  alpha = rz / pap (0 if done or pap <= 0)
-//   mode 1: rzn = sum partA, rr = sum partB;  beta = rzn / rz, rz = rzn
-//   mode 2: rz = sum partA, rr = sum partB, beta = 0 (a new or replaced residual)
-__global__ void scal32_kernel(const double* __restrict__ partA, int na, const double* __restrict__ partB, int nb,
-                              int mode, const int* __restrict__ done, double* __restrict__ rz,
-                              double* __restrict__ rr, double* __restrict__ pap, float* __restrict__ alpha,
-                              float* __restrict__ beta) {
+// Per-column scalars from partial sums in a fixed order: sum A over na block sums
+// in partA, or (groupsA not null) over the blocks of eight warp groups each,
+// ngroups groups in all at groupsA[col gpad ..]; sum B over nb block sums in partB.
+// The blocks i, i + 256, ... are one chain of additions (256 chains, then a tree).
+//   mode 0: pap = sum A;  alpha = rz / pap (0 if done or pap <= 0)
+//   mode 1: rzn = sum A, rr = sum B;  beta = rzn / rz, rz = rzn
+//   mode 2: rz = sum A, rr = sum B, beta = 0 (a new or replaced residual)
+// gridDim.x (a power of two) CTAs share a column's chains, because an SM adds only
+// two FP64 values per clock; the last of them to finish (`arrived`, left at zero)
+// does the tree and the scalars.  Measured over 30,000 blocks: 12 us (94 with one CTA).
+__global__ void __launch_bounds__(256) scal32_kernel(const float* __restrict__ groupsA, int ngroups, int gpad,
+                                                     const double* __restrict__ partA, int na,
+                                                     const double* __restrict__ partB, int nb, int mode,
+                                                     const int* __restrict__ done, double* __restrict__ chains,
+                                                     unsigned* __restrict__ arrived, double* __restrict__ rz,
+                                                     double* __restrict__ rr, double* __restrict__ pap,
+                                                     float* __restrict__ alpha, float* __restrict__ beta) {
   __shared__ double sh[2][256];
-  const int col = blockIdx.x;
+  __shared__ bool last;
+  const int col = blockIdx.y, tid = threadIdx.x, Q = gridDim.x;
+  const int W = 256 / Q, chain = tid & (W - 1), lane = tid / W;  // this CTA's chains Q-fold: blocks chain0 + chain + 256 j
+  const int first = int(blockIdx.x) * W + chain;
+  const int nblocks = groupsA ? (ngroups + 7) / 8 : na;
+  const float4* ga = reinterpret_cast<const float4*>(groupsA + int64_t(col) * gpad);  // zero past the last group
   double s1 = 0.0, s2 = 0.0;
-  for (int i = threadIdx.x; i < na; i += 256) s1 += partA[int64_t(col) * na + i];
+  for (int j0 = 0; int(blockIdx.x) * W + 256 * j0 < nblocks; j0 += Q) {
+    const int b = first + 256 * (j0 + lane);
+    double s = 0.0;
+    if (b < nblocks) {
+      if (groupsA) {
+        const float4 u = ga[2 * b], v = ga[2 * b + 1];
+        s += u.x; s += u.y; s += u.z; s += u.w;
+        s += v.x; s += v.y; s += v.z; s += v.w;
+      } else {
+        s = partA[int64_t(col) * na + b];
+      }
+    }
+    sh[0][tid] = s;
+    __syncthreads();
+    if (tid < W)
+      for (int q = 0; q < Q; ++q) s1 += sh[0][q * W + tid];
+    __syncthreads();
+  }
+  if (Q > 1) {
+    if (tid < W) {
+      chains[int64_t(col) * 256 + first] = s1;
+      __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(&arrived[col], 1u) == unsigned(Q - 1);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s1 = __ldcg(chains + int64_t(col) * 256 + tid);
+    if (tid == 0) arrived[col] = 0u;
+  }
   if (mode != 0)
-    for (int i = threadIdx.x; i < nb; i += 256) s2 += partB[int64_t(col) * nb + i];
-  sh[0][threadIdx.x] = s1;
-  sh[1][threadIdx.x] = s2;
+    for (int i = tid; i < nb; i += 256) s2 += partB[int64_t(col) * nb + i];
+  sh[0][tid] = s1;
+  sh[1][tid] = s2;
   __syncthreads();
   for (int k = 128; k > 0; k >>= 1) {
-    if (threadIdx.x < k) {
-      sh[0][threadIdx.x] += sh[0][threadIdx.x + k];
-      sh[1][threadIdx.x] += sh[1][threadIdx.x + k];
+    if (tid < k) {
+      sh[0][tid] += sh[0][tid + k];
+      sh[1][tid] += sh[1][tid + k];
     }
     __syncthreads();
   }
-  if (threadIdx.x != 0) return;
+  if (tid != 0) return;
   const double a = sh[0][0], b = sh[1][0];
   if (mode == 0) {
     pap[col] = a;
@@ -935,14 +1163,30 @@ __global__ void scal32_kernel(const double* __restrict__ partA, int na, const do
   }
 }
 
-//   p = z + beta p (finished columns unchanged)
-__global__ void p32c_kernel(float* __restrict__ pv, const float* __restrict__ zv, const float* __restrict__ beta,
-                            const int* __restrict__ done, int64_t n) {
-  const int col = blockIdx.y;
-  if (done[col]) return;
-  const float b = beta[col];
-  for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x)
-    pv[col * n + k] = fmaf(b, pv[col * n + k], zv[col * n + k]);
+//   p = z + beta p (finished columns unchanged), columns [lead + V y, + V)
+template <int V>
+__global__ void p32_kernel(float* __restrict__ pv, const float* __restrict__ zv, const float* __restrict__ beta,
+                           const int* __restrict__ done, int64_t n, int lead) {
+  const int c0 = lead + V * int(blockIdx.y);
+  float b[V];
+  bool run[V], any = false;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    b[v] = beta[c0 + v];
+    run[v] = !done[c0 + v];
+    any |= run[v];
+  }
+  if (!any) return;
+  Cols<V>* p = reinterpret_cast<Cols<V>*>(pv + c0 * n);
+  const Cols<V>* z = reinterpret_cast<const Cols<V>*>(zv + c0 * n);
+  for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x) {
+    Cols<V> pk = p[k];
+    const Cols<V> zk = z[k];
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+      if (run[v]) pk.v[v] = fmaf(b[v], pk.v[v], zk.v[v]);
+    p[k] = pk;
+  }
 }
 
 }  // namespace
@@ -1085,17 +1329,25 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   if (len >= (int64_t(1) << 31) || int64_t(p->sym.n) * kOff >= (int64_t(1) << 31) || nrhs > 65535) return 1;
   const int Mx = p->sym.Mx, Ny = p->sym.Ny, Ns = Mx * Ny, T = p->sym.T;
   cudaStream_t st = p->stream;
-  const int nsp = nblk(n, 256);  // blocks of the per-node kernels (stencil product, G, G^T)
+  const int nsp = nblk(n, 256);  // blocks of 256 consecutive nodes (dot products)
+  const int ngroups = nblk(n, 32), gpad = 8 * nsp;
+  const int nel = std::min(int(kElemBlocks), nsp);  // elementwise blocks with nodes
   const int na_max = std::max(nsp, int(kElemBlocks));
+  const int packed = kind == 4 ? 0 : 1;
   // FP64: true residual (row-major), block partials, per-column scalars
   const size_t need64 = size_t(len) + size_t(nrhs) * (na_max + kElemBlocks) + size_t(kDotBlocks) * nrhs +
-                        size_t(8 * nrhs) + size_t(nrhs);
+                        size_t(8 * nrhs) + size_t(nrhs) + size_t(257) * nrhs;
   double* base = scratch(p, need64);
-  // FP32 (column-major): r, z, p, Ap, x correction, G r; coefficients; observation term; alpha, beta
+  // FP32: r, z, p, Ap, x correction, G r (grouped columns); coefficients; observation
+  // term; warp-group sums; alpha, beta; rows of G^T next to observed nodes
   const bool near_bits = kind == 3 && with_obs;  // G^T needs the nodes next to observed ones
   const size_t nwords = size_t((n + 31) / 32);
-  const size_t need32 = size_t(6 * len) + size_t(kCoef32) * Ns + size_t(n) + size_t(2 * nrhs) +
-                        (kind == 4 ? size_t(kIcRow) * n : 0) + (near_bits ? nwords : 0);
+  const int64_t ncap = near_bits ? std::min<int64_t>(n, int64_t(kOff) * p->nob) : 0;
+  auto pad4 = [](size_t e) { return (e + 3) & ~size_t(3); };  // 16-byte sections
+  const size_t vlen = pad4(size_t(len));  // a group of columns then starts at a multiple of its width
+  const size_t need32 = 6 * vlen + size_t(nrhs) * gpad + pad4(size_t(kCoef32) * Ns) + pad4(size_t(n)) +
+                        pad4(size_t(2 * nrhs)) + (kind == 4 ? pad4(size_t(kIcRow) * n) : 0) +
+                        (near_bits ? 2 * pad4(nwords) + size_t(kOff) * ncap : 0);
   float* b32 = scratch32(p, need32);
   if (!base || !b32) return 4;
   double* r64 = base;
@@ -1105,13 +1357,18 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   double* sc = part64 + size_t(kDotBlocks) * nrhs;
   double *rz = sc, *pap = sc + nrhs, *rr = sc + 2 * nrhs, *bb = sc + 3 * nrhs, *rrt = sc + 4 * nrhs;
   int* done = reinterpret_cast<int*>(sc + 8 * nrhs);
-  float *r32 = b32, *z32 = r32 + len, *p32 = z32 + len, *ap32 = p32 + len, *xc32 = ap32 + len, *u32 = xc32 + len;
-  float* cf = u32 + len;
-  float* o32 = cf + size_t(kCoef32) * Ns;
-  float* alpha = o32 + n;
+  double* chains = sc + 9 * nrhs;  // 256 per column
+  unsigned* arrived = reinterpret_cast<unsigned*>(chains + size_t(256) * nrhs);
+  float *r32 = b32, *z32 = r32 + vlen, *p32 = z32 + vlen, *ap32 = p32 + vlen, *xc32 = ap32 + vlen, *u32 = xc32 + vlen;
+  float* gsum = u32 + vlen;  // warp groups' sums of a dot product, per column
+  float* cf = gsum + size_t(nrhs) * gpad;
+  float* o32 = cf + pad4(size_t(kCoef32) * Ns);
+  float* alpha = o32 + pad4(size_t(n));
   float* beta = alpha + nrhs;
-  float* Lic = beta + nrhs;  // IC(0) factor (kind 4)
-  uint32_t* near = reinterpret_cast<uint32_t*>(Lic + (kind == 4 ? size_t(kIcRow) * n : 0));
+  float* Lic = alpha + pad4(size_t(2 * nrhs));  // IC(0) factor (kind 4)
+  uint32_t* near = reinterpret_cast<uint32_t*>(Lic + (kind == 4 ? pad4(size_t(kIcRow) * n) : 0));
+  int* nrank = reinterpret_cast<int*>(near + (near_bits ? pad4(nwords) : 0));
+  float* near_w = reinterpret_cast<float*>(nrank + (near_bits ? pad4(nwords) : 0));
   const QStencil q = p->qstencil();
   const double* obs = with_obs ? p->d_obs_cnt : nullptr;
   const int sep = q.sep;
@@ -1130,16 +1387,41 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
     if (!ok) return 7;
     w += kCompactHeader;
   }
-  GWeights gw{w, near_bits ? p->d_obs_mask : nullptr, p->d_obs_rank, near_bits ? near : nullptr, p->nob, Ns, T,
-              kind == 3 ? 1 : 0};
+  GWeights gw{w, near_bits ? p->d_obs_mask : nullptr, p->d_obs_rank, p->nob, Ns, T, kind == 3 ? 1 : 0,
+              near_bits ? near : nullptr, nrank, near_w, int(ncap)};
   if (near_bits) {
     cudaMemsetAsync(near, 0, nwords * sizeof(uint32_t), st);
     if (p->nob > 0) near_obs_kernel<<<nblk(p->nob), 256, 0, st>>>(p->d_obs_nodes, p->nob, Mx, Ny, T, near);
+    bit_rank_kernel<<<1, 1024, 0, st>>>(near, int(nwords), nrank);
+    near_rows_kernel<<<nblk(n), 256, 0, st>>>(Mx, Ny, T, gw, near_w);
   }
+  cudaMemsetAsync(gsum, 0, size_t(nrhs) * gpad * sizeof(float), st);
+  cudaMemsetAsync(arrived, 0, size_t(nrhs) * sizeof(unsigned), st);
   coef32_kernel<<<nblk(Ns, 128), 128, 0, st>>>(q, cf);
   if (obs) obs32_kernel<<<nblk(n), 256, 0, st>>>(obs, tau, o32, n);
   const float* o = obs ? o32 : nullptr;
-  const dim3 gsp(nsp, nrhs), gel(kElemBlocks, nrhs);
+  // f(IntC<V>, first column, groups) for the columns in groups of V = 4, 2, 1
+  auto by_groups = [&](auto&& f) {
+    const int n4 = packed ? nrhs & ~3 : 0, n2 = packed ? nrhs & 2 : 0, n1 = nrhs - n4 - n2;
+    if (n4) f(IntC<4>{}, 0, n4 / 4);
+    if (n2) f(IntC<2>{}, n4, 1);
+    if (n1) f(IntC<1>{}, n4 + n2, n1);
+  };
+  // time steps per CTA of the per-node kernels: as many as leave the GPU two waves
+  // of CTAs (four per SM)
+  auto walk = [&](int groups, dim3* grid) {
+    Walk wk;
+    wk.P = std::max(1, (Ns + 16) / 32);
+    wk.R = std::max(1, std::min(wk.P, (Mx + 16) / 32));
+    wk.ngroups = ngroups;
+    wk.rows8 = ((wk.P + wk.R - 1) / wk.R + 7) / 8;
+    wk.bx = wk.R * wk.rows8;
+    const int nb = (ngroups + wk.P - 1) / wk.P;
+    wk.steps = 8;
+    while (wk.steps > 1 && int64_t(wk.bx) * ((nb + wk.steps - 1) / wk.steps) * groups < 2 * 4 * 152) wk.steps /= 2;
+    *grid = dim3(wk.bx * ((nb + wk.steps - 1) / wk.steps), groups);
+    return wk;
+  };
   const int nlev = (Mx - 1) + 3 * (Ny - 1) + 5 * (T - 1) + 1;
   const dim3 glev(nblk(int64_t(Ny) * T, 128), nrhs);
   if (kind == 4) {
@@ -1166,28 +1448,49 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   }
   // z = M r with the partial sums of r . z and r . r, after the update of r by alpha
   auto update_precond = [&]() {
-    update32c_kernel<<<gel, 256, 0, st>>>(Ns, T, sep, qe, qm, mode, cf, o, xc32, r32, p32, ap32, z32, alpha, partA,
-                                          partB);
-    if (mode == 2 && kind == 3) {
-      g32n_kernel<0, 1><<<gsp, 256, 0, st>>>(Mx, Ny, T, gw, r32, u32, nullptr, nullptr);
-      g32n_kernel<1, 1><<<gsp, 256, 0, st>>>(Mx, Ny, T, gw, u32, z32, r32, partA);
-    } else if (kind == 4) {
+    by_groups([&](auto vw, int lead, int groups) {
+      constexpr int V = decltype(vw)::value;
+      update32_kernel<V><<<dim3(nel, groups), 256, 0, st>>>(Ns, T, sep, qe, qm, mode, lead, cf, o, xc32, r32, p32, ap32,
+                                                            z32, alpha, partA, partB);
+      if (mode != 2 || kind == 4) return;
+      dim3 grid;
+      const Walk wk = walk(groups, &grid);
+      if (kind == 3) {
+        g32_kernel<V, 0, 1><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, r32, u32, nullptr, nullptr);
+        g32_kernel<V, 1, 1><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, u32, z32, r32, gsum);
+      } else {
+        g32_kernel<V, 0, 0><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, r32, u32, nullptr, nullptr);
+        g32_kernel<V, 1, 0><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, u32, z32, r32, gsum);
+      }
+    });
+    if (kind == 4) {
       for (int lev = 0; lev < nlev; ++lev)
         ic0_solve_kernel<1><<<glev, 128, 0, st>>>(lev, Mx, Ny, T, Lic, r32, u32);
       for (int lev = nlev - 1; lev >= 0; --lev)
         ic0_solve_kernel<0><<<glev, 128, 0, st>>>(lev, Mx, Ny, T, Lic, u32, z32);
-      dot32c_kernel<<<gsp, 256, 0, st>>>(r32, z32, int(n), partA);
-    } else if (mode == 2) {
-      g32n_kernel<0, 0><<<gsp, 256, 0, st>>>(Mx, Ny, T, gw, r32, u32, nullptr, nullptr);
-      g32n_kernel<1, 0><<<gsp, 256, 0, st>>>(Mx, Ny, T, gw, u32, z32, r32, partA);
+      dot32c_kernel<<<dim3(nsp, nrhs), 256, 0, st>>>(r32, z32, int(n), partA);
     }
   };
-  const int na = mode == 2 ? nsp : int(kElemBlocks);
+  // r . z: block sums of the update (none, Jacobi) or of IC(0)'s dot product, else G^T's group sums
+  const int na = mode == 2 ? nsp : nel;
+  const float* gz = mode == 2 && kind != 4 ? gsum : nullptr;
+  // CTAs per column of the scalar kernel: one per two blocks of each chain, up to 64
+  auto scalars = [&](const float* groups, int na_, int nb_, int what) {
+    int Q = 1;
+    while (Q < 64 && (groups ? nsp : na_) > 512 * Q) Q *= 2;
+    scal32_kernel<<<dim3(Q, nrhs), 256, 0, st>>>(groups, ngroups, gpad, partA, na_, partB, nb_, what, done, chains,
+                                                 arrived, rz, rr, pap, alpha, beta);
+  };
+  auto new_direction = [&]() {  // p = z + beta p
+    by_groups([&](auto vw, int lead, int groups) {
+      p32_kernel<decltype(vw)::value><<<dim3(nel, groups), 256, 0, st>>>(p32, z32, beta, done, n, lead);
+    });
+  };
   // a new residual r32: z = M r, rz = r . z (p unchanged)
   auto restart = [&]() {
     cudaMemsetAsync(alpha, 0, size_t(nrhs) * sizeof(float), st);
     update_precond();
-    scal32_kernel<<<nrhs, 256, 0, st>>>(partA, na, partB, kElemBlocks, 2, done, rz, rr, pap, alpha, beta);
+    scalars(gz, na, nel, 2);
   };
   auto true_residual = [&]() {
     launch_spmv(q, obs, tau, x, r64, nrhs, st);
@@ -1206,20 +1509,28 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
     if (!(hb[c] > 0.0)) hd[c] = 1;  // a zero right-hand side is solved by x = 0
   cudaMemcpyAsync(done, hd.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, st);
   href = hb;
-  to32cm_kernel<<<nblk(len), 256, 0, st>>>(b, r32, n, nrhs);
+  to32cm_kernel<<<nblk(len), 256, 0, st>>>(b, r32, n, nrhs, packed);
   restart();
-  p32c_kernel<<<gel, 256, 0, st>>>(p32, z32, beta, done, n);  // p = z
+  new_direction();  // p = z
   const double tol2 = tol * tol;
   const int every = std::max(1, std::min(check_every, 4));
   int it = 0, last_rep = 0;
   bool all_done = false, fresh = false;  // fresh: x holds every correction and rrt is its true residual
   for (int c = 0; c < nrhs; ++c) all_done = (c == 0 || all_done) && hd[c];
   while (it < maxit && !all_done) {
-    spmv32n_kernel<<<gsp, 256, 0, st>>>(Mx, Ny, T, sep, qe, qm, qo, cf, o, p32, ap32, partA);
-    scal32_kernel<<<nrhs, 256, 0, st>>>(partA, nsp, partB, 0, 0, done, rz, rr, pap, alpha, beta);
+    by_groups([&](auto vw, int lead, int groups) {
+      dim3 grid;
+      const Walk wk = walk(groups, &grid);
+      constexpr int V = decltype(vw)::value;
+      if (sep)
+        spmv32_kernel<V, 1><<<grid, 256, 0, st>>>(Mx, Ny, T, qe, qm, qo, wk, lead, gpad, cf, o, p32, ap32, gsum);
+      else
+        spmv32_kernel<V, 0><<<grid, 256, 0, st>>>(Mx, Ny, T, qe, qm, qo, wk, lead, gpad, cf, o, p32, ap32, gsum);
+    });
+    scalars(gsum, 0, 0, 0);
     update_precond();
-    scal32_kernel<<<nrhs, 256, 0, st>>>(partA, na, partB, kElemBlocks, 1, done, rz, rr, pap, alpha, beta);
-    p32c_kernel<<<gel, 256, 0, st>>>(p32, z32, beta, done, n);
+    scalars(gz, na, nel, 1);
+    new_direction();
     ++it;
     fresh = false;
     if (it % every != 0 && it != maxit) continue;
@@ -1229,7 +1540,7 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
     for (int c = 0; c < nrhs && !replace; ++c)
       if (!hd[c] && (hr[c] <= kReplaceDrop * kReplaceDrop * href[c] || hr[c] <= tol2 * hb[c])) replace = true;
     if (!replace) continue;
-    acc64cm_kernel<<<nblk(len), 256, 0, st>>>(x, xc32, n, nrhs);
+    acc64cm_kernel<<<nblk(len), 256, 0, st>>>(x, xc32, n, nrhs, packed);
     true_residual();
     cudaMemcpyAsync(hr.data(), rrt, nrhs * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return 2;
@@ -1244,11 +1555,11 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
     if (all_done) break;
     cudaMemcpyAsync(done, hd.data(), nrhs * sizeof(int), cudaMemcpyHostToDevice, st);
     // continue from the true residual (p kept)
-    to32cm_kernel<<<nblk(len), 256, 0, st>>>(r64, r32, n, nrhs);
+    to32cm_kernel<<<nblk(len), 256, 0, st>>>(r64, r32, n, nrhs, packed);
     restart();
   }
   if (!fresh) {
-    acc64cm_kernel<<<nblk(len), 256, 0, st>>>(x, xc32, n, nrhs);
+    acc64cm_kernel<<<nblk(len), 256, 0, st>>>(x, xc32, n, nrhs, packed);
     true_residual();
     cudaMemcpyAsync(hr.data(), rrt, nrhs * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return 2;
