@@ -37,6 +37,10 @@ constexpr int kTcMinKUpdate = 64;  // ... for the rank-64 updates inside a facto
 // shortest K of a cluster-pair task: below it the pair's per-task set-up and
 // pipeline fill outweigh its throughput, and the single-CTA kernel is faster
 constexpr int kPairMinK = 256;
+// Smallest FP64 product (rows, columns, k) on the tensor cores: a CUDA-core 64 x 64
+// tile takes about 1 us per k value (the FP64 pipe), a tensor-core tile a fixed 10 us
+// with its share of the split, and 2.3 us per 32 values.
+constexpr int kEmuMin = 32;
 enum { KT_NONE = 0, KT_A_UPPER, KT_B_LOWER, KT_BOTH_UPPER };
 constexpr int kPanel = 512;   // panel width of the two-level blocked factorisation
 
@@ -56,10 +60,14 @@ void Schedule::upload() {
   d_ext = upload_vec(ext);
   d_rows = upload_vec(rows);
   d_mirror = upload_vec(mirror);
+  d_esplit = upload_vec(esplit);
+  d_emu = upload_vec(emu);
 }
 void Schedule::release() {
   cudaFree(d_gemm); cudaFree(d_diag); cudaFree(d_ext); cudaFree(d_rows); cudaFree(d_mirror); cudaFree(d_maps);
+  cudaFree(d_esplit); cudaFree(d_emu);
   d_gemm = nullptr; d_diag = nullptr; d_ext = nullptr; d_rows = nullptr; d_mirror = nullptr; d_maps = nullptr;
+  d_esplit = nullptr; d_emu = nullptr;
 }
 
 // ----------------------------------------------------------- schedule helpers
@@ -67,8 +75,76 @@ struct Builder {
   Schedule& s;
   int TM, TN;
   bool pair_ok;   // products of at least 128 x 128 x kPairMinK may take 256 x 256 cluster-pair tiles (FP32 plan)
+  bool emu_ok;    // products of at least kEmuMin in every size go to OP_EMU (FP64 plan)
   int depth = 0;  // tree depth of the ops begun next
-  explicit Builder(Schedule& sc, int tm, int tn, bool pairs = false) : s(sc), TM(tm), TN(tn), pair_ok(pairs) {}
+  explicit Builder(Schedule& sc, int tm, int tn, bool pairs = false, bool emu = false)
+      : s(sc), TM(tm), TN(tn), pair_ok(pairs), emu_ok(emu) {}
+
+  // operands split by the op being built: (buffer, offset, ld, k) -> rows, digits, row exponents
+  struct EmuOperand { int rows; int64_t dst; int exp; };
+  std::map<std::tuple<int, int64_t, int, int>, EmuOperand> emu_operands;
+  int64_t emu_cursor = 0;
+  int emu_row_cursor = 0;
+  double emu_flops = 0.0;
+  size_t emu_first = 0, esplit_first = 0;
+
+  EmuOperand emu_operand(int buf, int which, int64_t off, int ld, int rows, int k) {
+    const auto key = std::make_tuple(buf, off, ld, k);
+    auto it = emu_operands.find(key);
+    if (it != emu_operands.end() && it->second.rows >= rows) return it->second;
+    const int nch = (k + 31) / 32;
+    EmuOperand o{rows, emu_cursor, emu_row_cursor};
+    for (int r = 0; r < rows; r += 64) {
+      s.esplit.push_back({off + int64_t(r) * ld, emu_cursor, ld, std::min(64, rows - r), k, nch, o.exp + r, which});
+      emu_cursor += nch * kEmuChunkBytes;
+    }
+    emu_row_cursor += (rows + 63) / 64 * 64;
+    emu_operands[key] = o;
+    return o;
+  }
+  // C (op)= A B' in 128 x 64 tiles of OP_EMU; arguments as gemm_tiles
+  void emu_tiles(int64_t a, int lda, int64_t b, int ldb, int64_t c, int ldc, int m, int n, int k, bool lower, int kt) {
+    const Op& op = s.ops.back();
+    const EmuOperand x = emu_operand(op.abuf, 0, a, lda, m, k), y = emu_operand(op.bbuf, 1, b, ldb, n, k);
+    const int64_t step = int64_t((k + 31) / 32) * kEmuChunkBytes;  // a 64-row tile
+    for (int j0 = 0; j0 < n; j0 += 64)
+      for (int i0 = lower ? j0 : 0; i0 < m; i0 += 128) {
+        int klo = 0, khi = k;
+        if (kt == KT_A_UPPER) klo = std::min(i0, k);
+        else if (kt == KT_B_LOWER) khi = std::min(k, j0 + 64);
+        else if (kt == KT_BOTH_UPPER) klo = std::min(std::max(i0, j0), k);
+        if (khi <= klo) { klo = 0; khi = std::min(k, 1); }
+        EmuTask t;
+        t.a = x.dst + i0 / 64 * step;
+        t.b = y.dst + j0 / 64 * step;
+        t.c = c + int64_t(i0) * ldc + j0;
+        t.a_step = m - i0 > 64 ? step : 0;
+        t.ldc = ldc;
+        t.m = std::min(128, m - i0);
+        t.n = std::min(64, n - j0);
+        t.k0 = klo / 32;
+        t.k1 = (khi + 31) / 32;
+        t.ea = x.exp + i0;
+        t.eb = y.exp + j0;
+        s.emu.push_back(t);
+        emu_flops += 2.0 * t.m * t.n * (khi - klo);
+      }
+  }
+  // an OP_EMU with the tiles collected since begin(), like the op `proto`
+  void emu_op(const Op& proto) {
+    Op o = proto;
+    o.kind = OP_EMU;
+    o.tc = kPathSimt;
+    o.off = int64_t(emu_first);
+    o.count = int(s.emu.size() - emu_first);
+    o.soff = int64_t(esplit_first);
+    o.scount = int(s.esplit.size() - esplit_first);
+    o.flops = emu_flops;
+    s.ops.push_back(o);
+    s.launches += 2;
+    s.emu_bytes = std::max(s.emu_bytes, emu_cursor);
+    s.emu_rows = std::max<int64_t>(s.emu_rows, emu_row_cursor);
+  }
 
   // TMA source of a row-major operand starting at element `off` of buffer `buf`,
   // inside the region [base, ...) with row stride ld: the map index and the
@@ -97,6 +173,12 @@ struct Builder {
     Op& o = s.ops.back();
     o.kind = kind;
     o.depth = depth;
+    emu_operands.clear();
+    emu_cursor = 0;
+    emu_row_cursor = 0;
+    emu_flops = 0.0;
+    emu_first = s.emu.size();
+    esplit_first = s.esplit.size();
     switch (kind) {
       case OP_GEMM: o.off = int64_t(s.gemm.size()); break;
       case OP_DIAG: o.off = int64_t(s.diag.size()); break;
@@ -107,8 +189,10 @@ struct Builder {
     return o;
   }
   void end() {
-    if (s.ops.back().kind == OP_GEMM) split_by_k();
+    const Op proto = s.ops.back();
+    if (proto.kind == OP_GEMM) split_by_k();
     finish(s.ops.back());
+    if (s.emu.size() > emu_first) emu_op(proto);
   }
   // Tiles with a short K (panel solves, rank-64 updates) run on the SIMT kernel,
   // the others on the tensor-core kernel: split one GEMM launch into two, the
@@ -196,6 +280,11 @@ struct Builder {
                   int64_t bbase = -1) {
     if (m <= 0 || n <= 0 || k <= 0) return;
     const Op& op = s.ops.back();
+    if (emu_ok && arow == lda && brow == ldb && op.al == kRow && op.bl == kRow && m >= kEmuMin && n >= kEmuMin &&
+        k >= kEmuMin && i_start == 0) {
+      emu_tiles(a, lda, b, ldb, c, ldc, m, n, k, lower, kt);
+      return;
+    }
     const bool pair = pair_ok && abase >= 0 && bbase >= 0 && arow == lda && brow == ldb && op.al == kRow &&
                       op.bl == kRow && m >= 128 && n >= 128 && k >= kPairMinK && i_start == 0;
     const int tm = pair ? kPairTile : TM, tn = pair ? kPairTile : TN;
@@ -243,8 +332,8 @@ struct Builder {
 
 static inline int nblocks(int ns) { return (ns + kNbk - 1) / kNbk; }
 
-static void build_factor_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, bool pairs) {
-  Builder b(sc, TM, TN, pairs);
+static void build_factor_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, bool pairs, bool emu) {
+  Builder b(sc, TM, TN, pairs, emu);
   const auto& F = S.fronts;
   for (int d = S.max_depth; d >= 0; --d) {
     const auto& fr = S.by_depth[d];
@@ -533,8 +622,8 @@ static void build_bwd_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, 
 // (row-major); for a node [a, b) of the halving tree with children [a, m), [m, b):
 //   TT = W_11^T L_21^T,  (W^T)_12 = -TT W_22^T,  W_21 = ((W^T)_12)^T.
 static void build_selinv_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, int64_t* scratch_elems,
-                                  bool pairs) {
-  Builder b(sc, TM, TN, pairs);
+                                  bool pairs, bool emu) {
+  Builder b(sc, TM, TN, pairs, emu);
   const auto& F = S.fronts;
   auto r4 = [](int64_t v) { return (v + 3) / 4 * 4; };
   int64_t scratch = 32;
@@ -1251,6 +1340,11 @@ struct Exec {
                          o.tc, o.nmax, p->tc_wait_ns);
           if (on_tc) tc_launch_log(o);
           break;
+        case OP_EMU:
+          if constexpr (sizeof(T) == sizeof(double))
+            launch_emu_gemm(s.d_esplit + o.soff, o.scount, s.d_emu + o.off, o.count, buf(o.abuf), buf(o.bbuf),
+                            buf(o.cbuf), o.mode, p->d_emu, p->d_emu_exp, p->d_emu_err, st, p->tc_wait_ns);
+          break;
         case OP_SGATHER_FWD: {
           int pd = o.depth & 1;
           sgather_fwd_kernel<T><<<o.count, 256, 0, st>>>(s.d_rows + o.off, p->d_fronts, p->d_rmap, buf(B_X),
@@ -1480,9 +1574,30 @@ int plan_build(Plan* p) {
     CUDA_TRY(cudaMalloc(&p->d_pool[k], size_t(p->pool_elems[k]) * es));
   }
   const bool pairs = p->precision == 1 && tc_gemm_enabled();
-  build_factor_schedule(S, p->sched_factor, TM, TM, pairs);
+  bool emu = p->precision == 0 && tc_gemm_enabled();
   int64_t sx_elems = 0;
-  build_selinv_schedule(S, p->sched_selinv, TM, TM, &sx_elems, pairs);
+  build_factor_schedule(S, p->sched_factor, TM, TM, pairs, emu);
+  build_selinv_schedule(S, p->sched_selinv, TM, TM, &sx_elems, pairs, emu);
+  if (emu) {
+    // digits and row exponents of the largest launch; without the memory the
+    // products stay on the CUDA cores
+    const int64_t bytes = std::max(p->sched_factor.emu_bytes, p->sched_selinv.emu_bytes);
+    const int64_t rows = std::max(p->sched_factor.emu_rows, p->sched_selinv.emu_rows);
+    if (bytes > 0 && (cudaMalloc(&p->d_emu, size_t(bytes)) != cudaSuccess ||
+                      cudaMalloc(&p->d_emu_exp, size_t(rows) * sizeof(int)) != cudaSuccess ||
+                      cudaMalloc(&p->d_emu_err, sizeof(int)) != cudaSuccess)) {
+      cudaGetLastError();
+      cudaFree(p->d_emu); cudaFree(p->d_emu_exp);
+      p->d_emu = nullptr;
+      p->d_emu_exp = nullptr;
+      p->sched_factor = Schedule();
+      p->sched_selinv = Schedule();
+      build_factor_schedule(S, p->sched_factor, TM, TM, pairs, false);
+      build_selinv_schedule(S, p->sched_selinv, TM, TM, &sx_elems, pairs, false);
+    } else if (bytes > 0) {
+      CUDA_TRY(cudaMemset(p->d_emu_err, 0, sizeof(int)));
+    }
+  }
   CUDA_TRY(cudaMalloc(&p->d_sx, size_t(sx_elems) * es));
   if (pairs) {
     const int64_t sizes[] = {S.l_size, p->pool_elems[0], p->pool_elems[1], sx_elems};
@@ -1506,6 +1621,21 @@ int plan_build(Plan* p) {
   return 0;
 }
 
+// Reads and clears the FP64 tensor-core products' wait-failure flag.
+static int emu_take_error(Plan* p) {
+  if (!p->d_emu_err) return 0;
+  int* h = p->pin_int() + 3;
+  *h = 0;
+  cudaMemcpyAsync(h, p->d_emu_err, sizeof(int), cudaMemcpyDeviceToHost, p->stream);
+  cudaStreamSynchronize(p->stream);
+  const int e = *h;
+  if (e) {
+    cudaMemsetAsync(p->d_emu_err, 0, sizeof(int), p->stream);
+    cudaStreamSynchronize(p->stream);
+  }
+  return e;
+}
+
 template <typename T>
 static int factor_t(Plan* p, int with_obs, double tau) {
   const Symbolic& S = p->sym;
@@ -1522,7 +1652,11 @@ static int factor_t(Plan* p, int with_obs, double tau) {
   CUDA_TRY(cudaGetLastError());
   const double sum = p->h_pin[1024];
   const int err = p->pin_int()[0];
-  if (tc_gemm_take_error(p->stream, p->pin_int() + 1)) { p->last_error = "tensor-core product timed out"; p->factored = 0; return 2; }
+  if (tc_gemm_take_error(p->stream, p->pin_int() + 1) || emu_take_error(p)) {
+    p->last_error = "tensor-core product timed out";
+    p->factored = 0;
+    return 2;
+  }
   if (err >= 0) {
     char buf[128];
     std::snprintf(buf, sizeof(buf), "matrix is not positive definite (front %d)", err);
@@ -1698,7 +1832,7 @@ static int selinv_t(Plan* p, double* zq) {
   p->launches_total += 1;
   CUDA_TRY(cudaStreamSynchronize(st));
   CUDA_TRY(cudaGetLastError());
-  if (tc_gemm_take_error(p->stream, p->pin_int() + 1)) {
+  if (tc_gemm_take_error(p->stream, p->pin_int() + 1) || emu_take_error(p)) {
     p->last_error = "tensor-core product timed out";
     p->factored = 0;
     return 2;

@@ -17,7 +17,8 @@ namespace spde {
 
 enum OpKind {
   OP_MEMSET = 0, OP_EXTEND, OP_DIAG, OP_GEMM, OP_SGATHER_FWD, OP_SGATHER_BWD, OP_ZGATHER, OP_MIRROR, OP_ZEXTRACT,
-  OP_FWD_CHAIN, OP_BWD_CHAIN
+  OP_FWD_CHAIN, OP_BWD_CHAIN,
+  OP_EMU  // FP64 products on the tensor cores (split, then product)
 };
 // profile class of a tiled product that ran on the tensor cores (the others count as OP_GEMM)
 constexpr int kProfTensorCore = 9;
@@ -47,6 +48,8 @@ struct Op {
   int abuf = B_NONE, bbuf = B_NONE, cbuf = B_NONE;
   int64_t elems = 0;  // memset length
   int depth = 0;
+  int64_t soff = 0;   // OP_EMU: first split task and their number
+  int scount = 0;
 };
 
 // 32 x 32 block copy, rows x cols of src: dst[j*ldd + i] = src[i*lds + j] when
@@ -78,6 +81,9 @@ struct Schedule {
   std::vector<MirrorTask> mirror;
   std::vector<MapReq> maps;
   std::map<std::tuple<int, int64_t, int>, int> map_index;
+  std::vector<EmuSplit> esplit;
+  std::vector<EmuTask> emu;
+  int64_t emu_bytes = 0, emu_rows = 0;  // digit scratch and row exponents of the largest launch
   // device copies
   GemmTask* d_gemm = nullptr;
   DiagTask* d_diag = nullptr;
@@ -85,6 +91,8 @@ struct Schedule {
   RowTask* d_rows = nullptr;
   MirrorTask* d_mirror = nullptr;
   CUtensorMap* d_maps = nullptr;
+  EmuSplit* d_esplit = nullptr;
+  EmuTask* d_emu = nullptr;
   int launches = 0;
   void upload();
   void release();
@@ -148,6 +156,11 @@ struct Plan {
   void* d_pool[2] = {nullptr, nullptr};
   void* d_sx = nullptr;  // selected-inversion scratch (triangular inverse, X^T)
   int64_t pool_elems[2] = {0, 0};
+  // FP64 plan: split operands of one launch of OP_EMU (digits, row exponents) and
+  // the flag its kernel sets when a wait gives up
+  uint8_t* d_emu = nullptr;
+  int* d_emu_exp = nullptr;
+  int* d_emu_err = nullptr;
   double* d_logpiv = nullptr;
   int* d_err = nullptr;
   // one-column triangular sweeps (engine.cu, fwd_chain_kernel / bwd_chain_kernel):

@@ -27,6 +27,7 @@
 #include <cstdint>
 
 #include "kernels.cuh"
+#include "tc_common.cuh"
 
 namespace spde {
 
@@ -47,10 +48,6 @@ constexpr int kTmemCols = 512;             // power of two >= 128 + kStages * 64
 constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s
 
 __device__ int g_tc_error = 0;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 // byte offset of the 16-byte chunk c4 (k = 4 c4 .. 4 c4 + 3) of row r inside a
 // 128 x 32 FP32 K-major tile with the 128-byte swizzle
@@ -79,28 +76,6 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
       "r"(tmem_a), "l"(b), "r"(kIdesc), "r"(acc));
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(mbar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
@@ -207,10 +182,6 @@ __device__ __forceinline__ void a_to_tmem(const uint8_t* raw, int row, int h, ui
   }
   tmem_st16(taddr + 16 * h, hi);
   tmem_st16(taddr + 32 + 16 * h, lo);
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 
 template <int MODE, int AL, int BL>
@@ -442,9 +413,6 @@ __device__ __forceinline__ bool mbar_try_cluster(uint32_t mbar, uint32_t parity)
       : "r"(mbar), "r"(parity)
       : "memory");
   return ok != 0;
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
 // 2-D TMA load of one box at (x, y) into shared memory; completion is counted on mbar
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
