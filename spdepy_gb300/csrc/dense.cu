@@ -474,193 +474,15 @@ template void launch_gemm<double>(const GemmTask*, int, const double*, const dou
 template void launch_gemm<float>(const GemmTask*, int, const float*, const float*, float*, int, int, int,
                                  cudaStream_t, int, int, unsigned long long);
 
-// --------------------------------------------------- diagonal block POTRF
-// Cholesky factor and inverse of one w x w diagonal block (w <= 64) per CTA.
-//
-// The factorisation runs in FP64 whatever the storage type, so the pivots and
-// the log-determinant carry FP64 arithmetic (an FP32 sweep measured 1e-6
-// relative log-likelihood error against 1e-7 at 960k nodes).  FP64 is a narrow
-// pipe on this part, so the sweep is arranged around it: the block lives in the
-// registers of 256 threads, thread (ty, tx) = (tid / 16, tid % 16) owning the
-// entries (i, k) = (ty + 16 m, tx + 16 n), m, n = 0..3.  Step j reads column j of
-// the partly reduced block from a shared buffer, applies
-// a_ik -= a_ij a_kj / a_jj (j < k <= i) and publishes column j + 1, one barrier
-// per column and one FP64 division per warp; square roots come at the end:
-// L_ij = a_ij / sqrt(d_j) and log L_jj = log(d_j) / 2 with d_j the j-th pivot.
-// L^-1 (consumed by the panel products as a product operand) then follows by
-// forward elimination in the storage type's arithmetic with the same ownership.
+// ------------------------------------------------------------ diagonal blocks
+// The mixed plan's diagonal blocks are eliminated in double-float arithmetic (value =
+// hi + lo, two FP32 numbers, about 44 significant bits; Dekker/Knuth error-free
+// transformations with FMA), which runs on the FP32 pipe instead of the narrow FP64
+// one (an FP32 sweep measured 1e-6 relative log-likelihood error against 1e-7 at 960k
+// nodes).  Pivots are converted to FP64 for the log-determinant; L and L^-1 are
+// rounded to FP32 for storage (L^-1 from the FP32 L).
 constexpr int kMaxNbk = 64;
 
-template <typename T>
-__global__ void __launch_bounds__(256) potrf_kernel(const DiagTask* __restrict__ tasks, T* __restrict__ L,
-                                                    T* __restrict__ dinv, double* __restrict__ logpiv,
-                                                    int* __restrict__ err) {
-  __shared__ double colb[2][kMaxNbk];
-  __shared__ double dpiv[kMaxNbk];
-  __shared__ double sq[kMaxNbk];
-  __shared__ T lsh[kMaxNbk][kMaxNbk + 1];
-  __shared__ T xrow[2][kMaxNbk];
-  __shared__ int bad;
-  const DiagTask tk = tasks[blockIdx.x];
-  const int w = tk.w;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  T* blk = L + tk.a;
-  double r[4][4];
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int i = ty + 16 * m, k = tx + 16 * n;
-      r[m][n] = (k <= i && i < w) ? double(blk[int64_t(i) * tk.lda + k]) : 0.0;
-    }
-  if (tid == 0) bad = 0;
-  if (tx == 0) {
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-      if (ty + 16 * m < w) colb[0][ty + 16 * m] = r[m][0];
-  }
-  __syncthreads();
-  for (int j = 0; j < w; ++j) {
-    const double* c = colb[j & 1];
-    double d = c[j];
-    if (!(d > 0.0) || !isfinite(d)) {
-      d = 1.0;
-      if (tid == 0) bad = 1;
-    }
-    double q = 0.0;
-    if ((tid & 31) == 0) q = 1.0 / d;
-    const double dv = __shfl_sync(0xffffffffu, q, 0);
-    if (tid == 0) dpiv[j] = d;
-    double ci[4], ck[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int i = ty + 16 * m;
-      ci[m] = (i > j && i < w) ? c[i] * dv : 0.0;
-    }
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int k = tx + 16 * n;
-      ck[n] = (k > j && k < w) ? c[k] : 0.0;
-    }
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      if (16 * m + 15 <= j) continue;  // block row finished (uniform over the CTA)
-#pragma unroll
-      for (int n = 0; n <= m; ++n) {
-        if (16 * n + 15 <= j) continue;
-        r[m][n] -= ci[m] * ck[n];
-      }
-    }
-    // publish column j + 1 (its owners hold it fully reduced by columns 0..j)
-    const int jn = j + 1;
-    if (jn < w && tx == (jn & 15)) {
-      const int n = jn >> 4;
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const int i = ty + 16 * m;
-        if (i >= jn && i < w) {
-#pragma unroll
-          for (int nn = 0; nn < 4; ++nn)
-            if (nn == n) colb[jn & 1][i] = r[m][nn];
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (tid < w) sq[tid] = sqrt(dpiv[tid]);
-  if (tid < 32) {
-    double s = 0.0;
-    for (int j = tid; j < w; j += 32) s += 0.5 * log(dpiv[j]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (tid == 0) {
-      logpiv[blockIdx.x] = s;
-      if (bad) atomicCAS(err, -1, tk.front);
-    }
-  }
-  __syncthreads();
-  // L = a_ik / sqrt(d_k) below the diagonal, sqrt(d_k) on it; zero above
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int i = ty + 16 * m, k = tx + 16 * n;
-      if (i < w && k < w) {
-        const T v = k < i ? T(r[m][n] / sq[k]) : (k == i ? T(sq[k]) : T(0));
-        lsh[i][k] = v;
-        blk[int64_t(i) * tk.lda + k] = v;
-      }
-    }
-  // X = L^-1: B = I; step j takes the finished row j of X and applies
-  // B_ic -= L_ij X_jc (i > j, c <= j); row j + 1 finishes as B_(j+1)c / L_(j+1)(j+1)
-  T b[4][4];
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) b[m][n] = (ty + 16 * m == tx + 16 * n) ? T(1) : T(0);
-  __syncthreads();
-  if (ty == 0 && tx == 0) {
-    b[0][0] = T(1) / lsh[0][0];
-    xrow[0][0] = b[0][0];
-  }
-  __syncthreads();
-  for (int j = 0; j < w; ++j) {
-    const T* xr = xrow[j & 1];
-    T li[4], xc[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int i = ty + 16 * m;
-      li[m] = (i > j && i < w) ? lsh[i][j] : T(0);
-    }
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int cc = tx + 16 * n;
-      xc[n] = cc <= j ? xr[cc] : T(0);
-    }
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      if (16 * m + 15 <= j) continue;
-#pragma unroll
-      for (int n = 0; n <= m; ++n) {
-        if (16 * n > j) continue;  // columns beyond j of row j of X are zero
-        b[m][n] -= li[m] * xc[n];
-      }
-    }
-    const int jn = j + 1;
-    if (jn < w && ty == (jn & 15)) {
-      const int m = jn >> 4;
-      const T inv = T(1) / lsh[jn][jn];
-#pragma unroll
-      for (int mm = 0; mm < 4; ++mm) {
-        if (mm != m) continue;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const int cc = tx + 16 * n;
-          if (cc <= jn) {
-            b[mm][n] *= inv;
-            xrow[jn & 1][cc] = b[mm][n];
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  T* dv = dinv + tk.dinv;
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int i = ty + 16 * m, cc = tx + 16 * n;
-      if (i < w && cc < w) dv[int64_t(i) * kMaxNbk + cc] = cc <= i ? b[m][n] : T(0);
-    }
-}
-
-// ---------------------------------------------- double-float diagonal block
-// The mixed path's diagonal blocks: the same register-blocked right-looking
-// sweep as potrf_kernel, in double-float arithmetic (value = hi + lo, two FP32
-// numbers, about 44 significant bits; Dekker/Knuth error-free transformations
-// with FMA), which runs on the FP32 pipe instead of the narrow FP64 one.  Pivots
-// are converted to FP64 for the log-determinant; L and L^-1 are rounded to FP32
-// for storage (L^-1 from the FP32 L, as in potrf_kernel).
 struct DF {
   float hi, lo;
 };
@@ -713,12 +535,12 @@ __device__ __forceinline__ float df_rsqrt(DF d) {
   return fmaf(0.5f * y, e, y);
 }
 
-// Double-float factorisation of one diagonal block A = L L^T (w <= 64) and its
-// inverse, one CTA per block.
+// Factorisation of one diagonal block A = L L^T (w <= 64) and its inverse, one CTA per
+// block; T the storage type, the elimination in double-float (FP32 storage) or FP64.
 //
 // The elimination is written A_ik -= (a_ic / d_c) a_kc, so that the pivots d_c
-// and the columns a_ic (at the time column c is eliminated) stay in double-float
-// and L_ic = a_ic / sqrt(d_c) is rounded to FP32 once, at the end.  Every entry
+// and the columns a_ic (at the time column c is eliminated) stay in the elimination's
+// arithmetic and L_ic = a_ic / sqrt(d_c) is rounded to storage once, at the end.  Every entry
 // takes its updates in the order of c, so the result does not depend on how the
 // work is split over threads.
 //
@@ -741,85 +563,140 @@ __device__ __forceinline__ float df_rsqrt(DF d) {
 // panel has more registers (30 us for one block) but 1,280 blocks take 143.
 constexpr int kDfSub = 16;
 constexpr int kDfLd = kMaxNbk + 4;          // row stride of L and L^-1 in shared memory (16-byte rows)
-constexpr int kDfPan = kDfSub + 2;          // row stride (double-floats) of a panel in shared memory
+constexpr int kDfPan = kDfSub + 2;          // row stride of a panel in shared memory
+template <typename T>
+constexpr int potrf_smem() { return (2 * kMaxNbk * kDfLd + 3 * kDfSub * kDfSub) * int(sizeof(T)); }
 
-template <int N>
-struct IntC {
-  static constexpr int value = N;
+// The elimination's arithmetic by storage type: numbers, their shared-memory form,
+// products, reciprocal and reciprocal square root of a pivot.
+template <typename T>
+struct Elim;
+template <>
+struct Elim<float> {
+  using Num = DF;
+  using Pair = float2;  // in shared memory
+  static constexpr int kMinCtas = 3;
+  static __device__ __forceinline__ DF from(float v) { return DF{v, 0.0f}; }
+  static __device__ __forceinline__ DF load(Pair v) { return DF{v.x, v.y}; }
+  static __device__ __forceinline__ Pair pack(DF v) { return make_float2(v.hi, v.lo); }
+  static __device__ __forceinline__ DF shfl(DF v, int lane) {
+    return DF{__shfl_sync(0xffffffffu, v.hi, lane), __shfl_sync(0xffffffffu, v.lo, lane)};
+  }
+  static __device__ __forceinline__ DF mul(DF a, DF b) { return df_mul(a, b); }
+  static __device__ __forceinline__ DF fms(DF a, DF b, DF c) { return df_fms(a, b, c); }
+  static __device__ __forceinline__ DF rcp(DF d) { return df_rcp(d); }
+  static __device__ __forceinline__ float rsqrt_of(DF d) { return df_rsqrt(d); }
+  static __device__ __forceinline__ bool bad(DF d) { return !(d.hi > 0.0f) || !isfinite(d.hi); }
+  static __device__ __forceinline__ float value(DF v) { return v.hi + v.lo; }
+  static __device__ __forceinline__ double wide(DF v) { return double(v.hi) + double(v.lo); }
+};
+template <>
+struct Elim<double> {
+  using Num = double;
+  using Pair = double;
+  static constexpr int kMinCtas = 2;
+  static __device__ __forceinline__ double from(double v) { return v; }
+  static __device__ __forceinline__ double load(Pair v) { return v; }
+  static __device__ __forceinline__ Pair pack(double v) { return v; }
+  static __device__ __forceinline__ double shfl(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+  static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
+  static __device__ __forceinline__ double fms(double a, double b, double c) { return fma(-b, c, a); }
+  // 1 / d for d > 0: the FP32 reciprocal of the significand and two Newton steps
+  // (four FP64 operations instead of a full division on the narrow pipe); pivots
+  // outside the normal range of d and 1 / d take the division
+  static __device__ __forceinline__ double rcp(double d) {
+    const long long b = __double_as_longlong(d);
+    const int f = int(b >> 52);
+    if (f < 2 || f > 2044) return 1.0 / d;
+    const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | (1023ll << 52));  // in [1, 2)
+    double y = double(__fdividef(1.0f, float(m)));
+    y = fma(y, fma(-m, y, 1.0), y);
+    y = fma(y, fma(-m, y, 1.0), y);
+    return __longlong_as_double(__double_as_longlong(y) - (static_cast<long long>(f - 1023) << 52));
+  }
+  static __device__ __forceinline__ double rsqrt_of(double d) { return rsqrt(d); }
+  static __device__ __forceinline__ bool bad(double d) { return !(d > 0.0) || !isfinite(d); }
+  static __device__ __forceinline__ double value(double v) { return v; }
+  static __device__ __forceinline__ double wide(double v) { return v; }
 };
 
-__global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __restrict__ tasks, float* __restrict__ L,
-                                                          float* __restrict__ dinv, double* __restrict__ logpiv,
-                                                          int* __restrict__ err) {
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+}
+__device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
+  *reinterpret_cast<double2*>(v) = *reinterpret_cast<const double2*>(p);
+  *reinterpret_cast<double2*>(v + 2) = *reinterpret_cast<const double2*>(p + 2);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
+    potrf_kernel(const DiagTask* __restrict__ tasks, T* __restrict__ L, T* __restrict__ dinv,
+                 double* __restrict__ logpiv, int* __restrict__ err) {
+  using E = Elim<T>;
+  using Num = typename E::Num;
+  using Pair = typename E::Pair;
   // L and L^-1; before that, two panel buffers and the panel's multipliers
-  __shared__ __align__(16) float smem[2 * kMaxNbk * kDfLd];
-  __shared__ float Tb[3 * kDfSub * kDfSub];
-  __shared__ float dph[kMaxNbk], dpl[kMaxNbk], rsq[kMaxNbk];
+  extern __shared__ __align__(16) uint8_t potrf_sm[];
+  __shared__ Pair dp[kMaxNbk];
+  __shared__ T rsq[kMaxNbk];
   __shared__ int bad;
-  static_assert(2 * kMaxNbk * kDfLd >= 3 * 2 * kMaxNbk * kDfPan, "panel buffers fit");
-  float (*Ls)[kDfLd] = reinterpret_cast<float (*)[kDfLd]>(smem);
-  float (*Xs)[kDfLd] = Ls + kMaxNbk;
-  float2 (*pan0)[kDfPan] = reinterpret_cast<float2 (*)[kDfPan]>(smem);
-  float2 (*mul)[kDfPan] = pan0 + 2 * kMaxNbk;  // S_ic = a_ic / d_c
+  static_assert(2 * kMaxNbk * kDfLd * sizeof(T) >= 3 * kMaxNbk * kDfPan * sizeof(Pair), "panel buffers fit");
+  T (*Ls)[kDfLd] = reinterpret_cast<T (*)[kDfLd]>(potrf_sm);
+  T (*Xs)[kDfLd] = Ls + kMaxNbk;
+  T* Tb = &Xs[kMaxNbk][0];                     // 3 x 256 products of the inverse
+  Pair (*pan0)[kDfPan] = reinterpret_cast<Pair (*)[kDfPan]>(potrf_sm);
+  Pair (*mul)[kDfPan] = pan0 + 2 * kMaxNbk;    // S_ic = a_ic / d_c
   const DiagTask tk = tasks[blockIdx.x];
   const int w = tk.w;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ty = tid >> 4, tx = tid & 15;
-  float* blk = L + tk.a;
-  DF r[4][4];                               // n <= m used
+  T* blk = L + tk.a;
+  Num r[4][4];                               // n <= m used
 #pragma unroll
   for (int m = 0; m < 4; ++m)
 #pragma unroll
     for (int n = 0; n <= m; ++n) {
       const int i = ty + 16 * m, k = tx + 16 * n;
-      r[m][n] = DF{(k <= i && i < w) ? blk[int64_t(i) * tk.lda + k] : 0.0f, 0.0f};
+      r[m][n] = E::from((k <= i && i < w) ? blk[int64_t(i) * tk.lda + k] : T(0));
     }
   if (tid == 0) bad = 0;
   for (int jb = 0; 16 * jb < w; ++jb) {
-    float2 (*pan)[kDfPan] = pan0 + (jb & 1) * kMaxNbk;
+    Pair (*pan)[kDfPan] = pan0 + (jb & 1) * kMaxNbk;
     const int c0 = 16 * jb, cw = min(kDfSub, w - c0);
     // block column jb to shared memory (the register indices are compile-time constants)
 #pragma unroll
     for (int n = 0; n < 4; ++n)
       if (n == jb) {
 #pragma unroll
-        for (int m = n; m < 4; ++m) pan[ty + 16 * m][tx] = make_float2(r[m][n].hi, r[m][n].lo);
+        for (int m = n; m < 4; ++m) pan[ty + 16 * m][tx] = E::pack(r[m][n]);
       }
     __syncthreads();
     if (warp == 0 || c0 + 16 * (warp + 1) < w) {
       const int row = lane < 16 ? c0 + lane : min(c0 + 16 * (warp + 1) + lane - 16, kMaxNbk - 1);
-      DF x[16];
+      Num x[16];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const float2 v = pan[row][k];
-        x[k] = DF{v.x, v.y};
-      }
+      for (int k = 0; k < 16; ++k) x[k] = E::load(pan[row][k]);
       __syncwarp();
       const bool own = lane >= 16 ? c0 + 16 * (warp + 1) < w : warp == 0;  // this lane's row is written by this warp
-      float piv_h = 1.0f, piv_l = 0.0f;
+      Num piv = E::from(T(1));
       bool failed = false;
       // columns >= cw are zero: their pivot counts as 1 and they change nothing
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        DF d{__shfl_sync(0xffffffffu, x[j].hi, j), __shfl_sync(0xffffffffu, x[j].lo, j)};
-        const bool nonpos = !(d.hi > 0.0f) || !isfinite(d.hi);
-        if (nonpos) d = DF{1.0f, 0.0f};
-        const DF sj = df_mul(x[j], df_rcp(d));
-        piv_h = lane == j ? d.hi : piv_h;
-        piv_l = lane == j ? d.lo : piv_l;
+        Num d = E::shfl(x[j], j);
+        const bool nonpos = E::bad(d);
+        if (nonpos) d = E::from(T(1));
+        const Num sj = E::mul(x[j], E::rcp(d));
+        if (lane == j) piv = d;
         failed |= nonpos && j < cw;
         if (own) {
-          pan[row][j] = make_float2(x[j].hi, x[j].lo);
-          mul[row][j] = make_float2(sj.hi, sj.lo);
+          pan[row][j] = E::pack(x[j]);
+          mul[row][j] = E::pack(sj);
         }
 #pragma unroll
-        for (int k = j + 1; k < 16; ++k) {
-          const DF a{__shfl_sync(0xffffffffu, x[j].hi, k), __shfl_sync(0xffffffffu, x[j].lo, k)};
-          x[k] = df_fms(x[k], sj, a);
-        }
+        for (int k = j + 1; k < 16; ++k) x[k] = E::fms(x[k], sj, E::shfl(x[j], k));
       }
       if (warp == 0 && lane < cw) {
-        dph[c0 + lane] = piv_h;
-        dpl[c0 + lane] = piv_l;
+        dp[c0 + lane] = E::pack(piv);
         if (failed) bad = 1;
       }
     }
@@ -828,24 +705,23 @@ __global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __rest
       constexpr int n = decltype(block)::value;
 #pragma unroll
       for (int m = n; m < 4; ++m) {  // the panel's final entries
-        const float2 v = pan[ty + 16 * m][tx];
-        r[m][n] = DF{v.x, v.y};
+        r[m][n] = E::load(pan[ty + 16 * m][tx]);
       }
       if (c0 + 16 < w) {
 #pragma unroll 4
-        for (int c = 0; c < kDfSub; c += 2) {
-          float4 sv[4], av[4];
+        for (int c = 0; c < kDfSub; c += 2) {  // two columns per 16-byte load
+          Pair sv[4][2], av[4][2];
 #pragma unroll
           for (int m = n + 1; m < 4; ++m) {
-            sv[m] = *reinterpret_cast<const float4*>(&mul[ty + 16 * m][c]);
-            av[m] = *reinterpret_cast<const float4*>(&pan[tx + 16 * m][c]);
+            *reinterpret_cast<float4*>(sv[m]) = *reinterpret_cast<const float4*>(&mul[ty + 16 * m][c]);
+            *reinterpret_cast<float4*>(av[m]) = *reinterpret_cast<const float4*>(&pan[tx + 16 * m][c]);
           }
 #pragma unroll
           for (int m = n + 1; m < 4; ++m)
 #pragma unroll
             for (int q = n + 1; q <= m; ++q) {
-              r[m][q] = df_fms(r[m][q], DF{sv[m].x, sv[m].y}, DF{av[q].x, av[q].y});
-              r[m][q] = df_fms(r[m][q], DF{sv[m].z, sv[m].w}, DF{av[q].z, av[q].w});
+              r[m][q] = E::fms(r[m][q], E::load(sv[m][0]), E::load(av[q][0]));
+              r[m][q] = E::fms(r[m][q], E::load(sv[m][1]), E::load(av[q][1]));
             }
         }
       }
@@ -858,19 +734,19 @@ __global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __rest
     }
   }
   __syncthreads();
-  if (tid < w) rsq[tid] = df_rsqrt(DF{dph[tid], dpl[tid]});
+  if (tid < w) rsq[tid] = E::rsqrt_of(E::load(dp[tid]));
   __syncthreads();
-  // L = a_ik / sqrt(d_k) (FP32), zero above the diagonal
+  // L = a_ik / sqrt(d_k), zero above the diagonal
 #pragma unroll
   for (int m = 0; m < 4; ++m)
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
       const int i = ty + 16 * m, k = tx + 16 * n;
       if (i < w && k < w) {
-        float v = 0.0f;
+        T v = T(0);
         if (n <= m) {
-          if (k < i) v = (r[m][n].hi + r[m][n].lo) * rsq[k];
-          else if (k == i) v = 1.0f / rsq[k];
+          if (k < i) v = E::value(r[m][n]) * rsq[k];
+          else if (k == i) v = T(1) / rsq[k];
         }
         Ls[i][k] = v;
         blk[int64_t(i) * tk.lda + k] = v;
@@ -882,24 +758,24 @@ __global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __rest
     // diagonal 16 x 16 inverse of sub-block `warp`, lane = column: x_ii = -(sum_{k < ii} L_(ii,k) x_k) / L_(ii,ii)
     if (lane < kDfSub) {
       const int c0 = warp * kDfSub, cw = min(kDfSub, w - c0), c = lane;
-      float sum[kDfSub];
+      T sum[kDfSub];
 #pragma unroll
-      for (int ii = 0; ii < kDfSub; ++ii) sum[ii] = 0.0f;
+      for (int ii = 0; ii < kDfSub; ++ii) sum[ii] = T(0);
 #pragma unroll
       for (int k = 0; k < kDfSub; ++k) {
         if (k >= cw) break;
-        float x = 0.0f;
+        T x = T(0);
         if (k == c) x = rsq[c0 + k];
         else if (k > c) x = -sum[k] * rsq[c0 + k];
         Xs[c0 + k][c0 + c] = x;
 #pragma unroll
         for (int ii = k + 1; ii < kDfSub; ++ii)
-          if (ii < cw) sum[ii] = fmaf(Ls[c0 + ii][c0 + k], x, sum[ii]);
+          if (ii < cw) sum[ii] = fma(Ls[c0 + ii][c0 + k], x, sum[ii]);
       }
     }
   } else if (warp == 7) {
     double s = 0.0;
-    for (int j = lane; j < w; j += 32) s += 0.5 * log(double(dph[j]) + double(dpl[j]));
+    for (int j = lane; j < w; j += 32) s += 0.5 * log(E::wide(E::load(dp[j])));
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) {
       logpiv[blockIdx.x] = s;
@@ -914,14 +790,13 @@ __global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __rest
 #pragma unroll
     for (int pi = 0; pi < 4 - dd; ++pi) {
       const int i = (dd + pi) * kDfSub + ty;  // rows >= w compute values that nothing reads
-      float s = 0.0f;
+      T s = T(0);
 #pragma unroll
       for (int k4 = 4 * pi; k4 < 4 * (pi + dd); ++k4) {
-        const float4 l = *reinterpret_cast<const float4*>(&Ls[i][4 * k4]);
-        s = fmaf(l.x, Xs[4 * k4 + 0][pi * kDfSub + tx], s);
-        s = fmaf(l.y, Xs[4 * k4 + 1][pi * kDfSub + tx], s);
-        s = fmaf(l.z, Xs[4 * k4 + 2][pi * kDfSub + tx], s);
-        s = fmaf(l.w, Xs[4 * k4 + 3][pi * kDfSub + tx], s);
+        T l[4];
+        load4(&Ls[i][4 * k4], l);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s = fma(l[e], Xs[4 * k4 + e][pi * kDfSub + tx], s);
       }
       Tb[(pi << 8) + tid] = s;
     }
@@ -929,14 +804,14 @@ __global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __rest
 #pragma unroll
     for (int pi = 0; pi < 4 - dd; ++pi) {
       const int bi = dd + pi, i = bi * kDfSub + ty;
-      float s = 0.0f;
+      T s = T(0);
 #pragma unroll
       for (int r4 = 0; r4 < kDfSub / 4; ++r4) {
-        const float4 xi = *reinterpret_cast<const float4*>(&Xs[i][bi * kDfSub + 4 * r4]);
-        const float xr[4] = {xi.x, xi.y, xi.z, xi.w};
+        T xr[4];
+        load4(&Xs[i][bi * kDfSub + 4 * r4], xr);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float nx = fmaf(xr[e], Tb[(pi << 8) + ((4 * r4 + e) << 4) + tx], s);
+          const T nx = fma(xr[e], Tb[(pi << 8) + ((4 * r4 + e) << 4) + tx], s);
           if (4 * r4 + e <= ty) s = nx;
         }
       }
@@ -944,24 +819,25 @@ __global__ void __launch_bounds__(256, 3) potrf_df_kernel(const DiagTask* __rest
     }
     __syncthreads();
   }
-  float* dvp = dinv + tk.dinv;
+  T* dvp = dinv + tk.dinv;
 #pragma unroll
   for (int m = 0; m < 4; ++m)
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
       const int i = ty + 16 * m, c = tx + 16 * n;
-      if (i < w && c < w) dvp[int64_t(i) * kMaxNbk + c] = c <= i ? Xs[i][c] : 0.0f;
+      if (i < w && c < w) dvp[int64_t(i) * kMaxNbk + c] = c <= i ? Xs[i][c] : T(0);
     }
 }
 
 template <typename T>
 void launch_potrf(const DiagTask* tasks, int ntasks, T* L, T* dinv, double* logpiv, int* err, cudaStream_t st) {
   if (ntasks <= 0) return;
-  if constexpr (sizeof(T) == sizeof(float)) {
-    potrf_df_kernel<<<ntasks, 256, 0, st>>>(tasks, L, dinv, logpiv, err);
-  } else {
-    potrf_kernel<T><<<ntasks, 256, 0, st>>>(tasks, L, dinv, logpiv, err);
-  }
+  static const bool attr = [] {  // once, thread-safely
+    cudaFuncSetAttribute(potrf_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, potrf_smem<T>());
+    return true;
+  }();
+  (void)attr;
+  potrf_kernel<T><<<ntasks, 256, potrf_smem<T>(), st>>>(tasks, L, dinv, logpiv, err);
 }
 template void launch_potrf<double>(const DiagTask*, int, double*, double*, double*, int*, cudaStream_t);
 template void launch_potrf<float>(const DiagTask*, int, float*, float*, double*, int*, cudaStream_t);

@@ -22,6 +22,12 @@ struct GemmTask {
   int pair = 0;
 };
 
+// an integer constant as a type (selects a kernel's template argument in a lambda)
+template <int N>
+struct IntC {
+  static constexpr int value = N;
+};
+
 enum GemmMode { kSub = 0, kStore = 1, kNegStore = 2, kAdd = 3 };
 enum GemmLayout { kRow = 0, kCol = 1 };
 

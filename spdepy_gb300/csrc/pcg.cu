@@ -492,11 +492,6 @@ __global__ void obs32_kernel(const double* __restrict__ obs, double tau, float* 
   if (k < n) o32[k] = float(tau * obs[k]);
 }
 
-template <int V>
-struct IntC {
-  static constexpr int value = V;
-};
-
 // FP32 vectors of the solver hold their columns in groups of four (four values per
 // node side by side, one 16-byte access), then a group of two and single
 // columns; `packed` false keeps every column by itself (IC(0)).  Column c of
