@@ -49,50 +49,81 @@ constexpr int kNotFinite = 1 << 20;                   // row exponent of a row t
 // ------------------------------------------------------------------ split
 // Eight CTAs per 64-row tile, a warp per row: the row's exponent from its largest
 // magnitude, then eight values per lane into their seven digits (16-byte stores).
+// Rows of up to 512 values are held in registers between the two steps, longer ones
+// read again (from L1 / L2).  Bound: latency for the short rows, memory (8 bytes read,
+// 14 written per value) for large operands.
+__device__ __forceinline__ void split_load(const double* x, int k0, int k, bool vec, double (&v)[8]) {
+  if (vec && k0 + 8 <= k) {
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) *reinterpret_cast<double2*>(v + u) = *reinterpret_cast<const double2*>(x + k0 + u);
+  } else {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = k0 + u < k ? x[k0 + u] : 0.0;
+  }
+}
+__device__ __forceinline__ unsigned exponent_field(double v) {
+  return unsigned((__double_as_longlong(v) >> 52) & 0x7FF);
+}
+// eight values to digits; field: the row's largest exponent field (at least 1)
+__device__ __forceinline__ void split_store(const double (&v)[8], int field, bool finite, uint8_t* dst, int k0) {
+  uint32_t out[kDigits][4];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    long long F = 0;  // round(x 2^(55 - e))
+    if (finite) {
+      const long long b = __double_as_longlong(v[u]);
+      const int f = int((b >> 52) & 0x7FF);
+      const long long m = (b & 0xFFFFFFFFFFFFFll) | (f ? 1ll << 52 : 0ll);
+      const int sh = max(f, 1) - field + 2;
+      if (sh >= 0) F = m << sh;
+      else if (sh >= -54) F = (m + (1ll << (-sh - 1))) >> -sh;
+      if (b < 0) F = -F;
+    }
+#pragma unroll
+    for (int s = kDigits - 1; s >= 0; --s) {
+      const int d = s > 0 ? int(int8_t(F & 0xFF)) : int(F);
+      F = (F - d) >> 8;
+      // d as a float by the spacing of floats near 1.5 2^23 (no conversion unit); exact in bf16
+      const uint32_t h = __float_as_uint(__fsub_rn(__uint_as_float(0x4B400000u + unsigned(d)), 12582912.0f)) >> 16;
+      if (u & 1) out[s][u >> 1] |= h << 16;
+      else out[s][u >> 1] = h;
+    }
+  }
+  uint8_t* q = dst + int64_t(k0 >> 5) * kChunkBytes + ((k0 >> 3) & 3) * 128;
+#pragma unroll
+  for (int s = 0; s < kDigits; ++s)
+    *reinterpret_cast<uint4*>(q + s * kBlkBytes) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
+}
+
 __global__ void __launch_bounds__(256) emu_split_kernel(const EmuSplit* __restrict__ tasks, const double* Ab,
                                                         const double* Bb, uint8_t* __restrict__ planes,
                                                         int* __restrict__ exps) {
   const EmuSplit tk = tasks[blockIdx.x >> 3];
-  const double* X = (tk.buf ? Bb : Ab) + tk.src;
   const int lane = threadIdx.x & 31, r = int(blockIdx.x & 7) * 8 + int(threadIdx.x >> 5);
-  if (r < tk.rows) {
-    const double* x = X + int64_t(r) * tk.ld;
-    unsigned top = 0;  // largest exponent field
-    for (int k = lane; k < tk.k; k += 32)
-      top = max(top, unsigned((__double_as_longlong(x[k]) >> 52) & 0x7FF));
-    top = __reduce_max_sync(0xffffffffu, top);
-    const bool finite = top != 0x7FF;
-    const int field = max(int(top), 1);
-    if (lane == 0) exps[tk.exp + r] = finite ? field - 1022 : kNotFinite;
-    uint8_t* dst = planes + tk.dst + (r >> 3) * 512 + (r & 7) * 16;
-    for (int k0 = 8 * lane; k0 < 32 * tk.nch; k0 += 256) {
-      uint32_t out[kDigits][4];
+  if (r >= tk.rows) return;
+  const double* x = (tk.buf ? Bb : Ab) + tk.src + int64_t(r) * tk.ld;
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  uint8_t* dst = planes + tk.dst + (r >> 3) * 512 + (r & 7) * 16;
+  double v[2][8];
+  unsigned top = 0;  // largest exponent field
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        long long F = 0;  // round(x 2^(55 - e))
-        if (k0 + u < tk.k && finite) {
-          const long long b = __double_as_longlong(x[k0 + u]);
-          const int f = int((b >> 52) & 0x7FF);
-          const long long m = (b & 0xFFFFFFFFFFFFFll) | (f ? 1ll << 52 : 0ll);
-          const int sh = max(f, 1) - field + 2;
-          if (sh >= 0) F = m << sh;
-          else if (sh >= -54) F = (m + (1ll << (-sh - 1))) >> -sh;
-          if (b < 0) F = -F;
-        }
+  for (int h = 0; h < 2; ++h) {
+    split_load(x, 8 * lane + 256 * h, tk.k, vec, v[h]);
 #pragma unroll
-        for (int s = kDigits - 1; s >= 0; --s) {
-          const int d = s > 0 ? int(int8_t(F & 0xFF)) : int(F);
-          F = (F - d) >> 8;
-          const uint32_t h = __float_as_uint(float(d)) >> 16;  // exact in bf16
-          if (u & 1) out[s][u >> 1] |= h << 16;
-          else out[s][u >> 1] = h;
-        }
-      }
-      uint8_t* q = dst + int64_t(k0 >> 5) * kChunkBytes + ((k0 >> 3) & 3) * 128;
+    for (int u = 0; u < 8; ++u) top = max(top, exponent_field(v[h][u]));
+  }
+#pragma unroll 4
+  for (int k = 512 + lane; k < tk.k; k += 32) top = max(top, exponent_field(x[k]));
+  top = __reduce_max_sync(0xffffffffu, top);
+  const bool finite = top != 0x7FF;
+  const int field = max(int(top), 1);
+  if (lane == 0) exps[tk.exp + r] = finite ? field - 1022 : kNotFinite;
 #pragma unroll
-      for (int s = 0; s < kDigits; ++s)
-        *reinterpret_cast<uint4*>(q + s * kBlkBytes) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
-    }
+  for (int h = 0; h < 2; ++h)
+    if (8 * lane + 256 * h < 32 * tk.nch) split_store(v[h], field, finite, dst, 8 * lane + 256 * h);
+  for (int k0 = 512 + 8 * lane; k0 < 32 * tk.nch; k0 += 256) {
+    split_load(x, k0, tk.k, vec, v[0]);
+    split_store(v[0], field, finite, dst, k0);
   }
 }
 

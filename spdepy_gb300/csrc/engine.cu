@@ -37,10 +37,12 @@ constexpr int kTcMinKUpdate = 64;  // ... for the rank-64 updates inside a facto
 // shortest K of a cluster-pair task: below it the pair's per-task set-up and
 // pipeline fill outweigh its throughput, and the single-CTA kernel is faster
 constexpr int kPairMinK = 256;
-// Smallest FP64 product (rows, columns, k) on the tensor cores: a CUDA-core 64 x 64
-// tile takes about 1 us per k value (the FP64 pipe), a tensor-core tile a fixed 10 us
-// with its share of the split, and 2.3 us per 32 values.
-constexpr int kEmuMin = 32;
+// Smallest FP64 product on the tensor cores: a CUDA-core 64 x 64 tile takes about 1 us
+// per k value (the FP64 pipe), a tensor-core tile a fixed 10 us with its share of the
+// split and 2.3 us per 32 values.  Measured with the limit at 32 (all sizes), 16 and
+// (8, k 4): 17.5, 17.0 and 16.6 ms per FP64 evaluation at 30 x 30 x 24, 55.8, 51.1
+// and 51.0 ms at 48 x 48 x 24 (the leaf fronts' narrow products).
+constexpr int kEmuMin = 8, kEmuMinK = 4;
 enum { KT_NONE = 0, KT_A_UPPER, KT_B_LOWER, KT_BOTH_UPPER };
 constexpr int kPanel = 512;   // panel width of the two-level blocked factorisation
 
@@ -281,7 +283,7 @@ struct Builder {
     if (m <= 0 || n <= 0 || k <= 0) return;
     const Op& op = s.ops.back();
     if (emu_ok && arow == lda && brow == ldb && op.al == kRow && op.bl == kRow && m >= kEmuMin && n >= kEmuMin &&
-        k >= kEmuMin && i_start == 0) {
+        k >= kEmuMinK && i_start == 0) {
       emu_tiles(a, lda, b, ldb, c, ldc, m, n, k, lower, kt);
       return;
     }
