@@ -1,4 +1,4 @@
-// Shared-memory barriers and tensor-core helpers of the tcgen05 kernels.
+// Asynchronous copies, shared-memory barriers and tensor-core helpers.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -37,6 +37,14 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 
 __device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
 }  // namespace spde

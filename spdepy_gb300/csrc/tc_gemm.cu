@@ -43,6 +43,7 @@ constexpr int kPlane = 128 * 32 * 4;       // one 128 x 32 FP32 operand plane (1
 constexpr int kStages = 4;                 // stage = raw A, raw B, residual B
 constexpr int kStageBytes = 3 * kPlane;
 constexpr int kSmem = kStages * kStageBytes + 1024;
+constexpr int kTileLd = kTN + 4;            // row stride of the accumulator in shared memory: 16-byte rows, 4 banks apart
 constexpr int kASlot0 = 128, kASlotCols = 64;  // TMEM: accumulator 0-127, A slot s at 128 + 64 s
 constexpr int kTmemCols = 512;             // power of two >= 128 + kStages * 64
 constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s
@@ -78,12 +79,6 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       "r"(tmem_a), "l"(b), "r"(kIdesc), "r"(acc));
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
 // the mbarrier receives one arrival when every cp.async this thread issued so far has landed
 __device__ __forceinline__ void cp_async_arrive(uint32_t mbar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(mbar) : "memory");
@@ -184,18 +179,108 @@ __device__ __forceinline__ void a_to_tmem(const uint8_t* raw, int row, int h, ui
   tmem_st16(taddr + 32 + 16 * h, lo);
 }
 
-template <int MODE, int AL, int BL>
-__global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const GemmTask* __restrict__ tasks, const float* Ab,
+// ------------------------------------------------------------------ epilogue
+// The accumulator is read one row per lane, which as a global access pattern would
+// touch 32 rows 16 bytes at a time; it goes through shared memory instead (the
+// stages are free once the MMAs are done), and whole rows are written, and read
+// for the updating modes, 512 bytes per warp instruction.  Measured: rank-512 panel
+// updates on pairs at 100 x 100 x 24 215 us a launch (239 with 16 bytes of 32 rows per
+// instruction), rank-128 updates on single CTAs 34 (41).
+// 32 accumulator columns of this lane's row to shared memory
+__device__ __forceinline__ void acc_to_smem(uint32_t taddr, float* dst) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
+        "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
+        "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 32; j += 4)
+    *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
+                                                      __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+}
+template <int MODE>
+__device__ __forceinline__ float apply_mode(float old, float v) {
+  if (MODE == kSub) return old - v;
+  if (MODE == kStore) return v;
+  if (MODE == kNegStore) return -v;
+  return old + v;
+}
+// The C tile of an updating product into L2 while the mainloop runs
+template <int COLS>
+__device__ __forceinline__ void prefetch_c(const float* C, int64_t ldc, int m, int n, int ltid) {
+  constexpr int kLines = COLS / 32;
+  for (int e = ltid; e < m * kLines; e += kLoad) {
+    const int r = e / kLines, c = 32 * (e - r * kLines);
+    if (c < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + r * ldc + c));
+  }
+}
+// Rows warp, warp + NW, ... of an m x n tile (rows of `ld` floats in shared memory,
+// COLS of them computed) into C, four rows in flight
+template <int MODE, int COLS, int NW>
+__device__ __forceinline__ void rows_to_global(const float* sm, int ld, float* C, int64_t ldc, int m, int n, int warp,
+                                               int lane) {
+  constexpr bool kRead = MODE == kSub || MODE == kAdd;
+  const bool vec = ((reinterpret_cast<uintptr_t>(C) & 15) == 0) && (ldc & 3) == 0;
+#pragma unroll 1
+  for (int r0 = warp; r0 < m; r0 += 4 * NW) {
+#pragma unroll
+    for (int c0 = 0; c0 < COLS; c0 += 128) {
+      const int c = c0 + 4 * lane;
+      if (vec && c0 + 128 <= n) {
+        float4 old[4];
+        if (kRead) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (r0 + u * NW < m) old[u] = *reinterpret_cast<const float4*>(C + (r0 + u * NW) * ldc + c);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (r0 + u * NW < m) {
+            const float4 v = *reinterpret_cast<const float4*>(sm + (r0 + u * NW) * ld + c);
+            *reinterpret_cast<float4*>(C + (r0 + u * NW) * ldc + c) =
+                make_float4(apply_mode<MODE>(old[u].x, v.x), apply_mode<MODE>(old[u].y, v.y),
+                            apply_mode<MODE>(old[u].z, v.z), apply_mode<MODE>(old[u].w, v.w));
+          }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {  // one column per lane
+          const int cj = c0 + lane + 32 * j;
+          float old[4];
+          if (kRead) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (r0 + u * NW < m && cj < n) old[u] = C[(r0 + u * NW) * ldc + cj];
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (r0 + u * NW < m && cj < n)
+              C[(r0 + u * NW) * ldc + cj] = apply_mode<MODE>(old[u], sm[(r0 + u * NW) * ld + cj]);
+        }
+      }
+    }
+  }
+}
+
+// ST stages: four with one CTA per SM, or two with two CTAs per SM, whose loads,
+// conversions, MMAs and epilogues then overlap.
+template <int MODE, int AL, int BL, int ST>
+__global__ void __launch_bounds__(kThreads, ST == 2 ? 2 : 1) tc_gemm_kernel(const GemmTask* __restrict__ tasks, const float* Ab,
                                                               const float* Bb, float* Cb, unsigned long long wait_ns) {
-  // Three roles hand chunk t (stage s = t % kStages) along through mbarriers:
-  //   loaders (warps 8-11): wait consumed[s] (MMAs of chunk t - kStages done),
+  // Three roles hand chunk t (stage s = t % ST) along through mbarriers:
+  //   loaders (warps 8-11): wait consumed[s] (MMAs of chunk t - ST done),
   //     issue the cp.async copies of A and B, arrive on full[s] when they land;
   //   converters (warps 0-7): wait full[s], write A hi/lo into TMEM slot s and
   //     the B hi/lo planes, arrive on ready[s]; afterwards they run the epilogue;
   //   MMA issuer (warp 12, one lane): wait ready[s], issue the chunk's 12 MMAs,
   //     commit to consumed[s]; a final commit arrives on done.
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t full[kStages], ready[kStages], consumed[kStages], done;
+  __shared__ uint64_t full[ST], ready[ST], consumed[ST], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag, mma_issued;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -208,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const GemmTask* __
   const bool bvec = ((reinterpret_cast<uintptr_t>(B) & 15) == 0) && ((tk.ldb & 3) == 0);
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < ST; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[s])), "r"(kLoad));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&ready[s])), "r"(kConv));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&consumed[s])));
@@ -220,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const GemmTask* __
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "n"(kTmemCols));
+                 "n"(ST == 2 ? 256 : 512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     asm volatile("tcgen05.fence::before_thread_sync;");
   }
@@ -249,8 +334,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const GemmTask* __
     // ---------------- converters (two groups on alternate chunks), then the epilogue
     const int g = tid / kConv, ct = tid - g * kConv;
     for (int t = g; t < nk; t += kGroups) {
-      const int s = t % kStages;
-      if (!wait(&full[s], uint32_t((t / kStages) & 1), true, wait_ns)) break;
+      const int s = t % ST;
+      if (!wait(&full[s], uint32_t((t / ST) & 1), true, wait_ns)) break;
       uint8_t* st = smem + s * kStageBytes;
       // warp w reaches TMEM lanes 32 (w % 4) ..; the group's warps 0-3 take k 0-15, warps 4-7 k 16-31
       a_to_tmem(st, ct & 127, ct >> 7,
@@ -261,64 +346,29 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const GemmTask* __
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(smem_u32(&ready[s]));
     }
-    const bool fin = nk == 0 || wait(&done, 0u, true, wait_ns);
+    const bool fin = nk > 0 && wait(&done, 0u, true, wait_ns);
+    float* tile = reinterpret_cast<float*>(smem);
     if (fin) {
       asm volatile("tcgen05.fence::after_thread_sync;");
       // warp w reads lanes 32 (w % 4) .. and accumulator columns kEpiCols (w / 4) ..
-      const int row = (warp & 3) * 32 + lane;
+      const uint32_t ta = tmem + (uint32_t((warp & 3) * 32) << 16);
 #pragma unroll
       for (int c = 0; c < kEpiCols / 32; ++c) {
         const int col0 = (warp >> 2) * kEpiCols + c * 32;
-        uint32_t r[32];
-        const uint32_t ta = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(col0);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-              "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-              "=r"(r[30]), "=r"(r[31])
-            : "r"(ta));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row < tk.m && nk > 0 && col0 < tk.n) {
-          float* dst = C + int64_t(row) * tk.ldc + col0;
-          const bool v4 = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) && col0 + 32 <= tk.n;
-          if (v4) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float4 v = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                                     __uint_as_float(r[j + 3]));
-              float4* d4 = reinterpret_cast<float4*>(dst + j);
-              if (MODE == kStore) { *d4 = v; }
-              else if (MODE == kNegStore) { *d4 = make_float4(-v.x, -v.y, -v.z, -v.w); }
-              else {
-                float4 o = *d4;
-                if (MODE == kSub) *d4 = make_float4(o.x - v.x, o.y - v.y, o.z - v.z, o.w - v.w);
-                else *d4 = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (col0 + j >= tk.n) break;
-              const float v = __uint_as_float(r[j]);
-              if (MODE == kSub) dst[j] -= v;
-              else if (MODE == kStore) dst[j] = v;
-              else if (MODE == kNegStore) dst[j] = -v;
-              else dst[j] += v;
-            }
-          }
-        }
+        acc_to_smem(ta + uint32_t(col0), tile + ((warp & 3) * 32 + lane) * kTileLd + col0);
       }
     }
+    // every converter warp comes here, also after a failed wait
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(kGroups * kConv) : "memory");
+    if (fin) rows_to_global<MODE, kTN, kGroups * kConv / 32>(tile, kTileLd, C, tk.ldc, tk.m, tk.n, warp, lane);
   } else if (warp < (kGroups * kConv + kLoad) / 32) {
     // ---------------- loaders
     const int ltid = tid - kGroups * kConv;
+    if (MODE == kSub || MODE == kAdd) prefetch_c<kTN>(C, tk.ldc, tk.m, tk.n, ltid);
     for (int t = 0; t < nk; ++t) {
-      const int s = t % kStages;
-      // stage s last held chunk t - kStages, read by its MMAs (B) and converters (A)
-      if (t >= kStages && !wait(&consumed[s], uint32_t(((t - kStages) / kStages) & 1), true, wait_ns)) break;
+      const int s = t % ST;
+      // stage s last held chunk t - ST, read by its MMAs (B) and converters (A)
+      if (t >= ST && !wait(&consumed[s], uint32_t(((t - ST) / ST) & 1), true, wait_ns)) break;
       const uint32_t d0 = smem_u32(smem + s * kStageBytes);
       stage_async<AL, kLoad>(A, tk.lda, tk.m, t * kTK, tk.k, avec, d0, ltid);
       stage_async<BL, kLoad>(B, tk.ldb, tk.n, t * kTK, tk.k, bvec, d0 + kPlane, ltid);
@@ -328,8 +378,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const GemmTask* __
   } else if (lane == 0) {
     // ---------------- MMA issuer
     for (int t = 0; t < nk; ++t) {
-      const int s = t % kStages;
-      if (!wait(&ready[s], uint32_t((t / kStages) & 1), true, wait_ns)) break;
+      const int s = t % ST;
+      if (!wait(&ready[s], uint32_t((t / ST) & 1), true, wait_ns)) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
       const uint32_t rb = smem_u32(smem + s * kStageBytes + kPlane), lb = rb + kPlane;
       const uint32_t ah = tmem + uint32_t(kASlot0 + s * kASlotCols), al = ah + 32;
@@ -354,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const GemmTask* __
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(ST == 2 ? 256 : 512));
 }
 
 // ---------------------------------------------------------------------------
@@ -385,6 +435,7 @@ constexpr int kPairASlot0 = 256;  // TMEM: accumulator columns 0-255, A slot s a
 constexpr int kPairGroups = 2;     // converter groups of the pair kernel (group g takes chunks t = g mod 2)
 constexpr int kPairThreads = kPairGroups * kConv + kLoad + 32;  // warps 0-15 converters, 16-19 loaders, 20 MMA
 constexpr int kPairEpiCols = 256 / (kPairGroups * kConv / 128);  // accumulator columns per epilogue warp
+constexpr int kPairTileLd = 256 + 4;  // row stride of the accumulator in shared memory: 16-byte rows, 4 banks apart
 constexpr uint32_t kIdescPair = (1u << 4) | (2u << 7) | (2u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -560,60 +611,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&ready[s]), 0));
     }
     const bool fin = nk > 0 && wait(&done, 0u, true, wait_ns);
+    float* tile = reinterpret_cast<float*>(smem);
     if (fin) {
       asm volatile("tcgen05.fence::after_thread_sync;");
       // warp w reads lanes 32 (w % 4) .. and accumulator columns kPairEpiCols (w / 4) ..
-      const int row = (warp & 3) * 32 + lane;
-      const int grow = row0 + row;
 #pragma unroll 1
       for (int c = 0; c < kPairEpiCols / 32; ++c) {
         const int col0 = (warp >> 2) * kPairEpiCols + c * 32;
-        uint32_t r[32];
-        const uint32_t ta = tmem + lane_base + uint32_t(col0);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-              "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-              "=r"(r[30]), "=r"(r[31])
-            : "r"(ta));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (grow < tk.m && col0 < tk.n) {
-          float* dst = Cb + tk.c + int64_t(grow) * tk.ldc + col0;
-          const bool v4 = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) && col0 + 32 <= tk.n;
-          if (v4) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float4 v = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                                     __uint_as_float(r[j + 3]));
-              float4* d4 = reinterpret_cast<float4*>(dst + j);
-              if (MODE == kStore) { *d4 = v; }
-              else if (MODE == kNegStore) { *d4 = make_float4(-v.x, -v.y, -v.z, -v.w); }
-              else {
-                float4 o = *d4;
-                if (MODE == kSub) *d4 = make_float4(o.x - v.x, o.y - v.y, o.z - v.z, o.w - v.w);
-                else *d4 = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (col0 + j >= tk.n) break;
-              const float v = __uint_as_float(r[j]);
-              if (MODE == kSub) dst[j] -= v;
-              else if (MODE == kStore) dst[j] = v;
-              else if (MODE == kNegStore) dst[j] = -v;
-              else dst[j] += v;
-            }
-          }
-        }
+        acc_to_smem(tmem + lane_base + uint32_t(col0), tile + ((warp & 3) * 32 + lane) * kPairTileLd + col0);
       }
     }
+    // every converter warp comes here, also after a failed wait
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(kPairGroups * kConv) : "memory");
+    if (fin && am > 0)
+      rows_to_global<MODE, 256, kPairGroups * kConv / 32>(tile, kPairTileLd, Cb + tk.c + int64_t(row0) * tk.ldc, tk.ldc,
+                                                          min(am, 128), tk.n, warp, lane);
   } else if (warp < (kPairGroups * kConv + kLoad) / 32) {
     // ---------------- loaders: TMA boxes (one elected thread) and / or cp.async
     const int ltid = tid - kPairGroups * kConv;
+    if ((MODE == kSub || MODE == kAdd) && am > 0)
+      prefetch_c<256>(Cb + tk.c + int64_t(row0) * tk.ldc, tk.ldc, min(am, 128), tk.n, ltid);
     int issued = 0;  // chunks whose TMA boxes this thread (ltid 0) issued
     for (int t = 0; t < nk; ++t) {
       const int s = t % kStages;
@@ -694,17 +711,27 @@ void launch_pair(const GemmTask* t, int n, const CUtensorMap* maps, const float*
   tc_pair_kernel<MODE><<<2 * n, kPairThreads, kSmem, st>>>(t, maps, A, B, C, wait_ns);
 }
 
-template <int MODE, int AL, int BL>
-void launch_one(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st,
-                unsigned long long wait_ns) {
+template <int MODE, int AL, int BL, int ST>
+void launch_stages(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st,
+                   unsigned long long wait_ns) {
   // once per instantiation; a function-local static is initialised thread-safely
   // (the second log-likelihood pipeline launches from its own host thread)
+  constexpr int smem = ST * kStageBytes + 1024;
   static const bool attr = [] {
-    cudaFuncSetAttribute(tc_gemm_kernel<MODE, AL, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    cudaFuncSetAttribute(tc_gemm_kernel<MODE, AL, BL, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     return true;
   }();
   (void)attr;
-  tc_gemm_kernel<MODE, AL, BL><<<n, kThreads, kSmem, st>>>(t, A, B, C, wait_ns);
+  tc_gemm_kernel<MODE, AL, BL, ST><<<n, kThreads, smem, st>>>(t, A, B, C, wait_ns);
+}
+// Four stages while every tile has an SM to itself (a shorter wait per tile), two
+// CTAs per SM beyond.  Measured: launches of up to 152 tiles 17.4 against 20.2 us, the
+// rank-128 updates at 100 x 100 x 24 (300 tiles a launch) 38.6 against 33.6 us.
+template <int MODE, int AL, int BL>
+void launch_one(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st,
+                unsigned long long wait_ns) {
+  if (n <= 152) launch_stages<MODE, AL, BL, 4>(t, n, A, B, C, st, wait_ns);
+  else launch_stages<MODE, AL, BL, 2>(t, n, A, B, C, st, wait_ns);
 }
 
 template <int MODE>
