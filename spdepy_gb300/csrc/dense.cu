@@ -9,28 +9,19 @@
 #include <stdlib.h>
 
 #include "kernels.cuh"
+#include "tc_common.cuh"
 
 namespace spde {
 
 // --------------------------------------------------------------------- GEMM
-template <typename T>
-struct GemmCfg;
-template <>
-struct GemmCfg<double> {
-  static constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
-};
-template <>
-struct GemmCfg<float> {
-  static constexpr int BM = 128, BN = 128, BK = 16, TM = 8, TN = 8;
-};
-
-// A, B and C may alias (in-place triangular solves): every block reads all of
-// its A and B tiles before its epilogue writes C, and blocks own disjoint C tiles.
-template <typename T, int MODE, int AL, int BL>
-__global__ void __launch_bounds__(256) gemm_kernel(const GemmTask* __restrict__ tasks, const T* Ab, const T* Bb,
-                                                   T* Cb) {
-  using C = GemmCfg<T>;
-  constexpr int BM = C::BM, BN = C::BN, BK = C::BK, TM = C::TM, TN = C::TN;
+// Tiled product on the CUDA cores, FP64 storage.  A, B and C may alias (in-place
+// triangular solves): every block reads all of its A and B tiles before its
+// epilogue writes C, and blocks own disjoint C tiles.
+template <int MODE, int AL, int BL>
+__global__ void __launch_bounds__(256) gemm64_kernel(const GemmTask* __restrict__ tasks, const double* Ab,
+                                                     const double* Bb, double* Cb) {
+  using T = double;
+  constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
   __shared__ T As[BK][BM + 4];
   __shared__ T Bs[BK][BN + 4];
   const GemmTask tk = tasks[blockIdx.x];
@@ -95,12 +86,163 @@ __global__ void __launch_bounds__(256) gemm_kernel(const GemmTask* __restrict__ 
   }
 }
 
+// The same in FP32: 128 x 128 tiles, 8 x 8 entries per thread, K in chunks of 32
+// copied asynchronously into one of two shared-memory buffers while the other is
+// used.  An operand lies in shared memory as in memory: rows of 32 k values (row
+// layout, read two k values at a time) or, per k, rows side by side (column layout);
+// a warp computes 32 x 64 entries, warps outside the task's rows or columns skip the
+// arithmetic.  Every entry adds its products in the order of k.  Same aliasing rule
+// as above.  Bound: the FP32 pipe for many tiles, latency for few.
+constexpr int kSgBk = 32, kSgRow = kSgBk + 4, kSgCol = 128 + 4;  // row strides: 16-byte rows, 4 banks apart
+constexpr int kSgOp = 128 * kSgRow;                              // floats of one operand's buffer (either layout)
+static_assert(kSgBk * kSgCol <= kSgOp, "column layout fits");
+constexpr int kSgSmem = 4 * kSgOp * int(sizeof(float));
+
+template <int LAYOUT>
+__device__ __forceinline__ void sg_stage(const float* X, int ld, int rows, int k0, int K, bool vec, float* sh, int tid) {
+  const uint32_t s0 = smem_u32(sh);
+  if (vec) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = tid + 256 * u;
+      const int r = LAYOUT == kRow ? e >> 3 : 4 * (e & 31), k = LAYOUT == kRow ? 4 * (e & 7) : e >> 5;
+      const int left = LAYOUT == kRow ? (r < rows ? K - k0 - k : 0) : (k0 + k < K ? rows - r : 0);
+      const int bytes = 4 * max(0, min(4, left));
+      const float* src = LAYOUT == kRow ? X + int64_t(r) * ld + k0 + k : X + int64_t(k0 + k) * ld + r;
+      cp_async16(s0 + 4 * (LAYOUT == kRow ? r * kSgRow + k : k * kSgCol + r), bytes ? src : X, bytes);
+    }
+  } else {
+#pragma unroll 4
+    for (int u = 0; u < 16; ++u) {
+      const int e = tid + 256 * u;
+      const int r = LAYOUT == kRow ? e >> 5 : e & 127, k = LAYOUT == kRow ? e & 31 : e >> 7;
+      const bool ok = r < rows && k0 + k < K;
+      const float* src = LAYOUT == kRow ? X + int64_t(r) * ld + k0 + k : X + int64_t(k0 + k) * ld + r;
+      cp_async4(s0 + 4 * (LAYOUT == kRow ? r * kSgRow + k : k * kSgCol + r), ok ? src : X, ok ? 4 : 0);
+    }
+  }
+}
+// index of entry q (of 8) along an operand's rows for position `p` of P in the warp
+template <int LAYOUT, int P>
+__device__ __forceinline__ int sg_row(int p, int q) { return LAYOUT == kRow ? p + P * q : 8 * p + q; }
+// k values kk, kk + 1 of the thread's eight rows
+template <int LAYOUT, int P>
+__device__ __forceinline__ void sg_frag(const float* sh, int base, int p, int kk, float (&f)[2][8]) {
+  if (LAYOUT == kRow) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float2 v = *reinterpret_cast<const float2*>(sh + (base + p + P * q) * kSgRow + kk);
+      f[0][q] = v.x;
+      f[1][q] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float4*>(&f[e][4 * h]) =
+            *reinterpret_cast<const float4*>(sh + (kk + e) * kSgCol + base + 8 * p + 4 * h);
+  }
+}
+
+template <int MODE, int AL, int BL>
+__global__ void __launch_bounds__(256, 2) gemm32_kernel(const GemmTask* __restrict__ tasks, const float* Ab,
+                                                        const float* Bb, float* Cb) {
+  extern __shared__ __align__(16) float sgm[];
+  const GemmTask tk = tasks[blockIdx.x];
+  const float* A = Ab + tk.a;
+  const float* B = Bb + tk.b;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wr = 32 * (warp & 3), wc = 64 * (warp >> 2), ly = lane >> 3, lx = lane & 7;
+  const bool avec = ((reinterpret_cast<uintptr_t>(A) & 15) == 0) && (tk.lda & 3) == 0;
+  const bool bvec = ((reinterpret_cast<uintptr_t>(B) & 15) == 0) && (tk.ldb & 3) == 0;
+  const bool active = wr < tk.m && wc < tk.n;
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  const int nk = (tk.k + kSgBk - 1) / kSgBk;
+  auto stage = [&](int t) {
+    float* buf = sgm + (t & 1) * 2 * kSgOp;
+    sg_stage<AL>(A, tk.lda, tk.m, t * kSgBk, tk.k, avec, buf, tid);
+    sg_stage<BL>(B, tk.ldb, tk.n, t * kSgBk, tk.k, bvec, buf + kSgOp, tid);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage(0);
+  for (int t = 0; t < nk; ++t) {
+    if (t + 1 < nk) {
+      stage(t + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    if (active) {
+      const float* As = sgm + (t & 1) * 2 * kSgOp;
+      const float* Bs = As + kSgOp;
+      const int kn = min(kSgBk, (tk.k - t * kSgBk + 1) & ~1);
+#pragma unroll 4
+      for (int kk = 0; kk < kn; kk += 2) {
+        float a[2][8], b[2][8];
+        sg_frag<AL, 4>(As, wr, ly, kk, a);
+        sg_frag<BL, 8>(Bs, wc, lx, kk, b);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[e][i], b[e][j], acc[i][j]);
+      }
+    }
+    __syncthreads();
+  }
+  if (!active) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = wr + sg_row<AL, 4>(ly, i);
+    if (r >= tk.m) continue;
+    float* dst = Cb + tk.c + int64_t(r) * tk.ldc;
+    float old[8];
+    if (MODE == kSub || MODE == kAdd) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c = wc + sg_row<BL, 8>(lx, j);
+        old[j] = c < tk.n ? dst[c] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int c = wc + sg_row<BL, 8>(lx, j);
+      if (c >= tk.n) continue;
+      if (MODE == kSub) dst[c] = old[j] - acc[i][j];
+      else if (MODE == kStore) dst[c] = acc[i][j];
+      else if (MODE == kNegStore) dst[c] = -acc[i][j];
+      else dst[c] = old[j] + acc[i][j];
+    }
+  }
+}
+
+template <typename T, int MODE, int AL, int BL>
+static void gemm_layout(const GemmTask* t, int n, const T* A, const T* B, T* C, cudaStream_t st) {
+  if constexpr (sizeof(T) == sizeof(float)) {
+    static const bool attr = [] {  // once, thread-safely
+      cudaFuncSetAttribute(gemm32_kernel<MODE, AL, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgSmem);
+      return true;
+    }();
+    (void)attr;
+    gemm32_kernel<MODE, AL, BL><<<n, 256, kSgSmem, st>>>(t, A, B, C);
+  } else {
+    gemm64_kernel<MODE, AL, BL><<<n, 256, 0, st>>>(t, A, B, C);
+  }
+}
+
 template <typename T, int MODE>
 static void gemm_mode(const GemmTask* t, int n, const T* A, const T* B, T* C, int al, int bl, cudaStream_t st) {
-  if (al == kRow && bl == kRow) gemm_kernel<T, MODE, kRow, kRow><<<n, 256, 0, st>>>(t, A, B, C);
-  else if (al == kRow && bl == kCol) gemm_kernel<T, MODE, kRow, kCol><<<n, 256, 0, st>>>(t, A, B, C);
-  else if (al == kCol && bl == kRow) gemm_kernel<T, MODE, kCol, kRow><<<n, 256, 0, st>>>(t, A, B, C);
-  else gemm_kernel<T, MODE, kCol, kCol><<<n, 256, 0, st>>>(t, A, B, C);
+  if (al == kRow && bl == kRow) gemm_layout<T, MODE, kRow, kRow>(t, n, A, B, C, st);
+  else if (al == kRow && bl == kCol) gemm_layout<T, MODE, kRow, kCol>(t, n, A, B, C, st);
+  else if (al == kCol && bl == kRow) gemm_layout<T, MODE, kCol, kRow>(t, n, A, B, C, st);
+  else gemm_layout<T, MODE, kCol, kCol>(t, n, A, B, C, st);
 }
 
 // ------------------------------------------------------------ narrow GEMM
