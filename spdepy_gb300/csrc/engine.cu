@@ -356,13 +356,19 @@ static void build_factor_schedule(const Symbolic& S, Schedule& sc, int TM, int T
       o.abuf = pc == 0 ? B_P0 : B_P1;
       o.cbuf = pd == 0 ? B_P0 : B_P1;
       o.depth = d;
+      // elements per block: 16k, down to 2k while the level has less than eight
+      // blocks per SM (a block's warps take its rows one after the other); row r
+      // holds r + 1 elements: 8 rows of the long rows, up to 128 of the short ones
+      // (16, two per warp, while SMs are idle)
+      int64_t total = 0;
+      for (int f : fr)
+        if (F[f].child[rank] >= 0) total += int64_t(F[F[f].child[rank]].nb) * F[F[f].child[rank]].nb / 2;
+      const int chunk = int(std::max<int64_t>(2048, std::min<int64_t>(16384, total / (8 * 152))));
       for (int f : fr) {
         int c = F[f].child[rank];
         if (c < 0 || F[c].nb == 0) continue;
-        // about 16k elements per block (row r holds r + 1): 8 rows of the long
-        // rows, up to 128 of the short ones
         for (int r0 = 0; r0 < F[c].nb;) {
-          const int rows = std::max(8, std::min(128, (16384 / (r0 + 1)) & ~7));
+          const int rows = std::max(8, std::min(chunk == 2048 ? 16 : 128, (chunk / (r0 + 1)) & ~7));
           const int r1 = std::min(F[c].nb, r0 + rows);
           sc.ext.push_back({c, r0, r1});
           o.nmax = std::max(o.nmax, r1);
