@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(256) gemm64_kernel(const GemmTask* __restrict_
   const T* B = Bb + tk.b;
   T* Cp = Cb + tk.c;
   const int tid = threadIdx.x;
+  chain_wait();
   const int tx = tid % (BN / TN);  // column group
   const int ty = tid / (BN / TN);  // row group
   T acc[TM][TN];
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(256, 2) gemm32_kernel(const GemmTask* __restri
     sg_stage<BL>(B, tk.ldb, tk.n, t * kSgBk, tk.k, bvec, buf + kSgOp, tid);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  chain_wait();
   stage(0);
   for (int t = 0; t < nk; ++t) {
     if (t + 1 < nk) {
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(256, 2) gemm32_kernel(const GemmTask* __restri
     }
     __syncthreads();
   }
+  chain_trigger();
   if (!active) return;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -231,9 +234,9 @@ static void gemm_layout(const GemmTask* t, int n, const T* A, const T* B, T* C, 
       return true;
     }();
     (void)attr;
-    gemm32_kernel<MODE, AL, BL><<<n, 256, kSgSmem, st>>>(t, A, B, C);
+    launch_chained(gemm32_kernel<MODE, AL, BL>, n, 256, kSgSmem, st, t, A, B, C);
   } else {
-    gemm64_kernel<MODE, AL, BL><<<n, 256, 0, st>>>(t, A, B, C);
+    launch_chained(gemm64_kernel<MODE, AL, BL>, n, 256, 0, st, t, A, B, C);
   }
 }
 
@@ -298,6 +301,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(const GemmTask* __restrict__ 
   T* C = Cb + tk.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = tk.n, m = tk.m;
+  chain_wait();
   if (AL == kRow) {
     // rows in batches of 8; warp w owns batches w and w + 8 (m <= 128); lanes
     // stride along k, 64 k values per step
@@ -473,6 +477,7 @@ __global__ void __launch_bounds__(256) panel64_kernel(const GemmTask* __restrict
   float* Bs = psm + ROWS * kPanelLd;   // Bs[j * kPanelLd + k] = B(j, k)
   const GemmTask tk = tasks[blockIdx.x / kSplit];
   const int row0 = int(blockIdx.x % kSplit) * ROWS, m = min(ROWS, tk.m - row0);
+  chain_wait();
   if (m <= 0) return;
   float* C = Cb + tk.c + int64_t(row0) * tk.ldc;
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
@@ -518,6 +523,7 @@ __global__ void __launch_bounds__(256) panel64_kernel(const GemmTask* __restrict
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r].w, b[c].w, acc[r][c]);
   }
+  chain_trigger();
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -540,7 +546,7 @@ static void panel64_rows(const GemmTask* t, int n, const float* A, const float* 
     return true;
   }();
   (void)attr;
-  panel64_kernel<MODE, ROWS><<<n * (128 / ROWS), 256, panel_smem(ROWS), st>>>(t, A, B, C);
+  launch_chained(panel64_kernel<MODE, ROWS>, n * (128 / ROWS), 256, panel_smem(ROWS), st, t, A, B, C);
 }
 template <int MODE>
 static void panel64_launch(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st) {
@@ -553,11 +559,11 @@ template <typename T, int MODE>
 static void gemv_mode(const GemmTask* t, int n, const T* A, const T* B, T* C, int al, int bl, cudaStream_t st,
                       int nmax) {
   if (nmax == 1) {
-    if (al == kRow) gemv_kernel<T, MODE, kRow, 1><<<n, 256, 0, st>>>(t, A, B, C, bl);
-    else gemv_kernel<T, MODE, kCol, 1><<<n, 256, 0, st>>>(t, A, B, C, bl);
+    if (al == kRow) launch_chained(gemv_kernel<T, MODE, kRow, 1>, n, 256, 0, st, t, A, B, C, bl);
+    else launch_chained(gemv_kernel<T, MODE, kCol, 1>, n, 256, 0, st, t, A, B, C, bl);
   } else {
-    if (al == kRow) gemv_kernel<T, MODE, kRow, kNarrowN><<<n, 256, 0, st>>>(t, A, B, C, bl);
-    else gemv_kernel<T, MODE, kCol, kNarrowN><<<n, 256, 0, st>>>(t, A, B, C, bl);
+    if (al == kRow) launch_chained(gemv_kernel<T, MODE, kRow, kNarrowN>, n, 256, 0, st, t, A, B, C, bl);
+    else launch_chained(gemv_kernel<T, MODE, kCol, kNarrowN>, n, 256, 0, st, t, A, B, C, bl);
   }
 }
 
@@ -792,6 +798,7 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
   const int w = tk.w;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ty = tid >> 4, tx = tid & 15;
   T* blk = L + tk.a;
+  chain_wait();
   Num r[4][4];                               // n <= m used
 #pragma unroll
   for (int m = 0; m < 4; ++m)
@@ -961,6 +968,7 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
     }
     __syncthreads();
   }
+  chain_trigger();
   T* dvp = dinv + tk.dinv;
 #pragma unroll
   for (int m = 0; m < 4; ++m)
@@ -979,7 +987,7 @@ void launch_potrf(const DiagTask* tasks, int ntasks, T* L, T* dinv, double* logp
     return true;
   }();
   (void)attr;
-  potrf_kernel<T><<<ntasks, 256, potrf_smem<T>(), st>>>(tasks, L, dinv, logpiv, err);
+  launch_chained(potrf_kernel<T>, ntasks, 256, potrf_smem<T>(), st, tasks, L, dinv, logpiv, err);
 }
 template void launch_potrf<double>(const DiagTask*, int, double*, double*, double*, int*, cudaStream_t);
 template void launch_potrf<float>(const DiagTask*, int, float*, float*, double*, int*, cudaStream_t);
@@ -1005,11 +1013,12 @@ __global__ void __launch_bounds__(256) extend_add_kernel(const ExtendTask* __res
   const DevFront c = fronts[tk.child];
   const DevFront p = fronts[c.parent];
   const int* rm = rmap + c.b_off;
-  const bool staged = tk.r1 <= kExtendSmemRows;
+  const bool staged = tk.r1 <= kExtendSmemRows;  // the row map is the plan's
   if (staged)
     for (int e = threadIdx.x; e < tk.r1; e += blockDim.x) srm[e] = rm[e];
   __syncthreads();
   const int* cm = staged ? srm : rm;
+  chain_wait();
   const T* U = Uc + c.u_off;
   T* P = L + p.p_off;
   T* Upar = Up + p.u_off;
@@ -1050,7 +1059,7 @@ void launch_extend_add(const ExtendTask* tasks, int ntasks, const DevFront* fron
                        T* L, T* U_parent, int max_r1, cudaStream_t st) {
   if (ntasks <= 0) return;
   const size_t smem = size_t(max_r1 <= kExtendSmemRows ? max_r1 : 0) * sizeof(int);
-  extend_add_kernel<T><<<ntasks, 256, smem, st>>>(tasks, fronts, rmap, U_child, L, U_parent);
+  launch_chained(extend_add_kernel<T>, ntasks, 256, smem, st, tasks, fronts, rmap, U_child, L, U_parent);
 }
 template void launch_extend_add<double>(const ExtendTask*, int, const DevFront*, const int*, const double*, double*,
                                         double*, int, cudaStream_t);

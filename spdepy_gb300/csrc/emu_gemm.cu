@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(256) emu_split_kernel(const EmuSplit* __restri
                                                         int* __restrict__ exps) {
   const EmuSplit tk = tasks[blockIdx.x >> 3];
   const int lane = threadIdx.x & 31, r = int(blockIdx.x & 7) * 8 + int(threadIdx.x >> 5);
+  chain_wait();
   if (r >= tk.rows) return;
   const double* x = (tk.buf ? Bb : Ab) + tk.src + int64_t(r) * tk.ld;
   const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask*
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
+  chain_wait();
   const int nk = tk.k1 - tk.k0;                       // chunks
   const int nw = (nk + kWindow - 1) / kWindow;        // windows between drains
 
@@ -252,6 +254,7 @@ __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask*
         }
       }
     }
+    chain_trigger();
     const int row = (warp & 3) * 32 + lane;
     if (ok && row < tk.m && col0 < tk.n) {
       const int ea = exps[tk.ea + row];
@@ -333,7 +336,7 @@ void launch_emu(const EmuTask* t, int n, const uint8_t* planes, const int* exps,
     return true;
   }();
   (void)attr;
-  emu_gemm_kernel<MODE><<<n, kEmuThreads, kEmuSmem, st>>>(t, planes, exps, C, err, wait_ns);
+  launch_chained(emu_gemm_kernel<MODE>, n, kEmuThreads, kEmuSmem, st, t, planes, exps, C, err, wait_ns);
 }
 
 }  // namespace
@@ -342,7 +345,7 @@ void launch_emu_gemm(const EmuSplit* splits, int nsplits, const EmuTask* tasks, 
                      const double* B, double* C, int mode, uint8_t* planes, int* exps, int* err, cudaStream_t st,
                      unsigned long long wait_ns) {
   if (ntasks <= 0) return;
-  emu_split_kernel<<<8 * nsplits, 256, 0, st>>>(splits, A, B, planes, exps);
+  launch_chained(emu_split_kernel, 8 * nsplits, 256, 0, st, splits, A, B, planes, exps);
   switch (mode) {
     case kSub: launch_emu<kSub>(tasks, ntasks, planes, exps, C, err, st, wait_ns); break;
     case kStore: launch_emu<kStore>(tasks, ntasks, planes, exps, C, err, st, wait_ns); break;

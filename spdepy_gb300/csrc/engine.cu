@@ -881,6 +881,7 @@ __global__ void __launch_bounds__(256) fwd_chain_kernel(const RowTask* __restric
   __shared__ T ys[64], acc[64];
   __shared__ int ticket, fail;
   const int tid = threadIdx.x, i = tid >> 2, q = tid & 3;
+  chain_wait();
   if (tid == 0) {
     ticket = int(atomicAdd(counter, 1u));
     fail = 0;
@@ -939,6 +940,7 @@ __global__ void __launch_bounds__(512) bwd_chain_kernel(const RowTask* __restric
   __shared__ T xs[64], acc[64], red[8][64];
   __shared__ int ticket, fail;
   const int tid = threadIdx.x, c = tid & 63, g = tid >> 6;
+  chain_wait();
   if (tid == 0) {
     ticket = int(atomicAdd(counter, 1u));
     fail = 0;
@@ -1059,6 +1061,7 @@ __global__ void sgather_fwd_kernel(const RowTask* __restrict__ tasks, const DevF
   const RowTask tk = tasks[blockIdx.x];
   const DevFront f = F[tk.front];
   const int nr = tk.r1 - tk.r0;
+  chain_wait();
   T* W = Wd + f.w_base * nrhs;
   for (int e = threadIdx.x; e < f.nb * nr; e += blockDim.x) W[int64_t(e / nr) * nrhs + tk.r0 + e % nr] = T(0);
   __syncthreads();
@@ -1085,6 +1088,7 @@ __global__ void sgather_bwd_kernel(const RowTask* __restrict__ tasks, const DevF
   const RowTask tk = tasks[blockIdx.x];
   const DevFront f = F[tk.front];
   const int nr = tk.r1 - tk.r0;
+  chain_wait();
   const int* bl = blist + f.b_off;
   T* Gf = G + f.w_base * nrhs;
   for (int e = threadIdx.x; e < f.nb * nr; e += blockDim.x) {
@@ -1104,6 +1108,7 @@ __global__ void zgather_kernel(const RowTask* __restrict__ tasks, const DevFront
   // flight per lane: the gather is latency-bound otherwise
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = tk.r0 + warp;
+  chain_wait();
   if (a >= tk.r1) return;
   const T* src = Zp + p.z_off + int64_t(rm[a]) * p.ldz;
   T* dst = Zc + f.z_off + int64_t(f.ns + a) * f.ldz + f.ns;
@@ -1128,6 +1133,7 @@ __global__ void mirror_kernel(const MirrorTask* __restrict__ tasks, int ntasks, 
   __shared__ T tile[kMirrorTiles][32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
   const int t0 = blockIdx.x * kMirrorTiles;
+  chain_wait();
 #pragma unroll
   for (int u = 0; u < kMirrorTiles; ++u) {
     if (t0 + u >= ntasks) break;
@@ -1157,6 +1163,7 @@ __global__ void zextract_kernel(const RowTask* __restrict__ tasks, const DevFron
   const RowTask tk = tasks[blockIdx.x];
   const DevFront f = F[tk.front];
   const int cnt = (tk.r1 - tk.r0) * nslots;
+  chain_wait();
   for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
     int v = f.s0 + tk.r0 + e / nslots, s = e % nslots;
     int k = iperm[v];
@@ -1355,24 +1362,24 @@ struct Exec {
           break;
         case OP_SGATHER_FWD: {
           int pd = o.depth & 1;
-          sgather_fwd_kernel<T><<<o.count, 256, 0, st>>>(s.d_rows + o.off, p->d_fronts, p->d_rmap, buf(B_X),
+          launch_chained(sgather_fwd_kernel<T>, o.count, 256, 0, st, s.d_rows + o.off, p->d_fronts, p->d_rmap, buf(B_X),
                                                          buf(pd ? B_W1 : B_W0), buf(pd ? B_W0 : B_W1), nrhs);
           break;
         }
         case OP_SGATHER_BWD: {
           int pd = o.depth & 1;
-          sgather_bwd_kernel<T><<<o.count, 256, 0, st>>>(s.d_rows + o.off, p->d_fronts, p->d_blist, buf(B_X),
+          launch_chained(sgather_bwd_kernel<T>, o.count, 256, 0, st, s.d_rows + o.off, p->d_fronts, p->d_blist, buf(B_X),
                                                          buf(pd ? B_G1 : B_G0), nrhs);
           break;
         }
         case OP_ZGATHER: {
           int pd = o.depth & 1;
-          zgather_kernel<T><<<o.count, 256, 0, st>>>(s.d_rows + o.off, p->d_fronts, p->d_rmap, buf(pd ? B_P0 : B_P1),
+          launch_chained(zgather_kernel<T>, o.count, 256, 0, st, s.d_rows + o.off, p->d_fronts, p->d_rmap, buf(pd ? B_P0 : B_P1),
                                                      buf(pd ? B_P1 : B_P0));
           break;
         }
         case OP_MIRROR:
-          mirror_kernel<T><<<(o.count + kMirrorTiles - 1) / kMirrorTiles, 256, 0, st>>>(s.d_mirror + o.off, o.count,
+          launch_chained(mirror_kernel<T>, (o.count + kMirrorTiles - 1) / kMirrorTiles, 256, 0, st, s.d_mirror + o.off, o.count,
                                                                                          buf(o.abuf), buf(o.cbuf));
           break;
         case OP_FWD_CHAIN:
@@ -1380,18 +1387,18 @@ struct Exec {
           cudaMemsetAsync(p->d_chain, 0, sizeof(unsigned), st);
           if (++p->chain_epoch == 0) ++p->chain_epoch;
           if (o.kind == OP_FWD_CHAIN)
-            fwd_chain_kernel<T><<<o.count, 256, 0, st>>>(s.d_rows + o.off, p->d_fronts, buf(B_L), buf(B_DINV),
+            launch_chained(fwd_chain_kernel<T>, o.count, 256, 0, st, s.d_rows + o.off, p->d_fronts, buf(B_L), buf(B_DINV),
                                                          buf(B_X), p->d_chain + 64, p->d_chain, p->chain_epoch,
                                                          p->d_chain_err, p->tc_wait_ns);
           else
-            bwd_chain_kernel<T><<<o.count, 512, 0, st>>>(s.d_rows + o.off, p->d_fronts, buf(B_L), buf(B_DINV),
+            launch_chained(bwd_chain_kernel<T>, o.count, 512, 0, st, s.d_rows + o.off, p->d_fronts, buf(B_L), buf(B_DINV),
                                                          buf(B_X), buf((o.depth & 1) == 0 ? B_G0 : B_G1),
                                                          p->d_chain + 64, p->d_chain, p->chain_epoch,
                                                          p->d_chain_err, p->tc_wait_ns);
           break;
         }
         case OP_ZEXTRACT:
-          zextract_kernel<T><<<o.count, 256, 0, st>>>(s.d_rows + o.off, p->d_fronts, p->d_iperm, p->d_amap,
+          launch_chained(zextract_kernel<T>, o.count, 256, 0, st, s.d_rows + o.off, p->d_fronts, p->d_iperm, p->d_amap,
                                                       p->sym.nslots, buf(o.cbuf), zq);
           break;
       }

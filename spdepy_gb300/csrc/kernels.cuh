@@ -22,6 +22,37 @@ struct GemmTask {
   int pair = 0;
 };
 
+// Kernels of a schedule are launched as dependents of their predecessor in the
+// stream: a kernel may be resident before the predecessor has finished (from the
+// moment all its blocks have called chain_trigger or ended), reads only what the
+// plan's set-up wrote until chain_wait, and every block calls chain_wait, so that a
+// finished kernel implies finished predecessors.  The trigger stands before a kernel's
+// last stores: earlier, waiting blocks would hold SMs that another stream can use.
+// Measured on evaluations (without / with): 16 x 16 x 8 2.00 / 1.74 ms, 47 x 39 x 13
+// 7.36 / 6.62 ms, 100 x 100 x 24 74.8 / 73.1 ms; 256 draws at 100 x 100 x 24 34.3 / 32.0 ms.
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void chain_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // an integer constant as a type (selects a kernel's template argument in a lambda)
 template <int N>
 struct IntC {

@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(kThreads, ST == 2 ? 2 : 1) tc_gemm_kernel(cons
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
   const int nk = (tk.k + kTK - 1) / kTK;
+  chain_wait();
 
   // bounded wait (wait_ns for the pipeline's waits; the clean-up below always
   // allows kWaitNs); with `honor_abort` it also gives up as soon as another
@@ -360,6 +361,7 @@ __global__ void __launch_bounds__(kThreads, ST == 2 ? 2 : 1) tc_gemm_kernel(cons
     }
     // every converter warp comes here, also after a failed wait
     asm volatile("barrier.cta.sync 1, %0;" ::"n"(kGroups * kConv) : "memory");
+    chain_trigger();
     if (fin) rows_to_global<MODE, kTN, kGroups * kConv / 32>(tile, kTileLd, C, tk.ldc, tk.m, tk.n, warp, lane);
   } else if (warp < (kGroups * kConv + kLoad) / 32) {
     // ---------------- loaders
@@ -572,6 +574,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
   const int nk = (tk.k + kTK - 1) / kTK;
+  chain_wait();
 
   auto wait = [&](uint64_t* bar, uint32_t parity, bool honor_abort, unsigned long long limit) -> bool {
     if (mbar_try(smem_u32(bar), parity)) return true;
@@ -623,6 +626,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
     // every converter warp comes here, also after a failed wait
     asm volatile("barrier.cta.sync 1, %0;" ::"n"(kPairGroups * kConv) : "memory");
+    chain_trigger();
     if (fin && am > 0)
       rows_to_global<MODE, 256, kPairGroups * kConv / 32>(tile, kPairTileLd, Cb + tk.c + int64_t(row0) * tk.ldc, tk.ldc,
                                                           min(am, 128), tk.n, warp, lane);
@@ -708,7 +712,7 @@ void launch_pair(const GemmTask* t, int n, const CUtensorMap* maps, const float*
     return true;
   }();
   (void)attr;
-  tc_pair_kernel<MODE><<<2 * n, kPairThreads, kSmem, st>>>(t, maps, A, B, C, wait_ns);
+  launch_chained(tc_pair_kernel<MODE>, 2 * n, kPairThreads, kSmem, st, t, maps, A, B, C, wait_ns);
 }
 
 template <int MODE, int AL, int BL, int ST>
@@ -722,7 +726,7 @@ void launch_stages(const GemmTask* t, int n, const float* A, const float* B, flo
     return true;
   }();
   (void)attr;
-  tc_gemm_kernel<MODE, AL, BL, ST><<<n, kThreads, smem, st>>>(t, A, B, C, wait_ns);
+  launch_chained(tc_gemm_kernel<MODE, AL, BL, ST>, n, kThreads, smem, st, t, A, B, C, wait_ns);
 }
 // Four stages while every tile has an SM to itself (a shorter wait per tile), two
 // CTAs per SM beyond.  Measured: launches of up to 152 tiles 17.4 against 20.2 us, the
