@@ -288,9 +288,10 @@ template void launch_scatter<float>(const QStencil&, int, const int*, const int*
 // time axis: the cell's time-invariant coefficients (25 in-block values, 9 to
 // t + 1 and the 9 mirrored from the neighbours to t - 1) are loaded once and
 // reused for all T blocks.
+// `wd` not null: y = x - wd A x (wd one weight per node), a damped Jacobi sweep.
 __global__ void __launch_bounds__(128) spmv_cells_kernel(QStencil q, const double* __restrict__ obs, double tau,
                                                          const double* __restrict__ x, double* __restrict__ y,
-                                                         int nrhs) {
+                                                         int nrhs, int steps, const double* __restrict__ wd) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= int64_t(q.Ns) * nrhs) return;
   const int c = int(e / nrhs), r = int(e - int64_t(c) * nrhs);
@@ -315,7 +316,8 @@ __global__ void __launch_bounds__(128) spmv_cells_kernel(QStencil q, const doubl
     }
   }
   const double cqs = q.T > 1 ? q.cQs[c] : 0.0;
-  for (int t = 0; t < q.T; ++t) {
+  const int t0 = int(blockIdx.y) * steps, t1 = min(q.T, t0 + steps);
+  for (int t = t0; t < t1; ++t) {
     const int64_t k = int64_t(t) * q.Ns + c;
     const double* xt = x + k * nrhs + r;
     double acc = 0.0;
@@ -350,7 +352,7 @@ __global__ void __launch_bounds__(128) spmv_cells_kernel(QStencil q, const doubl
       }
     }
     if (obs) acc = fma(tau * obs[k], xt[0], acc);
-    y[k * nrhs + r] = acc;
+    y[k * nrhs + r] = wd ? fma(-wd[k], acc, xt[0]) : acc;
   }
 }
 
@@ -393,11 +395,32 @@ __global__ void __launch_bounds__(128) spmv_sep_kernel(QStencil q, const double*
   }
 }
 
+// Time steps per thread: all of them when cells and columns fill the GPU, fewer (the
+// cell's 43 coefficients are then loaded more than once) down to one until about
+// 1,500 threads per SM run.  Measured at 100 x 100 x 12, two columns: 45 us with one
+// thread per cell and column, 21 us with two steps per thread.
+static dim3 spmv_grid(const QStencil& q, int nrhs, int* steps) {
+  const int64_t tot = int64_t(q.Ns) * nrhs;
+  *steps = q.T;
+  while (*steps > 1 && tot * ((q.T + *steps - 1) / *steps) < 152 * 1536) *steps = (*steps + 1) / 2;
+  return dim3(nblk(tot, 128), (q.T + *steps - 1) / *steps);
+}
 void launch_spmv(const QStencil& q, const double* obs, double tau, const double* x, double* y, int nrhs,
                  cudaStream_t st) {
   const int64_t tot = int64_t(q.Ns) * nrhs;
-  if (q.sep) spmv_sep_kernel<<<nblk(tot, 128), 128, 0, st>>>(q, obs, tau, x, y, nrhs);
-  else spmv_cells_kernel<<<nblk(tot, 128), 128, 0, st>>>(q, obs, tau, x, y, nrhs);
+  if (q.sep) {
+    spmv_sep_kernel<<<nblk(tot, 128), 128, 0, st>>>(q, obs, tau, x, y, nrhs);
+    return;
+  }
+  int steps;
+  const dim3 grid = spmv_grid(q, nrhs, &steps);
+  spmv_cells_kernel<<<grid, 128, 0, st>>>(q, obs, tau, x, y, nrhs, steps, nullptr);
+}
+void launch_jacobi_sweep(const QStencil& q, const double* obs, double tau, const double* wd, const double* x, double* y,
+                         int nrhs, cudaStream_t st) {
+  int steps;
+  const dim3 grid = spmv_grid(q, nrhs, &steps);
+  spmv_cells_kernel<<<grid, 128, 0, st>>>(q, obs, tau, x, y, nrhs, steps, wd);
 }
 void launch_diffusion_triplets(int M, int N, const double* H, int field, double hx, double hy, int bc, int* row,
                                int* col, double* val, cudaStream_t st) {

@@ -81,6 +81,9 @@ void launch_scatter(const QStencil& q, int nslots, const int* amap, const int* p
                     const DevFront* fronts, const double* obs, double tau, T* L, cudaStream_t st);
 void launch_spmv(const QStencil& q, const double* obs, double tau, const double* x, double* y, int nrhs,
                  cudaStream_t st);
+// y = x - wd A x, wd one weight per node (spatial and spatio-temporal layouts)
+void launch_jacobi_sweep(const QStencil& q, const double* obs, double tau, const double* wd, const double* x, double* y,
+                         int nrhs, cudaStream_t st);
 void launch_diffusion_triplets(int M, int N, const double* H, int field, double hx, double hy, int bc, int* row,
                                int* col, double* val, cudaStream_t st);
 void launch_advection_triplets(int M, int N, const double* G, const double* dG, int field, double hx, double hy,

@@ -108,20 +108,30 @@ __device__ __forceinline__ void pc_network(const QStencil& q, int c, int t, doub
 }
 
 // G weights of every node, offset-major (w[o n + p]), one thread per node.
+// The activations of a block's nodes are contiguous: staged in shared memory and
+// written in order.
 __global__ void __launch_bounds__(128) pc_forward_kernel(QStencil q, const double* __restrict__ obs, double tau,
                                                          const float* __restrict__ prm, float* __restrict__ w,
                                                          float* __restrict__ act) {
-  __shared__ float sp[kNP];
+  extern __shared__ float fsm[];
+  float* sp = fsm;
+  float* sact = fsm + kNP;  // 128 x kAct (with act)
   for (int i = threadIdx.x; i < kNP; i += blockDim.x) sp[i] = prm[i];
   __syncthreads();
   const int64_t n = int64_t(q.Ns) * q.T;
-  const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int t = int(p / q.Ns), c = int(p - int64_t(t) * q.Ns);
-  float wo[kOff];
-  pc_network(q, c, t, obs ? tau * obs[p] : 0.0, sp, wo, act ? act + p * kAct : nullptr);
+  const int64_t p0 = int64_t(blockIdx.x) * 128, p = p0 + threadIdx.x;
+  if (p < n) {
+    const int t = int(p / q.Ns), c = int(p - int64_t(t) * q.Ns);
+    float wo[kOff];
+    pc_network(q, c, t, obs ? tau * obs[p] : 0.0, sp, wo, act ? sact + threadIdx.x * kAct : nullptr);
 #pragma unroll
-  for (int o = 0; o < kOff; ++o) w[int64_t(o) * n + p] = wo[o];
+    for (int o = 0; o < kOff; ++o) w[int64_t(o) * n + p] = wo[o];
+  }
+  if (act) {
+    __syncthreads();
+    const int cnt = int(n - p0 < 128 ? n - p0 : 128) * kAct;
+    for (int i = threadIdx.x; i < cnt; i += 128) act[p0 * kAct + i] = sact[i];
+  }
 }
 
 // Compact weights.  A node's row of A depends on its time only through three
@@ -192,33 +202,86 @@ __global__ void pc_sub_kernel(const double* __restrict__ z, double* __restrict__
   if (i < len) v[i] = z[i] - v[i];
 }
 
-// dL/d(network output) per node: (sum_r e_pr u_(p+o)r + z_pr g_(p+o)r) * scale * s_p
-__global__ void pc_wgrad_kernel(QStencil q, const double* __restrict__ z, const double* __restrict__ e,
-                                const double* __restrict__ u, const double* __restrict__ g, int nrhs, double scale,
-                                const float* __restrict__ act, float* __restrict__ dout) {
+// dL/d(network output) per node: (sum_r e_pr u_(p+o)r + z_pr g_(p+o)r) * scale * s_p.
+// NR columns (0: nrhs of them) with the node's own values held in registers.
+template <int NR>
+__global__ void __launch_bounds__(128) pc_wgrad_kernel(QStencil q, const double* __restrict__ z,
+                                                       const double* __restrict__ e, const double* __restrict__ u,
+                                                       const double* __restrict__ g, int nrhs, double scale,
+                                                       const float* __restrict__ act, float* __restrict__ dout) {
+  __shared__ float so[128 * kOff];
   const int64_t n = int64_t(q.Ns) * q.T;
-  const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int t = int(p / q.Ns), c = int(p - int64_t(t) * q.Ns);
-  const int y = c / q.Mx, x = c - y * q.Mx;
-  const double s = act[p * kAct + kAct - 1];
-  for (int o = 0; o < kOff; ++o) {
-    int dx, dy, dt;
-    off27(o, &dx, &dy, &dt);
-    double acc = 0.0;
-    if (inside(q, x + dx, y + dy, t + dt)) {
-      const int64_t nb = p + (int64_t(dt) * q.Ny + dy) * q.Mx + dx;
-      for (int r = 0; r < nrhs; ++r)
-        acc += e[p * nrhs + r] * u[nb * nrhs + r] + z[p * nrhs + r] * g[nb * nrhs + r];
+  const int64_t p0 = int64_t(blockIdx.x) * 128, p = p0 + threadIdx.x;
+  if (p < n) {
+    const int t = int(p / q.Ns), c = int(p - int64_t(t) * q.Ns);
+    const int y = c / q.Mx, x = c - y * q.Mx;
+    const double s = act[p * kAct + kAct - 1];
+    double ep[NR > 0 ? NR : 1], zp[NR > 0 ? NR : 1];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      ep[r] = e[p * NR + r];
+      zp[r] = z[p * NR + r];
     }
-    dout[p * kOff + o] = float(acc * scale * s);
+#pragma unroll 3
+    for (int o = 0; o < kOff; ++o) {
+      int dx, dy, dt;
+      off27(o, &dx, &dy, &dt);
+      double acc = 0.0;
+      if (inside(q, x + dx, y + dy, t + dt)) {
+        const int64_t nb = p + (int64_t(dt) * q.Ny + dy) * q.Mx + dx;
+        if (NR > 0) {
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            acc = fma(ep[r], u[nb * NR + r], acc);
+            acc = fma(zp[r], g[nb * NR + r], acc);
+          }
+        } else {
+          for (int r = 0; r < nrhs; ++r) {
+            acc = fma(e[p * nrhs + r], u[nb * nrhs + r], acc);
+            acc = fma(z[p * nrhs + r], g[nb * nrhs + r], acc);
+          }
+        }
+      }
+      so[threadIdx.x * kOff + o] = float(acc * scale * s);
+    }
   }
+  __syncthreads();
+  const int cnt = int(n - p0 < 128 ? n - p0 : 128) * kOff;  // the block's rows are contiguous
+  for (int i = threadIdx.x; i < cnt; i += 128) dout[p0 * kOff + i] = so[i];
 }
 
 // Network backward: per block of kBwNodes nodes, the parameter gradient of the
 // block's nodes into its own row of `part` (nblocks x kNP).
+// Bound: shared-memory reads; every product is tiled in registers.
 constexpr int kBwNodes = 64;
-__global__ void __launch_bounds__(128) pc_backward_kernel(int64_t n, const float* __restrict__ prm,
+constexpr int kBwThreads = 192;
+static_assert(kFeat == 42 && kHid == 32 && kOff == 27, "tiles of the weight gradients");
+// out[i ldo + j] = sum over nodes a of D[a ldd + i] H[a ldh + j], R x C entries
+template <int R, int C>
+__device__ __forceinline__ void weight_tile(const float* D, int ldd, const float* H, int ldh, float* out, int ldo) {
+  float acc[R][C];
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j) acc[i][j] = 0.f;
+#pragma unroll 4
+  for (int a = 0; a < kBwNodes; ++a) {
+    float d[R], h[C];
+#pragma unroll
+    for (int i = 0; i < R; ++i) d[i] = D[a * ldd + i];
+#pragma unroll
+    for (int j = 0; j < C; ++j) h[j] = H[a * ldh + j];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < C; ++j) acc[i][j] = fmaf(d[i], h[j], acc[i][j]);
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j) out[i * ldo + j] = acc[i][j];
+}
+__global__ void __launch_bounds__(kBwThreads) pc_backward_kernel(int64_t n, const float* __restrict__ prm,
                                                           const float* __restrict__ act,
                                                           const float* __restrict__ dout, float* __restrict__ part) {
   extern __shared__ float sm[];
@@ -249,55 +312,88 @@ __global__ void __launch_bounds__(128) pc_backward_kernel(int64_t n, const float
     sdo[i] = a < cnt ? dout[(p0 + a) * kOff + (i - a * kOff)] : 0.f;
   }
   __syncthreads();
-  // dh2 = W3^T dout (1 - h2^2), then dh1 = W2^T dh2 (1 - h1^2)
-  for (int i = tid; i < kBwNodes * kHid; i += blockDim.x) {
-    const int a = i / kHid, j = i - a * kHid;
-    float acc = 0.f;
-    for (int o = 0; o < kOff; ++o) acc = fmaf(sW3[o * kHid + j], sdo[a * kOff + o], acc);
-    const float h = sh2[i];
-    sd2[i] = acc * (1.f - h * h);
-  }
-  __syncthreads();
-  for (int i = tid; i < kBwNodes * kHid; i += blockDim.x) {
-    const int a = i / kHid, j = i - a * kHid;
-    float acc = 0.f;
-    for (int k = 0; k < kHid; ++k) acc = fmaf(sW2[k * kHid + j], sd2[a * kHid + k], acc);
-    const float h = sh1[i];
-    sd1[i] = acc * (1.f - h * h);
-  }
-  __syncthreads();
-  float* out = part + int64_t(blockIdx.x) * kNP;
-  for (int e = tid; e < kNP; e += blockDim.x) {
-    float acc = 0.f;
-    if (e < kB1) {
-      const int i = e / kFeat, j = e - i * kFeat;
-      for (int a = 0; a < kBwNodes; ++a) acc = fmaf(sd1[a * kHid + i], sf[a * kFeat + j], acc);
-    } else if (e < kW2) {
-      const int i = e - kB1;
-      for (int a = 0; a < kBwNodes; ++a) acc += sd1[a * kHid + i];
-    } else if (e < kB2) {
-      const int i = (e - kW2) / kHid, j = (e - kW2) - i * kHid;
-      for (int a = 0; a < kBwNodes; ++a) acc = fmaf(sd2[a * kHid + i], sh1[a * kHid + j], acc);
-    } else if (e < kW3) {
-      const int i = e - kB2;
-      for (int a = 0; a < kBwNodes; ++a) acc += sd2[a * kHid + i];
-    } else if (e < kB3) {
-      const int o = (e - kW3) / kHid, j = (e - kW3) - o * kHid;
-      for (int a = 0; a < kBwNodes; ++a) acc = fmaf(sdo[a * kOff + o], sh2[a * kHid + j], acc);
-    } else {
-      const int o = e - kB3;
-      for (int a = 0; a < kBwNodes; ++a) acc += sdo[a * kOff + o];
+  // dh2 = W3^T dout (1 - h2^2), then dh1 = W2^T dh2 (1 - h1^2): lane = hidden unit,
+  // eight nodes per thread
+  const int j = tid & 31;
+  for (int a0 = 8 * (tid >> 5); a0 < kBwNodes; a0 += 8 * (kBwThreads / 32)) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+#pragma unroll 3
+    for (int o = 0; o < kOff; ++o) {
+      const float w = sW3[o * kHid + j];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, sdo[(a0 + i) * kOff + o], acc[i]);
     }
-    out[e] = acc;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float h = sh2[(a0 + i) * kHid + j];
+      sd2[(a0 + i) * kHid + j] = acc[i] * (1.f - h * h);
+    }
+  }
+  __syncthreads();
+  for (int a0 = 8 * (tid >> 5); a0 < kBwNodes; a0 += 8 * (kBwThreads / 32)) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < kHid; ++k) {
+      const float w = sW2[k * kHid + j];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, sd2[(a0 + i) * kHid + k], acc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float h = sh1[(a0 + i) * kHid + j];
+      sd1[(a0 + i) * kHid + j] = acc[i] * (1.f - h * h);
+    }
+  }
+  __syncthreads();
+  // dW = D^T H over the block's nodes, one register tile per thread: 56 tiles of
+  // 4 x 6 for W1, 64 of 4 x 4 for W2, 72 of 3 x 4 for W3
+  float* out = part + int64_t(blockIdx.x) * kNP;
+  if (tid < 56)
+    weight_tile<4, 6>(sd1 + 4 * (tid / 7), kHid, sf + 6 * (tid % 7), kFeat, out + kW1 + 4 * (tid / 7) * kFeat + 6 * (tid % 7),
+                      kFeat);
+  else if (tid < 120)
+    weight_tile<4, 4>(sd2 + 4 * ((tid - 56) / 8), kHid, sh1 + 4 * ((tid - 56) % 8), kHid,
+                      out + kW2 + 4 * ((tid - 56) / 8) * kHid + 4 * ((tid - 56) % 8), kHid);
+  else
+    weight_tile<3, 4>(sdo + 3 * ((tid - 120) / 8), kOff, sh2 + 4 * ((tid - 120) % 8), kHid,
+                      out + kW3 + 3 * ((tid - 120) / 8) * kHid + 4 * ((tid - 120) % 8), kHid);
+  if (tid < kHid + kHid + kOff) {  // biases
+    const float* d = tid < kHid ? sd1 + tid : tid < 2 * kHid ? sd2 + tid - kHid : sdo + tid - 2 * kHid;
+    const int ld = tid < 2 * kHid ? kHid : kOff;
+    float acc = 0.f;
+    for (int a = 0; a < kBwNodes; ++a) acc += d[a * ld];
+    out[tid < kHid ? kB1 + tid : tid < 2 * kHid ? kB2 + tid - kHid : kB3 + tid - 2 * kHid] = acc;
   }
 }
 
-// grad[e] = sum over blocks of part[b][e] (fixed order)
-__global__ void pc_colsum_kernel(const float* __restrict__ part, int nb, float* __restrict__ grad) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= kNP) return;
+// grad[e] = sum over blocks of part[b][e] in FP64 and a fixed order: kColParts CTAs
+// share the blocks of every 128 columns, the last of them to finish adds their sums
+constexpr int kColParts = 32;
+__global__ void __launch_bounds__(128) pc_colsum_kernel(const float* __restrict__ part, int nb,
+                                                        double* __restrict__ sums, unsigned* __restrict__ arrived,
+                                                        float* __restrict__ grad) {
+  __shared__ bool last;
+  const int e = blockIdx.x * 128 + threadIdx.x;
+  const int per = (nb + kColParts - 1) / kColParts, b0 = int(blockIdx.y) * per, b1 = min(nb, b0 + per);
   double acc = 0.0;
-  for (int b = 0; b < nb; ++b) acc += part[int64_t(b) * kNP + e];
+  if (e < kNP) {
+#pragma unroll 8
+    for (int b = b0; b < b1; ++b) acc += part[int64_t(b) * kNP + e];
+    sums[int64_t(blockIdx.y) * kNP + e] = acc;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&arrived[blockIdx.x], 1u) == kColParts - 1;
+  __syncthreads();
+  if (!last || e >= kNP) return;
+  __threadfence();
+  acc = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < kColParts; ++b) acc += __ldcg(sums + int64_t(b) * kNP + e);
   grad[e] = float(acc);
 }
 
@@ -359,6 +455,14 @@ __global__ void jacobi_sweep_kernel(QStencil q, const double* __restrict__ obs, 
   const int t = int(p / q.Ns), c = int(p - int64_t(t) * q.Ns);
   const double d = qval(q, c, t, 0, 0, 0) + (obs ? tau * obs[p] : 0.0);
   z[e] -= omega * az[e] / d;
+}
+// wd = omega / diag(A) per node
+__global__ void jacobi_weight_kernel(QStencil q, const double* __restrict__ obs, double tau, double omega,
+                                     double* __restrict__ wd) {
+  const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (p >= int64_t(q.Ns) * q.T) return;
+  const int t = int(p / q.Ns), c = int(p - int64_t(t) * q.Ns);
+  wd[p] = omega / (qval(q, c, t, 0, 0, 0) + (obs ? tau * obs[p] : 0.0));
 }
 // z[:, r] *= 1 / sqrt(ss[r] / n)
 __global__ void col_scale_kernel(double* __restrict__ z, const double* __restrict__ ss, int64_t n, int nrhs) {
@@ -1201,8 +1305,14 @@ int qsqrt_apply(Plan* p, int transpose, const double* x, double* y, int nrhs) {
 
 int pc_weights(Plan* p, int with_obs, double tau, const float* prm, float* w, float* act) {
   const int64_t n = p->sym.n;
-  pc_forward_kernel<<<nblk(n, 128), 128, 0, p->stream>>>(p->qstencil(), with_obs ? p->d_obs_cnt : nullptr, tau, prm,
-                                                          w, act);
+  constexpr int kActSmem = (kNP + 128 * kAct) * int(sizeof(float));
+  static const bool attr = [] {  // once, thread-safely
+    cudaFuncSetAttribute(pc_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kActSmem);
+    return true;
+  }();
+  (void)attr;
+  pc_forward_kernel<<<nblk(n, 128), 128, act ? kActSmem : kNP * int(sizeof(float)), p->stream>>>(
+      p->qstencil(), with_obs ? p->d_obs_cnt : nullptr, tau, prm, w, act);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
@@ -1212,13 +1322,15 @@ int pc_grad(Plan* p, int with_obs, double tau, const float* prm, const float* w,
   if (len >= (int64_t(1) << 31)) return 1;  // the stencil kernels index entries in 32 bits
   const int nbw = int((n + kBwNodes - 1) / kBwNodes);
   // y, u, e, g1, g2 (n x k doubles each) + partial sums + per-node dout and block partials (as floats)
-  const size_t dbl = size_t(5 * len) + size_t(kDotBlocks) * k + 8;
+  const size_t dbl = size_t(5 * len) + size_t(kDotBlocks) * k + 8 + size_t(kColParts) * kNP + 32;
   const size_t flt = size_t(n) * kOff + size_t(nbw) * kNP;
   double* base = scratch(p, dbl + (flt + 1) / 2);
   if (!base) return 4;
   double *y = base, *u = y + len, *e = u + len, *g1 = e + len, *g2 = g1 + len, *part = g2 + len;
   double* sums = part + size_t(kDotBlocks) * k;
-  float* dout = reinterpret_cast<float*>(sums + 8);
+  double* colsums = sums + 8;
+  unsigned* arrived = reinterpret_cast<unsigned*>(colsums + size_t(kColParts) * kNP);
+  float* dout = reinterpret_cast<float*>(colsums + size_t(kColParts) * kNP + 32);
   float* bpart = dout + size_t(n) * kOff;
   const QStencil q = p->qstencil();
   const double* obs = with_obs ? p->d_obs_cnt : nullptr;
@@ -1233,15 +1345,17 @@ int pc_grad(Plan* p, int with_obs, double tau, const float* prm, const float* w,
   pc_dot_partial_kernel<<<kDotBlocks, 256, 0, st>>>(e, e, len, 1, part);
   pc_dot_final_kernel<<<1, 64, 0, st>>>(part, kDotBlocks, 1, sums);
   const double scale = -2.0 / double(len);
-  pc_wgrad_kernel<<<nblk(n, 128), 128, 0, st>>>(q, z, e, u, g2, k, scale, act, dout);
+  if (k == 4) pc_wgrad_kernel<4><<<nblk(n, 128), 128, 0, st>>>(q, z, e, u, g2, k, scale, act, dout);
+  else pc_wgrad_kernel<0><<<nblk(n, 128), 128, 0, st>>>(q, z, e, u, g2, k, scale, act, dout);
   const size_t smem = sizeof(float) * (kHid * kHid + kOff * kHid + kBwNodes * (kFeat + 4 * kHid + kOff));
   static const bool attr = [smem] {  // once, thread-safely
     cudaFuncSetAttribute(pc_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     return true;
   }();
   (void)attr;
-  pc_backward_kernel<<<nbw, 128, smem, st>>>(n, prm, act, dout, bpart);
-  pc_colsum_kernel<<<nblk(kNP, 128), 128, 0, st>>>(bpart, nbw, grad);
+  pc_backward_kernel<<<nbw, kBwThreads, smem, st>>>(n, prm, act, dout, bpart);
+  cudaMemsetAsync(arrived, 0, 32 * sizeof(double), st);
+  pc_colsum_kernel<<<dim3(nblk(kNP, 128), kColParts), 128, 0, st>>>(bpart, nbw, colsums, arrived, grad);
   double h = 0.0;
   cudaMemcpyAsync(&h, sums, sizeof(double), cudaMemcpyDeviceToHost, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return 2;
@@ -1258,14 +1372,25 @@ int pc_adam(const float* g, float* prm, float* m, float* v, int n, float lr, flo
 
 int jacobi_smooth(Plan* p, int with_obs, double tau, double omega, int sweeps, double* z, int nrhs) {
   const int64_t n = p->sym.n, len = n * nrhs;
-  double* base = scratch(p, size_t(len) + size_t(kDotBlocks) * nrhs + size_t(nrhs));
+  double* base = scratch(p, size_t(len) + size_t(kDotBlocks) * nrhs + size_t(nrhs) + size_t(n));
   if (!base) return 4;
-  double *az = base, *part = az + len, *ss = part + size_t(kDotBlocks) * nrhs;
+  double *az = base, *part = az + len, *ss = part + size_t(kDotBlocks) * nrhs, *wd = ss + nrhs;
   const QStencil q = p->qstencil();
   const double* obs = with_obs ? p->d_obs_cnt : nullptr;
-  for (int it = 0; it < sweeps; ++it) {
-    launch_spmv(q, obs, tau, z, az, nrhs, p->stream);
-    jacobi_sweep_kernel<<<nblk(len), 256, 0, p->stream>>>(q, obs, tau, omega, az, z, nrhs);
+  if (q.sep) {
+    for (int it = 0; it < sweeps; ++it) {
+      launch_spmv(q, obs, tau, z, az, nrhs, p->stream);
+      jacobi_sweep_kernel<<<nblk(len), 256, 0, p->stream>>>(q, obs, tau, omega, az, z, nrhs);
+    }
+  } else {
+    // one launch per sweep, from z to the scratch block and back
+    jacobi_weight_kernel<<<nblk(n), 256, 0, p->stream>>>(q, obs, tau, omega, wd);
+    double *from = z, *to = az;
+    for (int it = 0; it < sweeps; ++it) {
+      launch_jacobi_sweep(q, obs, tau, wd, from, to, nrhs, p->stream);
+      std::swap(from, to);
+    }
+    if (from != z) cudaMemcpyAsync(z, from, size_t(len) * sizeof(double), cudaMemcpyDeviceToDevice, p->stream);
   }
   col_dots(p, z, z, nrhs, part, ss);
   col_scale_kernel<<<nblk(len), 256, 0, p->stream>>>(z, ss, n, nrhs);
