@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(128) spmv_sep_kernel(QStencil q, const double*
 // Time steps per thread: all of them when cells and columns fill the GPU, fewer (the
 // cell's 43 coefficients are then loaded more than once) down to one until about
 // 1,500 threads per SM run.  Measured at 100 x 100 x 12, two columns: 45 us with one
-// thread per cell and column, 21 us with two steps per thread.
+// thread per cell and column, 32 us with two steps per thread (37 with six).
 static dim3 spmv_grid(const QStencil& q, int nrhs, int* steps) {
   const int64_t tot = int64_t(q.Ns) * nrhs;
   *steps = q.T;
