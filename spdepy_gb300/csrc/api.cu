@@ -141,13 +141,16 @@ struct DevBuf {
   }
 };
 
-double host_sum_partials(const double* dpart, int nblk, cudaStream_t st) {
-  std::vector<double> h(nblk);
-  cudaMemcpyAsync(h.data(), dpart, nblk * sizeof(double), cudaMemcpyDeviceToHost, st);
+// Sums of nblk block partials at dpart, and (s2 not null) of the nblk after them
+void host_sum_partials(const double* dpart, int nblk, cudaStream_t st, double* s1, double* s2 = nullptr) {
+  std::vector<double> h(2 * nblk);
+  cudaMemcpyAsync(h.data(), dpart, (s2 ? 2 : 1) * nblk * sizeof(double), cudaMemcpyDeviceToHost, st);
   cudaStreamSynchronize(st);
-  double s = 0.0;
-  for (double v : h) s += v;
-  return s;
+  *s1 = 0.0;
+  for (int i = 0; i < nblk; ++i) *s1 += h[i];
+  if (!s2) return;
+  *s2 = 0.0;
+  for (int i = 0; i < nblk; ++i) *s2 += h[nblk + i];
 }
 
 int ntheta_of(const Plan& p) { return 4 * p.model.nk + p.model.nw + 6; }
@@ -811,7 +814,7 @@ int spde_loglike(SpdePlan* plan, const double* theta, int ntheta, const double* 
   const double tau = std::exp(theta[ntheta - 1]);
   LoglikeScratch& S = plan->s;
   const int nblk = 256;
-  API_CUDA(S.part.ensure(nblk));
+  API_CUDA(S.part.ensure(2 * nblk));
   const bool exact = grad_mode == 1, hutch = grad_mode == 2;
   if (exact) { API_CUDA(S.zq.ensure(size_t(n) * ns)); API_CUDA(S.zqc.ensure(size_t(n) * ns)); }
   if (hutch) { API_CUDA(S.trq.ensure(size_t(n) * nh1)); API_CUDA(S.trc.ensure(size_t(n) * nh1)); }
@@ -842,17 +845,54 @@ int spde_loglike(SpdePlan* plan, const double* theta, int ntheta, const double* 
   bool phased = qc != &p;
   if (phased && (rc = ensure_phase_streams(plan))) return rc;
   cudaStream_t qc_home = qc->stream;
+  double muqmu = 0.0, rss = 0.0;
   auto run_qc = [&]() {
     if (phased) move_to(qc, plan->phase[1][0], plan->phase_ev[1][0]);
     if ((rc_c = plan_factor(qc, 1, tau))) return;
     plog.mark("qc_factor", qc->stream);
     ldqc = qc->logdet;
+    // the selected inversion on its own stream and thread, beside the solve (both
+    // only read the factor); per-launch timing keeps them one after the other
+    std::thread inverter;
+    int rc_i = 0;
+    std::string err_i;
+    if (phased && exact && !qc->profile) {
+      const cudaStream_t to = plan->phase[1][1];
+      cudaEventRecord(plan->phase_ev[1][1], qc->stream);
+      cudaStreamWaitEvent(to, plan->phase_ev[1][1], 0);
+      try {
+        inverter = std::thread([&, to]() {
+          cudaSetDevice(p.device);
+          rc_i = plan_selinv_on(qc, S.zqc.p, to, &err_i);
+          plog.mark("qc_inverse", to);
+        });
+      } catch (...) {  // no thread available: after the solve
+      }
+    }
+    const bool beside = inverter.joinable();
     cudaMemsetAsync(S.b.p, 0, size_t(n) * r * sizeof(double), qc->stream);
     obs_rhs_kernel<<<int((int64_t(m) * r + 255) / 256), 256, 0, qc->stream>>>(p.d_obs_idx, m, r, tau, y, nullptr,
                                                                                S.b.p);
-    if ((rc_c = plan_solve(qc, S.b.p, S.mu.p, r, iters, tol, &res_c))) return;
+    rc_c = plan_solve(qc, S.b.p, S.mu.p, r, iters, tol, &res_c);
     plog.mark("qc_solve", qc->stream);
-    if (hutch && (rc_c = plan_solve(qc, V, S.trc.p, nh1, iters, tol, &res_c))) return;
+    if (!rc_c && hutch) rc_c = plan_solve(qc, V, S.trc.p, nh1, iters, tol, &res_c);
+    if (!rc_c) {  // quadratic terms
+      launch_spmv(p.qstencil(), nullptr, 0.0, S.mu.p, S.qmu.p, r, qc->stream);
+      dot_partial_kernel<<<nblk, 256, 0, qc->stream>>>(S.mu.p, S.qmu.p, int64_t(n) * r, S.part.p);
+      obs_resid_kernel<<<int((int64_t(m) * r + 255) / 256), 256, 0, qc->stream>>>(p.d_obs_idx, m, r, y, S.mu.p, S.d.p);
+      dot_partial_kernel<<<nblk, 256, 0, qc->stream>>>(S.d.p, nullptr, int64_t(m) * r, S.part.p + nblk);
+      host_sum_partials(S.part.p, nblk, qc->stream, &muqmu, &rss);
+    }
+    if (beside) {
+      inverter.join();
+      plan_selinv_done(qc);
+      if (!rc_c && rc_i) {
+        rc_c = rc_i;
+        qc->last_error = err_i;
+      }
+      return;
+    }
+    if (rc_c) return;
     if (phased) move_to(qc, plan->phase[1][1], plan->phase_ev[1][1]);
     if (exact && (rc_c = plan_selinv(qc, S.zqc.p))) return;
     plog.mark("qc_inverse", qc->stream);
@@ -888,13 +928,6 @@ int spde_loglike(SpdePlan* plan, const double* theta, int ntheta, const double* 
     if (qc != &p) p.last_error = qc->last_error;
     return rc_c;
   }
-  // quadratic terms
-  launch_spmv(p.qstencil(), nullptr, 0.0, S.mu.p, S.qmu.p, r, st);
-  dot_partial_kernel<<<nblk, 256, 0, st>>>(S.mu.p, S.qmu.p, int64_t(n) * r, S.part.p);
-  const double muqmu = host_sum_partials(S.part.p, nblk, st);
-  obs_resid_kernel<<<int((int64_t(m) * r + 255) / 256), 256, 0, st>>>(p.d_obs_idx, m, r, y, S.mu.p, S.d.p);
-  dot_partial_kernel<<<nblk, 256, 0, st>>>(S.d.p, nullptr, int64_t(m) * r, S.part.p);
-  const double rss = host_sum_partials(S.part.p, nblk, st);
   p.launches_total += 5;  // obs rhs, spmv, two dot partials, obs residual
   const double like = 0.5 * ldq * r + m * r * std::log(tau) / 2 - 0.5 * ldqc * r - 0.5 * muqmu - tau / 2 * rss;
   *f_out = -like / (double(m) * r);
@@ -913,11 +946,12 @@ int spde_loglike(SpdePlan* plan, const double* theta, int ntheta, const double* 
   API_CUDA(S.gradv.ensure(size_t(ntheta)));
   launch_adjoint(&p, S.gbar.p, S.gradv.p, S.work.p, st);
   std::vector<double> g(ntheta, 0.0);
-  API_CUDA(cudaMemcpyAsync(g.data(), S.gradv.p, (ntheta - 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
   const int centre = p.sym.nslots / 2;  // the (0, 0, 0) slot of every layout
   obs_trace_kernel<<<nblk, 256, 0, st>>>(p.d_obs_idx, m, exact ? S.zqc.p : nullptr, ns, centre, S.trc.p, V, nh1,
                                          S.part.p);
-  const double tr = host_sum_partials(S.part.p, nblk, st);
+  API_CUDA(cudaMemcpyAsync(g.data(), S.gradv.p, (ntheta - 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
+  double tr = 0.0;
+  host_sum_partials(S.part.p, nblk, st, &tr);
   plog.mark("gradient", st);
   p.launches_total += 5 + (hutch ? 1 : 0);  // gbar, adjoint (3), obs trace, probe difference
   API_CUDA(cudaGetLastError());
@@ -1056,7 +1090,8 @@ int spde_loglike_grad_pcg(SpdePlan* plan, double tau, const double* y, int r, co
   if ((rc = solve(1, w_qc, V, S.trc.p, nh1))) return rc;
   obs_resid_kernel<<<int((int64_t(m) * r + 255) / 256), 256, 0, st>>>(p.d_obs_idx, m, r, y, S.mu.p, S.d.p);
   dot_partial_kernel<<<nblk, 256, 0, st>>>(S.d.p, nullptr, int64_t(m) * r, S.part.p);
-  const double rss = host_sum_partials(S.part.p, nblk, st);
+  double rss = 0.0;
+  host_sum_partials(S.part.p, nblk, st, &rss);
   {
     const int64_t tot = int64_t(n) * nh1;
     sub_kernel<<<int((tot + 255) / 256), 256, 0, st>>>(S.trq.p, S.trc.p, tot);
@@ -1073,7 +1108,8 @@ int spde_loglike_grad_pcg(SpdePlan* plan, double tau, const double* y, int r, co
   API_CUDA(cudaMemcpyAsync(g.data(), S.gradv.p, (ntheta - 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
   const int centre = p.sym.nslots / 2;  // the (0, 0, 0) slot of every layout
   obs_trace_kernel<<<nblk, 256, 0, st>>>(p.d_obs_idx, m, nullptr, ns, centre, S.trc.p, V, nh1, S.part.p);
-  const double tr = host_sum_partials(S.part.p, nblk, st);
+  double tr = 0.0;
+  host_sum_partials(S.part.p, nblk, st, &tr);
   API_CUDA(cudaGetLastError());
   g[ntheta - 1] = m * r / 2.0 - 0.5 * r * tau * tr / nh1 - tau / 2 * rss;
   for (int i = 0; i < ntheta; ++i) jac[i] = -g[i] / (double(m) * r);

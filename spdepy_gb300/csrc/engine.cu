@@ -1301,6 +1301,7 @@ struct Exec {
   const Schedule& s;
   int nrhs;
   double* zq;
+  cudaStream_t st;
   T* buf(int id) const {
     switch (id) {
       case B_L: return static_cast<T*>(p->d_L);
@@ -1317,7 +1318,6 @@ struct Exec {
     }
   }
   void run() {
-    cudaStream_t st = p->stream;
     // optional per-depth timeline (SPDE_PHASE_LOG): an event at every change of depth
     static const bool depth_log = std::getenv("SPDE_PHASE_LOG") != nullptr;
     std::vector<std::pair<int, cudaEvent_t>> dmarks;
@@ -1421,7 +1421,6 @@ struct Exec {
       for (auto& m : dmarks) cudaEventDestroy(m.second);
       std::fprintf(stderr, "%s\n", line.c_str());
     }
-    p->launches_total += s.launches;
   }
 };
 
@@ -1637,16 +1636,15 @@ int plan_build(Plan* p) {
 }
 
 // Reads and clears the FP64 tensor-core products' wait-failure flag.
-static int emu_take_error(Plan* p) {
+static int emu_take_error(Plan* p, cudaStream_t st, int* pinned) {
   if (!p->d_emu_err) return 0;
-  int* h = p->pin_int() + 3;
-  *h = 0;
-  cudaMemcpyAsync(h, p->d_emu_err, sizeof(int), cudaMemcpyDeviceToHost, p->stream);
-  cudaStreamSynchronize(p->stream);
-  const int e = *h;
+  *pinned = 0;
+  cudaMemcpyAsync(pinned, p->d_emu_err, sizeof(int), cudaMemcpyDeviceToHost, st);
+  cudaStreamSynchronize(st);
+  const int e = *pinned;
   if (e) {
-    cudaMemsetAsync(p->d_emu_err, 0, sizeof(int), p->stream);
-    cudaStreamSynchronize(p->stream);
+    cudaMemsetAsync(p->d_emu_err, 0, sizeof(int), st);
+    cudaStreamSynchronize(st);
   }
   return e;
 }
@@ -1659,7 +1657,8 @@ static int factor_t(Plan* p, int with_obs, double tau) {
   CUDA_TRY(cudaMemsetAsync(p->d_err, 0xFF, sizeof(int), st));  // -1: no failed pivot
   launch_scatter<T>(p->qstencil(), S.nslots, p->d_amap, p->d_perm, p->d_front_of, p->d_fronts,
                     with_obs ? p->d_obs_cnt : nullptr, tau, static_cast<T*>(p->d_L), st);
-  Exec<T>{p, p->sched_factor, 0, nullptr}.run();
+  Exec<T>{p, p->sched_factor, 0, nullptr, st}.run();
+  p->launches_total += p->sched_factor.launches;
   sum_kernel<<<1, 256, 0, st>>>(p->d_logpiv, int64_t(p->sched_factor.diag.size()), p->d_scalar);
   CUDA_TRY(cudaMemcpyAsync(p->h_pin + 1024, p->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaMemcpyAsync(p->pin_int(), p->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1667,7 +1666,7 @@ static int factor_t(Plan* p, int with_obs, double tau) {
   CUDA_TRY(cudaGetLastError());
   const double sum = p->h_pin[1024];
   const int err = p->pin_int()[0];
-  if (tc_gemm_take_error(p->stream, p->pin_int() + 1) || emu_take_error(p)) {
+  if (tc_gemm_take_error(p->stream, p->pin_int() + 1) || emu_take_error(p, p->stream, p->pin_int() + 3)) {
     p->last_error = "tensor-core product timed out";
     p->factored = 0;
     return 2;
@@ -1731,8 +1730,9 @@ static void tri_solve(Plan* p, int nrhs) {
     build_bwd_schedule(p->sym, *bw, p->tile_m, p->tile_n, nrhs);
     bw->upload();
   }
-  Exec<T>{p, *fw, nrhs, nullptr}.run();
-  Exec<T>{p, *bw, nrhs, nullptr}.run();
+  Exec<T>{p, *fw, nrhs, nullptr, p->stream}.run();
+  Exec<T>{p, *bw, nrhs, nullptr, p->stream}.run();
+  p->launches_total += fw->launches + bw->launches;
 }
 
 // Reads and clears the one-column sweeps' wait-failure flag (page-locked read-back).
@@ -1816,7 +1816,8 @@ static int sample_t(Plan* p, const double* z, double* x, int nrhs) {
     bw->upload();
   }
   launch_to_new<T>(z, p->d_perm, n, nrhs, static_cast<T*>(p->d_X), st);
-  Exec<T>{p, *bw, nrhs, nullptr}.run();
+  Exec<T>{p, *bw, nrhs, nullptr, st}.run();
+  p->launches_total += bw->launches;
   launch_from_new<T>(static_cast<const T*>(p->d_X), p->d_perm, n, nrhs, x, 0, st);
   p->launches_total += 2;
   CUDA_TRY(cudaGetLastError());
@@ -1837,29 +1838,43 @@ int plan_solve(Plan* p, const double* b, double* x, int nrhs, int iters, double 
                            : solve_t<float>(p, b, x, nrhs, iters, tol, resid);
 }
 
+// The selected inversion reads the factor and writes its own pools and scratch, so
+// it may run on another stream, from another host thread, beside a solve with the
+// same factor; p->stream, p->last_error and the counters are left alone.
 template <typename T>
-static int selinv_t(Plan* p, double* zq) {
-  cudaStream_t st = p->stream;
+static int selinv_t(Plan* p, double* zq, cudaStream_t st, std::string* error) {
   const Symbolic& S = p->sym;
-  Exec<T>{p, p->sched_selinv, 0, zq}.run();
+  Exec<T>{p, p->sched_selinv, 0, zq, st}.run();
   int64_t tot = int64_t(S.n) * S.nslots;
   zsym_kernel<<<int((tot + 255) / 256), 256, 0, st>>>(S.Mx, S.Ny, S.T, S.nslots, p->d_amap, zq);
-  p->launches_total += 1;
-  CUDA_TRY(cudaStreamSynchronize(st));
-  CUDA_TRY(cudaGetLastError());
-  if (tc_gemm_take_error(p->stream, p->pin_int() + 1) || emu_take_error(p)) {
-    p->last_error = "tensor-core product timed out";
-    p->factored = 0;
+  cudaError_t e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    *error = std::string("selected inversion: ") + cudaGetErrorString(e);
     return 2;
   }
-  if (p->profile) prof_collect(p);
-  p->factored = 0;  // the factor's panels now hold intermediate products
+  if (tc_gemm_take_error(st, p->pin_int() + 5) || emu_take_error(p, st, p->pin_int() + 6)) {
+    *error = "tensor-core product timed out";
+    return 2;
+  }
   return 0;
+}
+
+int plan_selinv_on(Plan* p, double* zq, cudaStream_t st, std::string* error) {
+  return p->precision == 0 ? selinv_t<double>(p, zq, st, error) : selinv_t<float>(p, zq, st, error);
+}
+
+void plan_selinv_done(Plan* p) {
+  p->launches_total += p->sched_selinv.launches + 1;
+  p->factored = 0;  // a selected inversion ends the factor's life
 }
 
 int plan_selinv(Plan* p, double* zq) {
   if (!p->factored) { p->last_error = "no valid factor"; return 5; }
-  return p->precision == 0 ? selinv_t<double>(p, zq) : selinv_t<float>(p, zq);
+  const int rc = plan_selinv_on(p, zq, p->stream, &p->last_error);
+  if (!rc && p->profile) prof_collect(p);
+  plan_selinv_done(p);
+  return rc;
 }
 
 }  // namespace spde

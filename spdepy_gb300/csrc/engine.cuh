@@ -174,7 +174,8 @@ struct Plan {
   double* d_part = nullptr;    // block partial sums (1024)
   // page-locked host buffer for the scalars and partial sums read back during a
   // factorisation, solve or inversion: doubles 0-1023 partial sums, 1024 the
-  // log-pivot sum; ints at double 1536: the pivot error, the tensor-core flag
+  // log-pivot sum; ints at double 1536: the pivot error, the tensor-core flag, the
+  // sweeps' flag, the FP64 products' flag, and at 5 and 6 the selected inversion's two
   double* h_pin = nullptr;
   int* pin_int() { return reinterpret_cast<int*>(h_pin + 1536); }
   // model / assembly state (FP64)
@@ -255,6 +256,10 @@ int plan_build(Plan* p);
 int plan_factor(Plan* p, int with_obs, double tau);
 int plan_solve(Plan* p, const double* b_dev, double* x_dev, int nrhs, int refine_iters, double tol, double* resid);
 int plan_selinv(Plan* p, double* zq_dev);
+// the same on a stream of its own, possibly beside plan_solve on p->stream; the
+// caller calls plan_selinv_done when both have finished
+int plan_selinv_on(Plan* p, double* zq_dev, cudaStream_t st, std::string* error);
+void plan_selinv_done(Plan* p);
 int plan_sample(Plan* p, const double* z_dev, double* x_dev, int nrhs);
 void prof_collect(Plan* p);
 
