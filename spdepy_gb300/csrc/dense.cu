@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) gemm64_kernel(const GemmTask* __restrict_
 // as above.  Bound: the FP32 pipe for many tiles, latency for few.
 constexpr int kSgBk = 32, kSgRow = kSgBk + 4, kSgCol = 128 + 4;  // row strides: 16-byte rows, 4 banks apart
 constexpr int kSgOp = 128 * kSgRow;                              // floats of one operand's buffer (either layout)
-static_assert(kSgBk * kSgCol <= kSgOp, "column layout fits");
+static_assert(kSgBk * kSgCol <= kSgOp && 128 * kSgCol <= 4 * kSgOp, "column layout and the output tile fit");
 constexpr int kSgSmem = 4 * kSgOp * int(sizeof(float));
 
 template <int LAYOUT>
@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(256, 2) gemm32_kernel(const GemmTask* __restri
   };
   chain_wait();
   stage(0);
+  if (MODE == kSub || MODE == kAdd) prefetch_c<128, 256>(Cb + tk.c, tk.ldc, tk.m, tk.n, tid);
   for (int t = 0; t < nk; ++t) {
     if (t + 1 < nk) {
       stage(t + 1);
@@ -200,30 +201,23 @@ __global__ void __launch_bounds__(256, 2) gemm32_kernel(const GemmTask* __restri
     __syncthreads();
   }
   chain_trigger();
-  if (!active) return;
+  // through shared memory, so that whole rows of C are read and written
+  float* tile = sgm;
+  if (active) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = wr + sg_row<AL, 4>(ly, i);
-    if (r >= tk.m) continue;
-    float* dst = Cb + tk.c + int64_t(r) * tk.ldc;
-    float old[8];
-    if (MODE == kSub || MODE == kAdd) {
+    for (int i = 0; i < 8; ++i) {
+      float* row = tile + (wr + sg_row<AL, 4>(ly, i)) * kSgCol + wc;
+      if (BL == kRow) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int c = wc + sg_row<BL, 8>(lx, j);
-        old[j] = c < tk.n ? dst[c] : 0.f;
+        for (int j = 0; j < 8; ++j) row[lx + 8 * j] = acc[i][j];
+      } else {
+        *reinterpret_cast<float4*>(row + 8 * lx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        *reinterpret_cast<float4*>(row + 8 * lx + 4) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
       }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c = wc + sg_row<BL, 8>(lx, j);
-      if (c >= tk.n) continue;
-      if (MODE == kSub) dst[c] = old[j] - acc[i][j];
-      else if (MODE == kStore) dst[c] = acc[i][j];
-      else if (MODE == kNegStore) dst[c] = -acc[i][j];
-      else dst[c] = old[j] + acc[i][j];
-    }
   }
+  __syncthreads();
+  rows_to_global<MODE, 128, 8>(tile, kSgCol, Cb + tk.c, tk.ldc, tk.m, tk.n, warp, lane);
 }
 
 template <typename T, int MODE, int AL, int BL>

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "kernels.cuh"
+
 namespace spde {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -45,6 +47,70 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int by
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// ------------------------------------------------- C tiles of the FP32 products
+template <int MODE>
+__device__ __forceinline__ float apply_mode(float old, float v) {
+  if (MODE == kSub) return old - v;
+  if (MODE == kStore) return v;
+  if (MODE == kNegStore) return -v;
+  return old + v;
+}
+// The C tile of an updating product into L2 while the mainloop runs
+template <int COLS, int NT>
+__device__ __forceinline__ void prefetch_c(const float* C, int64_t ldc, int m, int n, int ltid) {
+  constexpr int kLines = COLS / 32;
+  for (int e = ltid; e < m * kLines; e += NT) {
+    const int r = e / kLines, c = 32 * (e - r * kLines);
+    if (c < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + r * ldc + c));
+  }
+}
+// Rows warp, warp + NW, ... of an m x n tile (rows of `ld` floats in shared memory,
+// COLS of them computed) into C, four rows in flight
+template <int MODE, int COLS, int NW>
+__device__ __forceinline__ void rows_to_global(const float* sm, int ld, float* C, int64_t ldc, int m, int n, int warp,
+                                               int lane) {
+  constexpr bool kRead = MODE == kSub || MODE == kAdd;
+  const bool vec = ((reinterpret_cast<uintptr_t>(C) & 15) == 0) && (ldc & 3) == 0;
+#pragma unroll 1
+  for (int r0 = warp; r0 < m; r0 += 4 * NW) {
+#pragma unroll
+    for (int c0 = 0; c0 < COLS; c0 += 128) {
+      const int c = c0 + 4 * lane;
+      if (vec && c0 + 128 <= n) {
+        float4 old[4];
+        if (kRead) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (r0 + u * NW < m) old[u] = *reinterpret_cast<const float4*>(C + (r0 + u * NW) * ldc + c);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (r0 + u * NW < m) {
+            const float4 v = *reinterpret_cast<const float4*>(sm + (r0 + u * NW) * ld + c);
+            *reinterpret_cast<float4*>(C + (r0 + u * NW) * ldc + c) =
+                make_float4(apply_mode<MODE>(old[u].x, v.x), apply_mode<MODE>(old[u].y, v.y),
+                            apply_mode<MODE>(old[u].z, v.z), apply_mode<MODE>(old[u].w, v.w));
+          }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {  // one column per lane
+          const int cj = c0 + lane + 32 * j;
+          float old[4];
+          if (kRead) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (r0 + u * NW < m && cj < n) old[u] = C[(r0 + u * NW) * ldc + cj];
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (r0 + u * NW < m && cj < n)
+              C[(r0 + u * NW) * ldc + cj] = apply_mode<MODE>(old[u], sm[(r0 + u * NW) * ld + cj]);
+        }
+      }
+    }
+  }
 }
 
 }  // namespace spde

@@ -204,69 +204,6 @@ __device__ __forceinline__ void acc_to_smem(uint32_t taddr, float* dst) {
     *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
                                                       __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
 }
-template <int MODE>
-__device__ __forceinline__ float apply_mode(float old, float v) {
-  if (MODE == kSub) return old - v;
-  if (MODE == kStore) return v;
-  if (MODE == kNegStore) return -v;
-  return old + v;
-}
-// The C tile of an updating product into L2 while the mainloop runs
-template <int COLS>
-__device__ __forceinline__ void prefetch_c(const float* C, int64_t ldc, int m, int n, int ltid) {
-  constexpr int kLines = COLS / 32;
-  for (int e = ltid; e < m * kLines; e += kLoad) {
-    const int r = e / kLines, c = 32 * (e - r * kLines);
-    if (c < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + r * ldc + c));
-  }
-}
-// Rows warp, warp + NW, ... of an m x n tile (rows of `ld` floats in shared memory,
-// COLS of them computed) into C, four rows in flight
-template <int MODE, int COLS, int NW>
-__device__ __forceinline__ void rows_to_global(const float* sm, int ld, float* C, int64_t ldc, int m, int n, int warp,
-                                               int lane) {
-  constexpr bool kRead = MODE == kSub || MODE == kAdd;
-  const bool vec = ((reinterpret_cast<uintptr_t>(C) & 15) == 0) && (ldc & 3) == 0;
-#pragma unroll 1
-  for (int r0 = warp; r0 < m; r0 += 4 * NW) {
-#pragma unroll
-    for (int c0 = 0; c0 < COLS; c0 += 128) {
-      const int c = c0 + 4 * lane;
-      if (vec && c0 + 128 <= n) {
-        float4 old[4];
-        if (kRead) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (r0 + u * NW < m) old[u] = *reinterpret_cast<const float4*>(C + (r0 + u * NW) * ldc + c);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (r0 + u * NW < m) {
-            const float4 v = *reinterpret_cast<const float4*>(sm + (r0 + u * NW) * ld + c);
-            *reinterpret_cast<float4*>(C + (r0 + u * NW) * ldc + c) =
-                make_float4(apply_mode<MODE>(old[u].x, v.x), apply_mode<MODE>(old[u].y, v.y),
-                            apply_mode<MODE>(old[u].z, v.z), apply_mode<MODE>(old[u].w, v.w));
-          }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {  // one column per lane
-          const int cj = c0 + lane + 32 * j;
-          float old[4];
-          if (kRead) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (r0 + u * NW < m && cj < n) old[u] = C[(r0 + u * NW) * ldc + cj];
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (r0 + u * NW < m && cj < n)
-              C[(r0 + u * NW) * ldc + cj] = apply_mode<MODE>(old[u], sm[(r0 + u * NW) * ld + cj]);
-        }
-      }
-    }
-  }
-}
-
 // ST stages: four with one CTA per SM, or two with two CTAs per SM, whose loads,
 // conversions, MMAs and epilogues then overlap.
 template <int MODE, int AL, int BL, int ST>
@@ -366,7 +303,7 @@ __global__ void __launch_bounds__(kThreads, ST == 2 ? 2 : 1) tc_gemm_kernel(cons
   } else if (warp < (kGroups * kConv + kLoad) / 32) {
     // ---------------- loaders
     const int ltid = tid - kGroups * kConv;
-    if (MODE == kSub || MODE == kAdd) prefetch_c<kTN>(C, tk.ldc, tk.m, tk.n, ltid);
+    if (MODE == kSub || MODE == kAdd) prefetch_c<kTN, kLoad>(C, tk.ldc, tk.m, tk.n, ltid);
     for (int t = 0; t < nk; ++t) {
       const int s = t % ST;
       // stage s last held chunk t - ST, read by its MMAs (B) and converters (A)
@@ -634,7 +571,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     // ---------------- loaders: TMA boxes (one elected thread) and / or cp.async
     const int ltid = tid - kPairGroups * kConv;
     if ((MODE == kSub || MODE == kAdd) && am > 0)
-      prefetch_c<256>(Cb + tk.c + int64_t(row0) * tk.ldc, tk.ldc, min(am, 128), tk.n, ltid);
+      prefetch_c<256, kLoad>(Cb + tk.c + int64_t(row0) * tk.ldc, tk.ldc, min(am, 128), tk.n, ltid);
     int issued = 0;  // chunks whose TMA boxes this thread (ltid 0) issued
     for (int t = 0; t < nk; ++t) {
       const int s = t % kStages;
