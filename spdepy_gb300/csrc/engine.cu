@@ -341,17 +341,7 @@ static void build_factor_schedule(const Symbolic& S, Schedule& sc, int TM, int T
     const auto& fr = S.by_depth[d];
     b.depth = d;
     const int pd = d & 1, pc = (d + 1) & 1;
-    // zero this depth's update blocks
-    int64_t used = 0;
-    for (int f : fr) used = std::max(used, F[f].u_off + int64_t(F[f].nb) * F[f].ldu);
-    if (used > 0) {
-      Op& o = b.begin(OP_MEMSET);
-      o.cbuf = pd == 0 ? B_P0 : B_P1;
-      o.elems = used;
-      b.end();
-    }
-    // extend-add of the children's update blocks, one launch per child rank
-    for (int rank = 0; rank < 2; ++rank) {
+    {  // the fronts' lower triangles from their children's update blocks
       Op& o = b.begin(OP_EXTEND);
       o.abuf = pc == 0 ? B_P0 : B_P1;
       o.cbuf = pd == 0 ? B_P0 : B_P1;
@@ -359,19 +349,21 @@ static void build_factor_schedule(const Symbolic& S, Schedule& sc, int TM, int T
       // elements per block: 16k, down to 2k while the level has less than eight
       // blocks per SM (a block's warps take its rows one after the other); row r
       // holds r + 1 elements: 8 rows of the long rows, up to 128 of the short ones
-      // (16, two per warp, while SMs are idle)
+      // (16, two per warp, while SMs are idle).  A front without children or without
+      // rows below its separator has only its update block to clear, or nothing.
+      auto first_row = [&](int f) { return F[f].nchild > 0 ? 0 : F[f].ns; };
       int64_t total = 0;
-      for (int f : fr)
-        if (F[f].child[rank] >= 0) total += int64_t(F[F[f].child[rank]].nb) * F[F[f].child[rank]].nb / 2;
+      for (int f : fr) {
+        const int64_t h = F[f].ns + F[f].nb, h0 = first_row(f);
+        total += (h * h - h0 * h0) / 2;
+      }
       const int chunk = int(std::max<int64_t>(2048, std::min<int64_t>(16384, total / (8 * 152))));
       for (int f : fr) {
-        int c = F[f].child[rank];
-        if (c < 0 || F[c].nb == 0) continue;
-        for (int r0 = 0; r0 < F[c].nb;) {
+        const int h = F[f].ns + F[f].nb;
+        for (int r0 = first_row(f); r0 < h;) {
           const int rows = std::max(8, std::min(chunk == 2048 ? 16 : 128, (chunk / (r0 + 1)) & ~7));
-          const int r1 = std::min(F[c].nb, r0 + rows);
-          sc.ext.push_back({c, r0, r1});
-          o.nmax = std::max(o.nmax, r1);
+          const int r1 = std::min(h, r0 + rows);
+          sc.ext.push_back({f, r0, r1});
           r0 = r1;
         }
       }
@@ -1336,8 +1328,8 @@ struct Exec {
       switch (o.kind) {
         case OP_MEMSET: cudaMemsetAsync(buf(o.cbuf), 0, size_t(o.elems) * sizeof(T), st); break;
         case OP_EXTEND:
-          launch_extend_add<T>(s.d_ext + o.off, o.count, p->d_fronts, p->d_rmap, buf(o.abuf), buf(B_L), buf(o.cbuf),
-                               o.nmax, st);
+          launch_extend<T>(s.d_ext + o.off, o.count, p->d_fronts, p->d_esrc[0], p->d_esrc[1],
+                           buf(o.abuf), buf(B_L), buf(o.cbuf), st);
           break;
         case OP_DIAG:
           launch_potrf<T>(s.d_diag + o.off, o.count, buf(B_L), buf(B_DINV), p->d_logpiv + o.off, p->d_err, st);
@@ -1560,6 +1552,24 @@ int plan_build(Plan* p) {
     d.parent = x.parent; d.depth = x.depth;
     d.child[0] = x.child[0]; d.child[1] = x.child[1];
   }
+  {  // extend-add source maps: for every front position, its index in either child's update block
+    int64_t total = 0;
+    for (size_t f = 0; f < S.fronts.size(); ++f) {
+      df[f].i_off = total;
+      total += S.fronts[f].ns + S.fronts[f].nb;
+    }
+    for (int rank = 0; rank < 2; ++rank) {
+      std::vector<int> src(size_t(std::max<int64_t>(total, 1)), -1);
+      for (size_t f = 0; f < S.fronts.size(); ++f) {
+        const int c = S.fronts[f].child[rank];
+        if (c < 0) continue;
+        const int* rm = S.rmap.data() + S.fronts[c].b_off;
+        int* dst = src.data() + df[f].i_off;
+        for (int i = 0; i < S.fronts[c].nb; ++i) dst[rm[i]] = i;
+      }
+      p->d_esrc[rank] = upload_vec(src);
+    }
+  }
   p->d_fronts = upload_vec(df);
   // the permutations come from the device ordering, checked against the
   // symbolic analysis that laid out the fronts
@@ -1579,7 +1589,7 @@ int plan_build(Plan* p) {
   p->d_blist = upload_vec(S.blist);
   p->d_rmap = upload_vec(S.rmap);
   p->d_amap = upload_vec(S.amap);
-  if (!p->d_fronts || !p->d_perm || !p->d_amap) { p->last_error = "device allocation failed (symbolic)"; return 4; }
+  if (!p->d_fronts || !p->d_perm || !p->d_amap || !p->d_esrc[0] || !p->d_esrc[1]) { p->last_error = "device allocation failed (symbolic)"; return 4; }
   const size_t es = p->esize();
   CUDA_TRY(cudaMalloc(&p->d_L, size_t(S.l_size) * es));
   CUDA_TRY(cudaMalloc(&p->d_dinv, size_t(std::max<int64_t>(S.dinv_size, 1)) * es));

@@ -150,6 +150,8 @@ struct Plan {
   DevFront* d_fronts = nullptr;
   int *d_perm = nullptr, *d_iperm = nullptr, *d_front_of = nullptr, *d_blist = nullptr, *d_rmap = nullptr;
   int* d_amap = nullptr;
+  // extend-add: per front position, its index in child 0's / child 1's update block or -1
+  int* d_esrc[2] = {nullptr, nullptr};
   // numeric arenas (element type = double for precision 0, float for 1)
   void* d_L = nullptr;
   void* d_dinv = nullptr;

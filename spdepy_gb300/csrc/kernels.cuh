@@ -72,14 +72,15 @@ struct DiagTask {
   int front;
 };
 
-// Extend-add task: rows [r0, r1) of a child's update block.
+// Extend-add task: rows [r0, r1) of a front (positions, separator first).
 struct ExtendTask {
-  int child;
+  int front;
   int r0, r1;
 };
 
 struct DevFront {
   int64_t p_off, u_off, z_off, b_off, d_off;
+  int64_t i_off;   // first entry of the front's positions in the extend-add source maps
   int64_t w_base;  // offset (per right-hand side) of this front's solve vectors in its depth pool
   int s0, ns, nb, ld, ldu, ldz, parent, depth;
   int child[2];
@@ -134,7 +135,7 @@ template <typename T>
 void launch_potrf(const DiagTask* tasks, int ntasks, T* L, T* dinv, double* logpiv, int* err, cudaStream_t st);
 
 template <typename T>
-void launch_extend_add(const ExtendTask* tasks, int ntasks, const DevFront* fronts, const int* rmap, const T* U_child,
-                       T* L, T* U_parent, int max_r1, cudaStream_t st);
+void launch_extend(const ExtendTask* tasks, int ntasks, const DevFront* fronts, const int* src0, const int* src1,
+                   const T* U_child, T* L, T* U_parent, cudaStream_t st);
 
 }  // namespace spde
