@@ -654,6 +654,54 @@ __device__ __forceinline__ DF df_fms(DF a, DF b, DF c) {
   err = __fadd_rn(err, __fsub_rn(a.lo, e));
   return df_renorm(s, err);
 }
+// Two FP32 values per register pair and instruction (add, mul and fma.rn.f32x2: each
+// half rounds as the scalar instruction does)
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2_pack(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+struct DF2 {
+  F2 hi, lo;
+};
+// df_fms for two entries: x - s a, the same roundings in the same order; ns = -s.hi,
+// and a difference u - w is formed as fma(w, -1, u), which rounds once like it
+__device__ __forceinline__ DF2 df2_fms(DF2 x, DF2 s, F2 ns, DF2 a, F2 minus1) {
+  const F2 np = f2_mul(ns, a.hi);  // -p
+  F2 e = f2_fma(s.hi, a.hi, np);
+  e = f2_fma(s.hi, a.lo, e);
+  e = f2_fma(s.lo, a.hi, e);
+  const F2 h = f2_add(x.hi, np);
+  const F2 v = f2_fma(x.hi, minus1, h);
+  F2 t = f2_fma(f2_fma(v, minus1, h), minus1, x.hi);  // x.hi - (h - v)
+  t = f2_add(t, f2_fma(v, minus1, np));
+  t = f2_add(t, f2_fma(e, minus1, x.lo));
+  const F2 r = f2_add(h, t);
+  return DF2{r, f2_fma(f2_fma(h, minus1, r), minus1, t)};
+}
 // 1 / d: FP32 reciprocal estimate refined by one Newton step with a
 // double-float residual (the step squares the estimate's relative error, so
 // the hardware approximation is enough)
@@ -699,10 +747,14 @@ __device__ __forceinline__ float df_rsqrt(DF d) {
 // advance together) beside the pivot logarithms on a fifth warp, then the
 // off-diagonal blocks by distance from the diagonal, X_ij = -X_ii (sum_{i > k >= j}
 // L_ik X_kj), the factor's entries read four at a time.
-// Measured (CUDA events, 64 x 64 blocks): one block 32 us (67 for the same sweep with
-// the columns exchanged through shared memory and the inverse by rows), 608
-// blocks 78 us (102), 1,280 blocks 124 us (239).  Three CTAs per SM: at two the
-// panel has more registers (30 us for one block) but 1,280 blocks take 143.
+// The double-float updates (14 FP32 operations each) issue in pairs of entries as
+// add, mul and fma.f32x2, half the instructions of a panel's and a trailing update's
+// chain.  Measured at 100 x 100 x 24 (mean over its launches, mostly of one to a few
+// blocks): 31.4 us, with scalar operations 36.7; the columns exchanged through shared
+// memory and the inverse by rows, without pairs, took 67 us for one block.  Two CTAs
+// per SM: with three the registers spill the pairs (32.2 us), and the levels with
+// many blocks gain nothing from the third (100 x 100 x 24 evaluation 66.4 ms both).
+// The inverse finished by idle warps during the next panel was slower (39.8 us).
 constexpr int kDfSub = 16;
 constexpr int kDfLd = kMaxNbk + 4;          // row stride of L and L^-1 in shared memory (16-byte rows)
 constexpr int kDfPan = kDfSub + 2;          // row stride of a panel in shared memory
@@ -717,7 +769,7 @@ template <>
 struct Elim<float> {
   using Num = DF;
   using Pair = float2;  // in shared memory
-  static constexpr int kMinCtas = 3;
+  static constexpr int kMinCtas = 2;
   static __device__ __forceinline__ DF from(float v) { return DF{v, 0.0f}; }
   static __device__ __forceinline__ DF load(Pair v) { return DF{v.x, v.y}; }
   static __device__ __forceinline__ Pair pack(DF v) { return make_float2(v.hi, v.lo); }
@@ -726,6 +778,15 @@ struct Elim<float> {
   }
   static __device__ __forceinline__ DF mul(DF a, DF b) { return df_mul(a, b); }
   static __device__ __forceinline__ DF fms(DF a, DF b, DF c) { return df_fms(a, b, c); }
+  // two entries at once: x0 -= s0 a0, x1 -= s1 a1
+  static __device__ __forceinline__ void fms2(DF& x0, DF& x1, DF s0, DF s1, DF a0, DF a1) {
+    const DF2 x = df2_fms(DF2{f2_pack(x0.hi, x1.hi), f2_pack(x0.lo, x1.lo)},
+                          DF2{f2_pack(s0.hi, s1.hi), f2_pack(s0.lo, s1.lo)}, f2_pack(-s0.hi, -s1.hi),
+                          DF2{f2_pack(a0.hi, a1.hi), f2_pack(a0.lo, a1.lo)}, f2_pack(-1.0f, -1.0f));
+    const float2 h = f2_unpack(x.hi), l = f2_unpack(x.lo);
+    x0 = DF{h.x, l.x};
+    x1 = DF{h.y, l.y};
+  }
   static __device__ __forceinline__ DF rcp(DF d) { return df_rcp(d); }
   static __device__ __forceinline__ float rsqrt_of(DF d) { return df_rsqrt(d); }
   static __device__ __forceinline__ bool bad(DF d) { return !(d.hi > 0.0f) || !isfinite(d.hi); }
@@ -743,6 +804,10 @@ struct Elim<double> {
   static __device__ __forceinline__ double shfl(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
   static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
   static __device__ __forceinline__ double fms(double a, double b, double c) { return fma(-b, c, a); }
+  static __device__ __forceinline__ void fms2(double& x0, double& x1, double s0, double s1, double a0, double a1) {
+    x0 = fma(-s0, a0, x0);
+    x1 = fma(-s1, a1, x1);
+  }
   // 1 / d for d > 0: the FP32 reciprocal of the significand and two Newton steps
   // (four FP64 operations instead of a full division on the narrow pipe); pivots
   // outside the normal range of d and 1 / d take the division
@@ -835,8 +900,10 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
           pan[row][j] = E::pack(x[j]);
           mul[row][j] = E::pack(sj);
         }
+        if (j % 2 == 0 && j < 15) x[j + 1] = E::fms(x[j + 1], sj, E::shfl(x[j], j + 1));
 #pragma unroll
-        for (int k = j + 1; k < 16; ++k) x[k] = E::fms(x[k], sj, E::shfl(x[j], k));
+        for (int k = (j + 2) & ~1; k < 16; k += 2)
+          E::fms2(x[k], x[k + 1], sj, sj, E::shfl(x[j], k), E::shfl(x[j], k + 1));
       }
       if (warp == 0 && lane < cw) {
         dp[c0 + lane] = E::pack(piv);
@@ -859,13 +926,21 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
             *reinterpret_cast<float4*>(sv[m]) = *reinterpret_cast<const float4*>(&mul[ty + 16 * m][c]);
             *reinterpret_cast<float4*>(av[m]) = *reinterpret_cast<const float4*>(&pan[tx + 16 * m][c]);
           }
+          auto s_of = [&](int m, int h) { return E::load(sv[m][h]); };
+          auto a_of = [&](int q, int h) { return E::load(av[q][h]); };
 #pragma unroll
-          for (int m = n + 1; m < 4; ++m)
-#pragma unroll
-            for (int q = n + 1; q <= m; ++q) {
-              r[m][q] = E::fms(r[m][q], E::load(sv[m][0]), E::load(av[q][0]));
-              r[m][q] = E::fms(r[m][q], E::load(sv[m][1]), E::load(av[q][1]));
+          for (int h = 0; h < 2; ++h) {
+            if (n == 0) {
+              E::fms2(r[2][1], r[2][2], s_of(2, h), s_of(2, h), a_of(1, h), a_of(2, h));
+              E::fms2(r[3][1], r[3][2], s_of(3, h), s_of(3, h), a_of(1, h), a_of(2, h));
+              E::fms2(r[1][1], r[3][3], s_of(1, h), s_of(3, h), a_of(1, h), a_of(3, h));
+            } else if (n == 1) {
+              E::fms2(r[2][2], r[3][2], s_of(2, h), s_of(3, h), a_of(2, h), a_of(2, h));
+              r[3][3] = E::fms(r[3][3], s_of(3, h), a_of(3, h));
+            } else if (n == 2) {
+              r[3][3] = E::fms(r[3][3], s_of(3, h), a_of(3, h));
             }
+          }
         }
       }
     };
