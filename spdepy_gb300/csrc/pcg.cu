@@ -681,7 +681,9 @@ __device__ __forceinline__ float warp_sum(float v) {
 // columns per thread share the coefficients' loads and the index arithmetic.
 // Measured at 200 x 200 x 24: 16 columns 155 us (417 with one column per thread), at
 // 400 x 400 x 48 one column 178 us (228); with a branch per neighbour instead of
-// a zero coefficient 356 us for the 16 columns.
+// a zero coefficient 356 us for the 16 columns.  Long runs of steps of one column go
+// to spmv32_steps_kernel below; with four columns its registers leave too few warps
+// (171 us against 155).
 template <int V, int SEP>
 __global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, float qe, float qm, float qo,
                                                         Walk wk, int lead, int gpad, const float* __restrict__ cf,
@@ -776,6 +778,175 @@ __global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, f
       if (lane == 0) part[int64_t(c0 + v) * gpad + g] = w;
     }
   }
+}
+
+// The same product for one column, a thread taking one cell through the time steps
+// [t0, t1) of its CTA: the 43 coefficients (25 separable), which are the same at every
+// interior step, stay in registers, and so do the 3 x 3 values around the cell that
+// the next two steps read again, so that a step loads 25 values instead of 86.
+// Every entry's products are added in spmv32_kernel's order.  With DOT (Ns % 32 = 0: a warp's
+// nodes are a warp group) also the groups' sums of p . ap into part; otherwise
+// group_dot_kernel forms them.
+// Bound: latency, the loads in flight of 24 warps per SM (three CTAs; at two 175 us
+// without spills, at four 152); the values two steps ahead are fetched to L2
+// (130 us without).  Measured at 400 x 400 x 48: 124 us, spmv32_kernel 177.
+// Warps take runs of 32 cells as in Walk, with P runs per time step (the last one ragged).
+struct CellWalk {
+  int R, P, bx, steps;  // runs per grid row and per time step, CTAs per time step, time steps per CTA
+};
+constexpr int kAhead = 2;               // time steps between a value's fetch to L2 and its use
+constexpr int kStepsCtas = 2 * 3 * 152;  // CTAs that the chunks of time steps are to leave
+// Fewer steps per CTA than this do not pay for the coefficients' loads and, where the
+// groups' sums take a launch of their own, for that launch (6 us at 10^6 nodes).
+// Measured, against spmv32_kernel: 24 steps (400 x 400 x 48) 124 / 177 us, 5 (201 x 150 x
+// 36, sums apart) 30.3 / 31.1, 4 (301 x 299 x 12, sums apart) 34 / 32, 1 (48 x 40 x 24) 6.3 / 6.1.
+constexpr int kStepsMin = 5;
+template <int SEP, int DOT>
+__global__ void __launch_bounds__(256, 3) spmv32_steps_kernel(int Mx, int Ny, int T, float qe, float qm, float qo,
+                                                              CellWalk wk, int lead, int gpad,
+                                                              const float* __restrict__ cf,
+                                                              const float* __restrict__ o32,
+                                                              const float* __restrict__ pv, float* __restrict__ apv,
+                                                              float* __restrict__ part) {
+  const int Ns = Mx * Ny, n = Ns * T, lane = threadIdx.x & 31;
+  const int by = int(blockIdx.x) / wk.bx, cta = int(blockIdx.x) - by * wk.bx;
+  const int ry = cta / wk.R;
+  const int a = (cta - ry * wk.R) + wk.R * (8 * ry + int(threadIdx.x >> 5));
+  if (a >= wk.P) return;
+  const int t0 = by * wk.steps, t1 = min(T, t0 + wk.steps);
+  const int col = lead + int(blockIdx.y);
+  const float* x = pv + int64_t(col) * n;
+  float* out = apv + int64_t(col) * n;
+  const bool mine = 32 * a + lane < Ns;  // the last run's other lanes repeat the last cell and store nothing
+  const int c = min(32 * a + lane, Ns - 1);
+  const int cy = c / Mx, cx = c - cy * Mx;
+  // A neighbour outside the grid counts with coefficient zero on a value inside it.
+  int xo[5], yo[5];
+  bool xi[5], yi[5];
+#pragma unroll
+  for (int d = 0; d < 5; ++d) {
+    xi[d] = cx + d - 2 >= 0 && cx + d - 2 < Mx;
+    yi[d] = cy + d - 2 >= 0 && cy + d - 2 < Ny;
+    xo[d] = xi[d] ? d - 2 : 0;
+    yo[d] = yi[d] ? (d - 2) * Mx : 0;
+  }
+  const float* cc = cf + c;
+  float qd[25], qn[9], qp[9], qs = 0.f;
+  auto load_diag = [&](int sb) {
+#pragma unroll
+    for (int s = 0; s < 25; ++s) {
+      const float q = cc[(sb + s) * Ns];
+      qd[s] = (xi[s % 5] && yi[s / 5]) ? q : 0.f;
+    }
+  };
+  if (SEP) {
+    load_diag(25);
+  } else {
+    qs = cc[68 * Ns];
+#pragma unroll
+    for (int s = 0; s < 9; ++s) {
+      const bool in = xi[s % 3 + 1] && yi[s / 3 + 1];
+      const float u = cc[(50 + s) * Ns], w = cc[(59 + s) * Ns];
+      qn[s] = in ? u : 0.f;
+      qp[s] = in ? w : 0.f;
+    }
+  }
+  auto ahead = [&](int t) {
+    if (t >= T) return;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (t * Ns + c)));
+    if (o32) asm volatile("prefetch.global.L2 [%0];" ::"l"(o32 + (t * Ns + c)));
+  };
+  // the 3 x 3 values around the cell at time t
+  auto inner = [&](int t, float (&v)[9]) {
+    const float* xt = x + (t * Ns + c);
+#pragma unroll
+    for (int s = 0; s < 9; ++s) v[s] = xt[yo[s / 3 + 1] + xo[s % 3 + 1]];
+  };
+  // the diagonal block (25 neighbours) at time t, whose inner values are u
+  auto block25 = [&](int t, const float (&u)[9]) {
+    const float* xt = x + (t * Ns + c);
+    float acc = 0.f;
+#pragma unroll
+    for (int s = 0; s < 25; ++s) {
+      const int dx = s % 5, dy = s / 5;
+      const bool in3 = dx >= 1 && dx <= 3 && dy >= 1 && dy <= 3;
+      acc = fmaf(qd[s], in3 ? u[in3 ? 3 * (dy - 1) + dx - 1 : 0] : xt[yo[dy] + xo[dx]], acc);
+    }
+    return acc;
+  };
+  auto finish = [&](int t, float x0, float acc) {
+    const int k = t * Ns + c;
+    if (o32) acc = fmaf(o32[k], x0, acc);
+    if (mine) out[k] = acc;
+    if (DOT) {
+      const float w = warp_sum(__fmul_rn(x0, acc));
+      if (lane == 0) part[int64_t(col) * gpad + t * wk.P + a] = w;
+    }
+  };
+  if (SEP) {
+    // Q = Qt (x) Qs: Qt_tt (Qs x_t) + Qt_off (Qs x_(t-1) + Qs x_(t+1)), every Qs x_t formed once
+    float u[9], sp = 0.f;
+    if (t0 > 0) {
+      inner(t0 - 1, u);
+      sp = block25(t0 - 1, u);
+    }
+    inner(t0, u);
+    float x0 = u[4], sc = block25(t0, u);
+    for (int t = t0; t < t1; ++t) {
+      ahead(t + 1 + kAhead);
+      float xn = 0.f, sn = 0.f;
+      if (t + 1 < T) {
+        inner(t + 1, u);
+        xn = u[4];
+        sn = block25(t + 1, u);
+      }
+      float acc = (t == 0 || t == T - 1 ? qe : qm) * sc;
+      acc = fmaf(qo, sp, acc);
+      acc = fmaf(qo, sn, acc);
+      finish(t, x0, acc);
+      sp = sc;
+      sc = sn;
+      x0 = xn;
+    }
+  } else {
+    float pr[9], cu[9], nx[9];
+    inner(t0, cu);
+    if (t0 > 0) inner(t0 - 1, pr);
+    for (int t = t0; t < t1; ++t) {
+      if (t == t0 || t == 1) load_diag(t == 0 && T > 1 ? 0 : 25);
+      ahead(t + kAhead);
+      if (t + 1 < T) inner(t + 1, nx);
+      float acc = block25(t, cu);
+      if (t + 1 < T) {
+        acc = fmaf(qs, cu[4], acc);
+#pragma unroll
+        for (int s = 0; s < 9; ++s) acc = fmaf(qn[s], nx[s], acc);
+      }
+      if (t > 0) {
+#pragma unroll
+        for (int s = 0; s < 9; ++s) acc = fmaf(qp[s], pr[s], acc);
+      }
+      finish(t, cu[4], acc);
+#pragma unroll
+      for (int s = 0; s < 9; ++s) {
+        pr[s] = cu[s];
+        cu[s] = nx[s];
+      }
+    }
+  }
+}
+
+// The warp groups' sums of p . ap for the columns lead + y, one warp per group.  Bound:
+// memory (8 bytes per node).
+__global__ void __launch_bounds__(256) group_dot_kernel(int n, int ngroups, int lead, int gpad,
+                                                        const float* __restrict__ pv, const float* __restrict__ apv,
+                                                        float* __restrict__ part) {
+  const int g = int(blockIdx.x) * 8 + int(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (g >= ngroups) return;
+  const int64_t col = lead + int(blockIdx.y);
+  const int k = 32 * g + lane;
+  const float w = warp_sum(k < n ? __fmul_rn(pv[col * n + k], apv[col * n + k]) : 0.f);
+  if (lane == 0) part[col * gpad + g] = w;
 }
 
 // Diagonal of A at node (cell c, time t) from the FP32 coefficients
@@ -1639,9 +1810,35 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   for (int c = 0; c < nrhs; ++c) all_done = (c == 0 || all_done) && hd[c];
   while (it < maxit && !all_done) {
     by_groups([&](auto vw, int lead, int groups) {
-      dim3 grid;
-      const Walk wk = walk(groups, &grid);
       constexpr int V = decltype(vw)::value;
+      dim3 grid;
+      if (V == 1) {
+        CellWalk cw;
+        cw.P = (Ns + 31) / 32;
+        cw.R = std::max(1, std::min(cw.P, (Mx + 16) / 32));
+        cw.bx = cw.R * (((cw.P + cw.R - 1) / cw.R + 7) / 8);
+        // few chunks of time steps, but kStepsCtas CTAs
+        const int64_t per = int64_t(cw.bx) * groups;
+        const int chunks = int(std::min<int64_t>(T, (kStepsCtas + per - 1) / per));
+        cw.steps = (T + chunks - 1) / chunks;
+        if (cw.steps >= kStepsMin) {
+          grid = dim3(cw.bx * ((T + cw.steps - 1) / cw.steps), groups);
+          auto product = [&](auto sp, auto dot) {
+            spmv32_steps_kernel<decltype(sp)::value, decltype(dot)::value><<<grid, 256, 0, st>>>(
+                Mx, Ny, T, qe, qm, qo, cw, lead, gpad, cf, o, p32, ap32, gsum);
+          };
+          const bool dot = Ns % 32 == 0;
+          if (sep && dot) product(IntC<1>{}, IntC<1>{});
+          else if (sep) product(IntC<1>{}, IntC<0>{});
+          else if (dot) product(IntC<0>{}, IntC<1>{});
+          else product(IntC<0>{}, IntC<0>{});
+          if (!dot)
+            group_dot_kernel<<<dim3((ngroups + 7) / 8, groups), 256, 0, st>>>(int(n), ngroups, lead, gpad, p32, ap32,
+                                                                              gsum);
+          return;
+        }
+      }
+      const Walk wk = walk(groups, &grid);
       if (sep)
         spmv32_kernel<V, 1><<<grid, 256, 0, st>>>(Mx, Ny, T, qe, qm, qo, wk, lead, gpad, cf, o, p32, ap32, gsum);
       else

@@ -62,3 +62,21 @@ def test_true_residual_separable(M, N, T, nrhs):
     x, _, _ = mod.plan.pcg(torch.as_tensor(b), False, 0.0, "jacobi", tol=1e-9, maxit=20000)
     res = np.linalg.norm(b - A @ x.cpu().numpy().reshape(n, nrhs), axis=0)
     assert (res <= 1e-9 * (1 + 1e-6) * np.linalg.norm(b, axis=0)).all()
+
+
+@pytest.mark.parametrize("M,N,T,separable", [(8, 4, 3652, False), (11, 3, 3652, False), (11, 3, 3652, True),
+                                             (8, 4, 3650, True), (129, 67, 105, False)])
+def test_one_column_through_time(M, N, T, separable):
+    """Long runs of time steps of a single column keep the coefficients in registers; the
+    column's arithmetic is that of any other grouping, so the solutions are the same bits."""
+    mod = _plan(M, N, T, separable=separable)
+    n, plan = mod.grid.n, mod.plan
+    rng = np.random.default_rng(n)
+    plan.set_obs(np.sort(rng.choice(n, n // 7, replace=False)))
+    b = torch.as_tensor(rng.normal(size=(n, 1)))
+    one, it1, rel1 = plan.pcg(b, True, 3.0, "jacobi", tol=1e-9, maxit=20000)
+    two, it2, rel2 = plan.pcg(b.repeat(1, 2), True, 3.0, "jacobi", tol=1e-9, maxit=20000)
+    one, two = one.cpu().numpy().reshape(n), two.cpu().numpy().reshape(n, 2)
+    assert it1 == it2
+    assert np.isfinite(one).all() and one.any()
+    assert np.array_equal(one, two[:, 0]) and np.array_equal(one, two[:, 1])
