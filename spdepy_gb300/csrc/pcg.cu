@@ -949,10 +949,12 @@ __global__ void __launch_bounds__(256) group_dot_kernel(int n, int ngroups, int 
   if (lane == 0) part[col * gpad + g] = w;
 }
 
-// Diagonal of A at node (cell c, time t) from the FP32 coefficients
+// Diagonal of A at node (cell c, time t) from the FP32 coefficients.  The separable
+// product rounds by itself, whatever is added to it, so that a column's bits do not depend
+// on how many columns go together.
 __device__ __forceinline__ float diag32(const float* __restrict__ cf, int Ns, int T, int sep, float qe, float qm,
                                         int c, int t) {
-  if (sep) return (t == 0 || t == T - 1 ? qe : qm) * cf[int64_t(25 + 12) * Ns + c];
+  if (sep) return __fmul_rn(t == 0 || t == T - 1 ? qe : qm, cf[int64_t(25 + 12) * Ns + c]);
   if (T == 1) return cf[int64_t(25 + 12) * Ns + c];
   if (t == 0) return cf[int64_t(12) * Ns + c] + cf[int64_t(68) * Ns + c];
   return cf[int64_t(25 + 12) * Ns + c] + (t < T - 1 ? cf[int64_t(68) * Ns + c] : 0.f);
