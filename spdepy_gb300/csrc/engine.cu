@@ -1602,12 +1602,18 @@ int plan_build(Plan* p) {
   int64_t sx_elems = 0;
   build_factor_schedule(S, p->sched_factor, TM, TM, pairs, emu);
   build_selinv_schedule(S, p->sched_selinv, TM, TM, &sx_elems, pairs, emu);
+  CUDA_TRY(cudaMalloc(&p->d_sx, size_t(sx_elems) * es));
   if (emu) {
-    // digits and row exponents of the largest launch; without the memory the
-    // products stay on the CUDA cores
+    // digits and row exponents of the largest launch.  They are taken only if that leaves as
+    // much memory free as the arenas hold (a second pipeline, the solves' vectors), so
+    // that they never make a call fail; without them the products stay on the CUDA cores
     const int64_t bytes = std::max(p->sched_factor.emu_bytes, p->sched_selinv.emu_bytes);
     const int64_t rows = std::max(p->sched_factor.emu_rows, p->sched_selinv.emu_rows);
-    if (bytes > 0 && (cudaMalloc(&p->d_emu, size_t(bytes)) != cudaSuccess ||
+    const size_t arenas = size_t(S.l_size + S.dinv_size + p->pool_elems[0] + p->pool_elems[1] + sx_elems) * es;
+    size_t room = 0, total = 0;
+    if (bytes > 0 && (cudaMemGetInfo(&room, &total) != cudaSuccess ||
+                      room < size_t(bytes) + size_t(rows) * sizeof(int) + arenas ||
+                      cudaMalloc(&p->d_emu, size_t(bytes)) != cudaSuccess ||
                       cudaMalloc(&p->d_emu_exp, size_t(rows) * sizeof(int)) != cudaSuccess ||
                       cudaMalloc(&p->d_emu_err, sizeof(int)) != cudaSuccess)) {
       cudaGetLastError();
@@ -1622,7 +1628,6 @@ int plan_build(Plan* p) {
       CUDA_TRY(cudaMemset(p->d_emu_err, 0, sizeof(int)));
     }
   }
-  CUDA_TRY(cudaMalloc(&p->d_sx, size_t(sx_elems) * es));
   if (pairs) {
     const int64_t sizes[] = {S.l_size, p->pool_elems[0], p->pool_elems[1], sx_elems};
     encode_maps(p, p->sched_factor, sizes);
