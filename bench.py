@@ -65,8 +65,8 @@ def _tf32_tflops(torch, n=8192, reps=10):
 
 
 def _dgemm_tflops(torch, n=4096, reps=5):
-    """cuBLAS FP64 GEMM, best of `reps`: the ceiling of the FP64 plan's dense
-    products (the plain FP64 path the mixed plan is compared with)."""
+    """cuBLAS FP64 GEMM, best of `reps`: a library product in FP64, beside the FP64
+    plan's dense products (whose digit products on the tensor cores are not bound by the FP64 pipe)."""
     try:
         a = torch.randn(n, n, device="cuda", dtype=torch.float64)
         b = torch.randn(n, n, device="cuda", dtype=torch.float64)

@@ -29,7 +29,7 @@ extern "C" {
 #define SPDE_ERR_STATE 5
 #define SPDE_ERR_NOT_CONVERGED 6
 
-#define SPDE_PRECISION_FP64 0 /* factor, solves and inverse in FP64 */
+#define SPDE_PRECISION_FP64 0 /* factor, solves and inverse in FP64 (products from exact digit products, rounded to FP64) */
 #define SPDE_PRECISION_MIXED 1 /* FP32 factor, FP64 pivots / log-det / refinement */
 #define SPDE_PRECISION_ITERATIVE 2 /* no factorisation: assembly, products, PCG */
 
@@ -133,7 +133,7 @@ int spde_plan_read_sites(SpdePlan* plan, double* ms, double* flops, int64_t* til
  * factorisations' latency-bound top levels overlap; it doubles the factor and
  * inverse memory.  Each pipeline then runs its factorisation and solve on a
  * greatest-priority stream and its inversion on a least-priority stream of the
- * plan, ordered after the work already on the plan's stream and joined back to
+ * plan (that of Q + tau S^T S beside the solve, which reads the factor only), ordered after the work already on the plan's stream and joined back to
  * it before spde_loglike returns.  1 runs them one after the other on the plan's
  * stream and one set of arenas. */
 int spde_plan_set_pipelines(SpdePlan* plan, int pipelines);
