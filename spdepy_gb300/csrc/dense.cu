@@ -252,6 +252,10 @@ static void gemm_mode(const GemmTask* t, int n, const T* A, const T* B, T* C, in
 // writes C (in-place solves stay valid).
 constexpr int kNarrowN = 8;
 constexpr int kNarrowBEnt = 2048;  // shared entries: staged B (NB x k chunk), then the k-split partial sums
+// Column layout: loads in flight per thread.  Measured over the 54 launches of a 301 x 203
+// evaluation with four right-hand sides: with 8, and a chunk's last ones one at a time,
+// 1,468 us; 8 in every round 796; 16 697 (the evaluation: 5.29, 4.77, 4.68 ms; 32 4.73).
+constexpr int kNarrowRows = 16;
 
 // Sum of v[r] over the 32 lanes of the warp for the eight rows r: lanes with
 // (lane >> 2) == r receive row r (a butterfly that halves the rows each lane
@@ -375,7 +379,8 @@ __global__ void __launch_bounds__(256) gemv_kernel(const GemmTask* __restrict__ 
       }
     }
   } else {
-    // thread (h, i): row i, every H-th k value starting at h; 8 loads in flight
+    // thread (h, i): row i, every H-th k value starting at h; kNarrowRows loads in flight, also
+    // in the last ones of a chunk (past it a load repeats its last value and is dropped)
     const int rsh = m <= 32 ? 5 : (m <= 64 ? 6 : 7);
     const int i = tid & ((1 << rsh) - 1), h = tid >> rsh, H = 256 >> rsh;
     T s[NB];
@@ -393,20 +398,15 @@ __global__ void __launch_bounds__(256) gemv_kernel(const GemmTask* __restrict__ 
       __syncthreads();
       if (i < m) {
         const T* ac = A + int64_t(k0) * tk.lda + i;
-        int kk = h;
-        for (; kk + 7 * H < kn; kk += 8 * H) {
-          T a[8];
+        for (int kk = h; kk < kn; kk += kNarrowRows * H) {
+          T a[kNarrowRows];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) a[u] = ac[int64_t(kk + u * H) * tk.lda];
+          for (int u = 0; u < kNarrowRows; ++u) a[u] = ac[int64_t(min(kk + u * H, kn - 1)) * tk.lda];
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
+          for (int u = 0; u < kNarrowRows; ++u)
+            if (kk + u * H < kn)
 #pragma unroll
-            for (int j = 0; j < NB; ++j) s[j] = fma(a[u], sh[j * kc + kk + u * H], s[j]);
-        }
-        for (; kk < kn; kk += H) {
-          const T a = ac[int64_t(kk) * tk.lda];
-#pragma unroll
-          for (int j = 0; j < NB; ++j) s[j] = fma(a, sh[j * kc + kk], s[j]);
+              for (int j = 0; j < NB; ++j) s[j] = fma(a[u], sh[j * kc + kk + u * H], s[j]);
         }
       }
     }
