@@ -740,7 +740,10 @@ __device__ __forceinline__ float df_rsqrt(DF d) {
 // rows below its diagonal block: lanes 0-15 hold the diagonal block's rows (the
 // same in every warp), lanes 16-31 the warp's own rows, one row per lane in
 // registers, so that pivots and multipliers travel by shuffle and no warp waits for
-// another inside a panel.  The trailing rank-16 update is spread over all 256
+// another inside a panel.  Between the two barriers around a panel a warp writes only
+// rows that no other warp reads there: its own rows in place, and the diagonal block's,
+// which every warp loads, into the same rows of the other panel buffer, where the next
+// panel writes only rows below them.  The trailing rank-16 update is spread over all 256
 // threads, each holding the entries (ty + 16 m, tx + 16 n), n <= m, in registers.
 // Then L^-1 (FP32) by 16-column sub-blocks: the four diagonal inverses (a warp
 // each, one lane per column, right-looking so that the partial sums of all rows
@@ -869,6 +872,7 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
   if (tid == 0) bad = 0;
   for (int jb = 0; 16 * jb < w; ++jb) {
     Pair (*pan)[kDfPan] = pan0 + (jb & 1) * kMaxNbk;
+    Pair (*fin)[kDfPan] = pan0 + (~jb & 1) * kMaxNbk;  // takes the panel's finished diagonal rows
     const int c0 = 16 * jb, cw = min(kDfSub, w - c0);
     // block column jb to shared memory (the register indices are compile-time constants)
 #pragma unroll
@@ -897,7 +901,7 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
         if (lane == j) piv = d;
         failed |= nonpos && j < cw;
         if (own) {
-          pan[row][j] = E::pack(x[j]);
+          (lane < 16 ? fin : pan)[row][j] = E::pack(x[j]);
           mul[row][j] = E::pack(sj);
         }
         if (j % 2 == 0 && j < 15) x[j + 1] = E::fms(x[j + 1], sj, E::shfl(x[j], j + 1));
@@ -915,7 +919,7 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
       constexpr int n = decltype(block)::value;
 #pragma unroll
       for (int m = n; m < 4; ++m) {  // the panel's final entries
-        r[m][n] = E::load(pan[ty + 16 * m][tx]);
+        r[m][n] = E::load((m == n ? fin : pan)[ty + 16 * m][tx]);
       }
       if (c0 + 16 < w) {
 #pragma unroll 4
