@@ -840,8 +840,8 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
 
 template <typename T>
 __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
-    potrf_kernel(const DiagTask* __restrict__ tasks, T* __restrict__ L, T* __restrict__ dinv,
-                 double* __restrict__ logpiv, int* __restrict__ err) {
+    potrf_kernel(const DiagTask* __restrict__ tasks, T* L, T* dinv,
+                 double* logpiv, int* err) {
   using E = Elim<T>;
   using Num = typename E::Num;
   using Pair = typename E::Pair;
@@ -1084,8 +1084,7 @@ constexpr int kExtUnroll = 8;
 // ADD: dst += the children's values where there are any, else dst = their sum.
 template <typename T, int CH, bool ADD>
 __device__ __forceinline__ void extend_row(const int* __restrict__ m0, const int* __restrict__ m1,
-                                           const T* __restrict__ a0, const T* __restrict__ a1, T* __restrict__ dst,
-                                           int n, int lane) {
+                                           const T* a0, const T* a1, T* dst, int n, int lane) {
   for (int j0 = lane; j0 < n; j0 += 32 * kExtUnroll) {
     T v0[kExtUnroll], v1[kExtUnroll], o[kExtUnroll];
     int x0[kExtUnroll], x1[kExtUnroll];
@@ -1116,8 +1115,8 @@ __device__ __forceinline__ void extend_row(const int* __restrict__ m0, const int
 template <typename T>
 __global__ void __launch_bounds__(256) extend_kernel(const ExtendTask* __restrict__ tasks,
                                                      const DevFront* __restrict__ fronts, const int* __restrict__ src0,
-                                                     const int* __restrict__ src1, const T* __restrict__ Uc,
-                                                     T* __restrict__ L, T* __restrict__ Up) {
+                                                     const int* __restrict__ src1, const T* Uc,
+                                                     T* L, T* Up) {
   const ExtendTask tk = tasks[blockIdx.x];
   const DevFront f = fronts[tk.front];
   const int *m0 = src0 + f.i_off, *m1 = src1 + f.i_off;

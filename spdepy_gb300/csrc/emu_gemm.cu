@@ -96,8 +96,8 @@ __device__ __forceinline__ void split_store(const double (&v)[8], int field, boo
 }
 
 __global__ void __launch_bounds__(256) emu_split_kernel(const EmuSplit* __restrict__ tasks, const double* Ab,
-                                                        const double* Bb, uint8_t* __restrict__ planes,
-                                                        int* __restrict__ exps) {
+                                                        const double* Bb, uint8_t* planes,
+                                                        int* exps) {
   const EmuSplit tk = tasks[blockIdx.x >> 3];
   const int lane = threadIdx.x & 31, r = int(blockIdx.x & 7) * 8 + int(threadIdx.x >> 5);
   chain_wait();
@@ -173,9 +173,9 @@ __device__ __forceinline__ double emu_value(long long hi, long long lo, int e) {
 
 template <int MODE>
 __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask* __restrict__ tasks,
-                                                                  const uint8_t* __restrict__ planes,
-                                                                  const int* __restrict__ exps, double* Cb,
-                                                                  int* __restrict__ err, unsigned long long wait_ns) {
+                                                                  const uint8_t* planes,
+                                                                  const int* exps, double* Cb,
+                                                                  int* err, unsigned long long wait_ns) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full[kEmuStages], consumed[kEmuStages], dready, dfree, done;
   __shared__ uint32_t tmem_slot;

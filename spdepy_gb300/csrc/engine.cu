@@ -864,10 +864,10 @@ __device__ __forceinline__ T load_cg(const T* p) {
 // block k, flag base of the front; sorted by k).  Thread (row i, quarter q).
 template <typename T>
 __global__ void __launch_bounds__(256) fwd_chain_kernel(const RowTask* __restrict__ tasks,
-                                                        const DevFront* __restrict__ fronts, const T* __restrict__ L,
-                                                        const T* __restrict__ dinv, T* __restrict__ X,
-                                                        unsigned* __restrict__ flags, unsigned* __restrict__ counter,
-                                                        unsigned epoch, int* __restrict__ err,
+                                                        const DevFront* __restrict__ fronts, const T* L,
+                                                        const T* dinv, T* X,
+                                                        unsigned* flags, unsigned* counter,
+                                                        unsigned epoch, int* err,
                                                         unsigned long long wait_ns) {
   __shared__ T sD[64][65];
   __shared__ T ys[64], acc[64];
@@ -923,11 +923,11 @@ __global__ void __launch_bounds__(256) fwd_chain_kernel(const RowTask* __restric
 // of eight): the border term, which depends on no other block, comes first.
 template <typename T>
 __global__ void __launch_bounds__(512) bwd_chain_kernel(const RowTask* __restrict__ tasks,
-                                                        const DevFront* __restrict__ fronts, const T* __restrict__ L,
-                                                        const T* __restrict__ dinv, T* __restrict__ X,
-                                                        const T* __restrict__ G, unsigned* __restrict__ flags,
-                                                        unsigned* __restrict__ counter, unsigned epoch,
-                                                        int* __restrict__ err, unsigned long long wait_ns) {
+                                                        const DevFront* __restrict__ fronts, const T* L,
+                                                        const T* dinv, T* X,
+                                                        const T* G, unsigned* flags,
+                                                        unsigned* counter, unsigned epoch,
+                                                        int* err, unsigned long long wait_ns) {
   __shared__ T sD[64][65];
   __shared__ T xs[64], acc[64], red[8][64];
   __shared__ int ticket, fail;
@@ -1048,8 +1048,8 @@ __global__ void __launch_bounds__(512) bwd_chain_kernel(const RowTask* __restric
 // ------------------------------------------------------------ small kernels
 template <typename T>
 __global__ void sgather_fwd_kernel(const RowTask* __restrict__ tasks, const DevFront* __restrict__ F,
-                                   const int* __restrict__ rmap, T* __restrict__ X, T* __restrict__ Wd,
-                                   const T* __restrict__ Wc, int nrhs) {
+                                   const int* __restrict__ rmap, T* X, T* Wd,
+                                   const T* Wc, int nrhs) {
   const RowTask tk = tasks[blockIdx.x];
   const DevFront f = F[tk.front];
   const int nr = tk.r1 - tk.r0;
@@ -1075,7 +1075,7 @@ __global__ void sgather_fwd_kernel(const RowTask* __restrict__ tasks, const DevF
 
 template <typename T>
 __global__ void sgather_bwd_kernel(const RowTask* __restrict__ tasks, const DevFront* __restrict__ F,
-                                   const int* __restrict__ blist, const T* __restrict__ X, T* __restrict__ G,
+                                   const int* __restrict__ blist, const T* X, T* G,
                                    int nrhs) {
   const RowTask tk = tasks[blockIdx.x];
   const DevFront f = F[tk.front];
@@ -1091,7 +1091,7 @@ __global__ void sgather_bwd_kernel(const RowTask* __restrict__ tasks, const DevF
 
 template <typename T>
 __global__ void zgather_kernel(const RowTask* __restrict__ tasks, const DevFront* __restrict__ F,
-                               const int* __restrict__ rmap, const T* __restrict__ Zp, T* __restrict__ Zc) {
+                               const int* __restrict__ rmap, const T* Zp, T* Zc) {
   const RowTask tk = tasks[blockIdx.x];
   const DevFront f = F[tk.front];
   const DevFront p = F[f.parent];
@@ -1151,7 +1151,7 @@ __global__ void mirror_kernel(const MirrorTask* __restrict__ tasks, int ntasks, 
 template <typename T>
 __global__ void zextract_kernel(const RowTask* __restrict__ tasks, const DevFront* __restrict__ F,
                                 const int* __restrict__ iperm, const int* __restrict__ amap, int nslots,
-                                const T* __restrict__ Z, double* __restrict__ zq) {
+                                const T* Z, double* zq) {
   const RowTask tk = tasks[blockIdx.x];
   const DevFront f = F[tk.front];
   const int cnt = (tk.r1 - tk.r0) * nslots;
