@@ -676,7 +676,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // ap = A p in FP32 for the columns [lead + V y, + V), one thread per node and V
 // columns, and the warp groups' sums of p . ap into part[col gpad + group].  Node
-// and coefficient offsets fit in 32 bits (checked by the caller).
+// offsets fit in 32 bits (27 n does, checked by the caller), and so do those inside a group of
+// 25 coefficients; where a group starts (up to 68 Ns) they may not, with one or two time steps.
 // Bound: L1 / L2 loads (43 coefficients and 43 V vector values per node).  Four
 // columns per thread share the coefficients' loads and the index arithmetic.
 // Measured at 200 x 200 x 24: 16 columns 155 us (417 with one column per thread), at
@@ -712,28 +713,30 @@ __global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, f
       float acc[V];
       // a neighbour outside the grid counts with coefficient zero (on the node's own
       // value): no branches, so that the loads of a node overlap
-      auto add = [&](int slot, int dx, int dy, int dt, bool in) {
-        const float q = in ? cc[slot * Ns] : 0.f;
+      auto add = [&](const float* qs, int s, int dx, int dy, int dt, bool in) {
+        const float q = in ? qs[s * Ns] : 0.f;
         const Cols<V> xv = xt[in ? dt * Ns + dy * Mx + dx : 0];
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v] = fmaf(q, xv.v[v], acc[v]);
       };
       auto block25 = [&](int sb, int dt) {
         const bool vd = (vt >> (dt + 1)) & 1u;
+        const float* qs = cc + int64_t(sb) * Ns;
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v] = 0.f;
 #pragma unroll
         for (int s = 0; s < 25; ++s) {
           const int dx = s % 5 - 2, dy = s / 5 - 2;
-          add(sb + s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
+          add(qs, s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
         }
       };
       auto block9 = [&](int s0, int dt) {
         const bool vd = (vt >> (dt + 1)) & 1u;
+        const float* qs = cc + int64_t(s0) * Ns;
 #pragma unroll
         for (int s = 0; s < 9; ++s) {
           const int dx = s % 3 - 1, dy = s / 3 - 1;
-          add(s0 + s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
+          add(qs, s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
         }
       };
       if (SEP) {
@@ -752,7 +755,7 @@ __global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, f
         for (int v = 0; v < V; ++v) acc[v] = s[v];
       } else {
         block25(t == 0 && T > 1 ? 0 : 25, 0);
-        add(68, 0, 0, 0, T > 1 && t < T - 1);
+        add(cc + int64_t(68) * Ns, 0, 0, 0, 0, T > 1 && t < T - 1);
         if (T > 1) {
           block9(50, 1);
           block9(59, -1);
@@ -1110,8 +1113,8 @@ __global__ void near_rows_kernel(int Mx, int Ny, int T, GWeights gw, float* __re
     if (xq >= 0 && xq < Mx && yq >= 0 && yq < Ny && tq >= 0 && tq < T) {
       const int cq = yq * Mx + xq, q = tq * Ns + cq;
       const uint32_t m = gw.mask[q >> 5], b = 1u << (q & 31);
-      if (m & b) v = gw.w[3 * kOff * Ns + o * gw.nob + gw.rank[q >> 5] + __popc(m & (b - 1u))];
-      else v = gw.w[(time_class(tq, T) * kOff + o) * Ns + cq];
+      if (m & b) v = gw.w[int64_t(3 * kOff) * Ns + o * gw.nob + gw.rank[q >> 5] + __popc(m & (b - 1u))];
+      else v = gw.w[int64_t(time_class(tq, T) * kOff + o) * Ns + cq];
     }
     near_w[int64_t(o) * gw.ncap + i] = v;
   }
@@ -1123,7 +1126,8 @@ __global__ void near_rows_kernel(int Mx, int Ny, int T, GWeights gw, float* __re
 // row is one base, stride and neighbour shift per time offset, so that observed
 // nodes, their neighbours and the boundary differ from the interior by a
 // predicate per offset and not by another path (a warp holds several kinds).
-// Offsets fit in 32 bits (checked by the caller).  Bound: L1 / L2 loads.
+// Offsets inside a class of rows fit in 32 bits (27 n does, checked by the caller); a class starts at
+// up to 81 Ns, which may not.  Bound: L1 / L2 loads.
 // Measured at 200 x 200 x 24 with 1 % observed, 16 columns: G 101 us (413 with one
 // column per thread), G^T 150 us (1,026: near an observed node, which is in nearly
 // every warp, each of 27 weights was looked up through bitmask and rank).
@@ -1167,13 +1171,13 @@ __global__ void __launch_bounds__(256, V == 1 ? 4 : 3) g32_kernel(int Mx, int Ny
         if (word & bit) {
           const int i = (TRANS ? gw.nrank : gw.rank)[p >> 5] + __popc(word & (bit - 1u));
           stride = TRANS ? gw.ncap : gw.nob;
-          row[0] = row[1] = row[2] = (TRANS ? gw.near_w : gw.w + 3 * kOff * Ns) + i;
+          row[0] = row[1] = row[2] = (TRANS ? gw.near_w : gw.w + int64_t(3 * kOff) * Ns) + i;
         } else {
           stride = Ns;
           shift_y = TRANS ? Mx : 0;
           shift_x = TRANS ? 1 : 0;
 #pragma unroll
-          for (int d = 0; d < 3; ++d) row[d] = gw.w + time_class(TRANS ? t - (d - 1) : t, T) * kOff * Ns + c;
+          for (int d = 0; d < 3; ++d) row[d] = gw.w + int64_t(time_class(TRANS ? t - (d - 1) : t, T) * kOff) * Ns + c;
         }
       }
       float acc[V];
@@ -1254,7 +1258,7 @@ void ic_tables(IcTables* tb) {
 }
 
 // A(i, i + o) in FP32 from the coefficient copies (spatio-temporal layout)
-__device__ __forceinline__ float aval32(const float* __restrict__ cf, const float* __restrict__ o32, int Ns, int T,
+__device__ __forceinline__ float aval32(const float* __restrict__ cf, const float* __restrict__ o32, int64_t Ns, int T,
                                         int k, int c, int t, int dx, int dy, int dt) {
   if (dt == -1) return cf[(59 + (dy + 1) * 3 + dx + 1) * Ns + c];
   if (dt == 1) return cf[(50 + (dy + 1) * 3 + dx + 1) * Ns + c];
@@ -1618,7 +1622,7 @@ constexpr int kReplaceEvery = 64;
 int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const double* b, double* x, int nrhs,
               double tol, int maxit, int check_every, int* iters, double* relres) {
   const int64_t n = p->sym.n, len = n * nrhs;
-  // the stencil kernels index nodes, weights (27 n) and coefficients (69 Ns) in 32 bits
+  // the stencil kernels index nodes and the weights of one class (27 n at most) in 32 bits
   if (len >= (int64_t(1) << 31) || int64_t(p->sym.n) * kOff >= (int64_t(1) << 31) || nrhs > 65535) return 1;
   const int Mx = p->sym.Mx, Ny = p->sym.Ny, Ns = Mx * Ny, T = p->sym.T;
   cudaStream_t st = p->stream;

@@ -13,6 +13,8 @@ import tempfile
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "spdepy_gb300", "csrc")
 
+FLAGS = ["-std=c++17", "-O1", "-ffp-contract=off", "-fwrapv", "-w", "-shared", "-fPIC"]  # integers wrap as on the GPU
+
 RUNTIME = r"""
 #include <math.h>
 #include <stdint.h>
@@ -168,13 +170,12 @@ def compile_host(parts, tail):
     code = re.sub(r"asm( volatile)?\(.*?\);", ";", code, flags=re.S)
     code = code.replace("extern __shared__", "extern").replace("__shared__", "static")
     text = RUNTIME + "namespace host { Block* blk; }\n" + code + tail
-    out = os.path.join(tempfile.gettempdir(), "host_kernels_%s.so" % hashlib.sha1(text.encode()).hexdigest()[:16])
+    out = os.path.join(tempfile.gettempdir(), "host_kernels_%s.so" % hashlib.sha1((text + repr(FLAGS)).encode()).hexdigest()[:16])
     if not os.path.exists(out):
         with tempfile.TemporaryDirectory() as d:
             src, lib = os.path.join(d, "k.cpp"), os.path.join(d, "k.so")
             with open(src, "w") as f:
                 f.write(text)
-            subprocess.run(["g++", "-std=c++17", "-O1", "-ffp-contract=off", "-w", "-shared", "-fPIC", src, "-o", lib],
-                           check=True)
+            subprocess.run(["g++", *FLAGS, src, "-o", lib], check=True)
             os.replace(lib, out)
     return ctypes.CDLL(out)
