@@ -141,16 +141,22 @@ struct DevBuf {
   }
 };
 
-// Sums of nblk block partials at dpart, and (s2 not null) of the nblk after them
-void host_sum_partials(const double* dpart, int nblk, cudaStream_t st, double* s1, double* s2 = nullptr) {
+// Sums of nblk block partials at dpart, and (s2 not null) of the nblk after them; the status of
+// the copy, of the work before it on the stream, and of this thread's launches
+[[nodiscard]] cudaError_t host_sum_partials(const double* dpart, int nblk, cudaStream_t st, double* s1,
+                                            double* s2 = nullptr) {
   std::vector<double> h(2 * nblk);
-  cudaMemcpyAsync(h.data(), dpart, (s2 ? 2 : 1) * nblk * sizeof(double), cudaMemcpyDeviceToHost, st);
-  cudaStreamSynchronize(st);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(h.data(), dpart, (s2 ? 2 : 1) * nblk * sizeof(double), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return e;
   *s1 = 0.0;
   for (int i = 0; i < nblk; ++i) *s1 += h[i];
-  if (!s2) return;
+  if (!s2) return e;
   *s2 = 0.0;
   for (int i = 0; i < nblk; ++i) *s2 += h[nblk + i];
+  return e;
 }
 
 int ntheta_of(const Plan& p) { return 4 * p.model.nk + p.model.nw + 6; }
@@ -881,7 +887,12 @@ int spde_loglike(SpdePlan* plan, const double* theta, int ntheta, const double* 
       dot_partial_kernel<<<nblk, 256, 0, qc->stream>>>(S.mu.p, S.qmu.p, int64_t(n) * r, S.part.p);
       obs_resid_kernel<<<int((int64_t(m) * r + 255) / 256), 256, 0, qc->stream>>>(p.d_obs_idx, m, r, y, S.mu.p, S.d.p);
       dot_partial_kernel<<<nblk, 256, 0, qc->stream>>>(S.d.p, nullptr, int64_t(m) * r, S.part.p + nblk);
-      host_sum_partials(S.part.p, nblk, qc->stream, &muqmu, &rss);
+      // on this thread: the caller's own error state does not show a launch that failed here
+      const cudaError_t e = host_sum_partials(S.part.p, nblk, qc->stream, &muqmu, &rss);
+      if (e != cudaSuccess) {
+        qc->last_error = std::string("quadratic terms: ") + cudaGetErrorString(e);
+        rc_c = SPDE_ERR_CUDA;
+      }
     }
     if (beside) {
       inverter.join();
@@ -951,7 +962,7 @@ int spde_loglike(SpdePlan* plan, const double* theta, int ntheta, const double* 
                                          S.part.p);
   API_CUDA(cudaMemcpyAsync(g.data(), S.gradv.p, (ntheta - 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
   double tr = 0.0;
-  host_sum_partials(S.part.p, nblk, st, &tr);
+  API_CUDA(host_sum_partials(S.part.p, nblk, st, &tr));
   plog.mark("gradient", st);
   p.launches_total += 5 + (hutch ? 1 : 0);  // gbar, adjoint (3), obs trace, probe difference
   API_CUDA(cudaGetLastError());
@@ -1091,7 +1102,7 @@ int spde_loglike_grad_pcg(SpdePlan* plan, double tau, const double* y, int r, co
   obs_resid_kernel<<<int((int64_t(m) * r + 255) / 256), 256, 0, st>>>(p.d_obs_idx, m, r, y, S.mu.p, S.d.p);
   dot_partial_kernel<<<nblk, 256, 0, st>>>(S.d.p, nullptr, int64_t(m) * r, S.part.p);
   double rss = 0.0;
-  host_sum_partials(S.part.p, nblk, st, &rss);
+  API_CUDA(host_sum_partials(S.part.p, nblk, st, &rss));
   {
     const int64_t tot = int64_t(n) * nh1;
     sub_kernel<<<int((tot + 255) / 256), 256, 0, st>>>(S.trq.p, S.trc.p, tot);
@@ -1109,7 +1120,7 @@ int spde_loglike_grad_pcg(SpdePlan* plan, double tau, const double* y, int r, co
   const int centre = p.sym.nslots / 2;  // the (0, 0, 0) slot of every layout
   obs_trace_kernel<<<nblk, 256, 0, st>>>(p.d_obs_idx, m, nullptr, ns, centre, S.trc.p, V, nh1, S.part.p);
   double tr = 0.0;
-  host_sum_partials(S.part.p, nblk, st, &tr);
+  API_CUDA(host_sum_partials(S.part.p, nblk, st, &tr));
   API_CUDA(cudaGetLastError());
   g[ntheta - 1] = m * r / 2.0 - 0.5 * r * tau * tr / nh1 - tau / 2 * rss;
   for (int i = 0; i < ntheta; ++i) jac[i] = -g[i] / (double(m) * r);
