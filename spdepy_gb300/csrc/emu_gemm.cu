@@ -18,7 +18,7 @@
 // Why: FP64 is a narrow pipe on this part (two FMAs per clock and SM, 1.26 TFLOP/s),
 // while 28 bf16 products cost 28 / 2250 of it.
 //
-// Split operands lie in scratch as the shared-memory images the tensor core reads:
+// Split operands lie in memory that the plan's arenas do not use at the time, as the shared-memory images the tensor core reads:
 // [64-row tile][32-wide k chunk][digit][8-row group][8-wide k core][row][8 x bf16], 4 KB
 // per digit, so that a stage is filled by a few bulk copies.  A CTA computes a
 // 128 x 64 tile: the seven accumulators take 448 of 512 TMEM columns, and a stage (seven
@@ -44,6 +44,8 @@ constexpr int kWindow = 4;                            // chunks between two drai
 constexpr int kEpiWarps = 16;
 constexpr int kEmuThreads = (kEpiWarps + 2) * 32;     // epilogue warps, loader, MMA issuer
 constexpr unsigned long long kEmuWaitNs = 2000000000ull;
+constexpr int kFracBits = 8 * kDigits - 1;            // an operand value in units of 2^-kFracBits of its row's scale
+constexpr int kLoBits = 8 * (kDigits - 4);            // bits below the unit of the orders 0 to 3 (2^-38)
 constexpr int kNotFinite = 1 << 20;                   // row exponent of a row that holds an infinity or NaN
 
 // ------------------------------------------------------------------ split
@@ -69,12 +71,12 @@ __device__ __forceinline__ void split_store(const double (&v)[8], int field, boo
   uint32_t out[kDigits][4];
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
-    long long F = 0;  // round(x 2^(55 - e))
+    long long F = 0;  // round(x 2^(kFracBits - e))
     if (finite) {
       const long long b = __double_as_longlong(v[u]);
       const int f = int((b >> 52) & 0x7FF);
       const long long m = (b & 0xFFFFFFFFFFFFFll) | (f ? 1ll << 52 : 0ll);
-      const int sh = max(f, 1) - field + 2;
+      const int sh = max(f, 1) - field + kFracBits - 53;
       if (sh >= 0) F = m << sh;
       else if (sh >= -54) F = (m + (1ll << (-sh - 1))) >> -sh;
       if (b < 0) F = -F;
@@ -96,15 +98,14 @@ __device__ __forceinline__ void split_store(const double (&v)[8], int field, boo
 }
 
 __global__ void __launch_bounds__(256) emu_split_kernel(const EmuSplit* __restrict__ tasks, const double* Ab,
-                                                        const double* Bb, uint8_t* planes,
-                                                        int* exps) {
+                                                        const double* Bb, uint8_t* scratch) {
   const EmuSplit tk = tasks[blockIdx.x >> 3];
   const int lane = threadIdx.x & 31, r = int(blockIdx.x & 7) * 8 + int(threadIdx.x >> 5);
   chain_wait();
   if (r >= tk.rows) return;
   const double* x = (tk.buf ? Bb : Ab) + tk.src + int64_t(r) * tk.ld;
   const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  uint8_t* dst = planes + tk.dst + (r >> 3) * 512 + (r & 7) * 16;
+  uint8_t* dst = scratch + tk.dst + (r >> 3) * 512 + (r & 7) * 16;
   double v[2][8];
   unsigned top = 0;  // largest exponent field
 #pragma unroll
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(256) emu_split_kernel(const EmuSplit* __restri
   top = __reduce_max_sync(0xffffffffu, top);
   const bool finite = top != 0x7FF;
   const int field = max(int(top), 1);
-  if (lane == 0) exps[tk.exp + r] = finite ? field - 1022 : kNotFinite;
+  if (lane == 0) reinterpret_cast<int*>(scratch)[tk.exp + r] = finite ? field - 1022 : kNotFinite;
 #pragma unroll
   for (int h = 0; h < 2; ++h)
     if (8 * lane + 256 * h < 32 * tk.nch) split_store(v[h], field, finite, dst, 8 * lane + 256 * h);
@@ -154,14 +155,14 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
-// (hi 2^24 + lo) 2^e in FP64 for |hi| < 2^54, |lo| < 2^62: the leading 62 bits of the
+// (hi 2^kLoBits + lo) 2^e in FP64 for |hi| < 2^54, |lo| < 2^62: the leading 62 bits of the
 // sum (all of them up to 2^62), converted with one rounding
 __device__ __forceinline__ double emu_value(long long hi, long long lo, int e) {
-  hi += lo >> 24;
-  const long long frac = lo & 0xFFFFFF;
-  const int bits = 64 - __clzll(hi < 0 ? -hi : hi);   // |hi| < 2^bits
-  const int drop = bits > 38 ? bits - 38 : 0;         // low bits of frac left out
-  const long long v = hi * (1ll << (24 - drop)) + (frac >> drop);
+  hi += lo >> kLoBits;
+  const long long frac = lo & ((1ll << kLoBits) - 1);
+  const int bits = 64 - __clzll(hi < 0 ? -hi : hi);                 // |hi| < 2^bits
+  const int drop = bits > 62 - kLoBits ? bits - (62 - kLoBits) : 0;  // low bits of frac left out
+  const long long v = hi * (1ll << (kLoBits - drop)) + (frac >> drop);
   e += drop;
   if (v == 0) return 0.0;
   const double d = double(v);
@@ -173,9 +174,8 @@ __device__ __forceinline__ double emu_value(long long hi, long long lo, int e) {
 
 template <int MODE>
 __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask* __restrict__ tasks,
-                                                                  const uint8_t* planes,
-                                                                  const int* exps, double* Cb,
-                                                                  int* err, unsigned long long wait_ns) {
+                                                                  const uint8_t* scratch, double* Cb, int* err,
+                                                                  unsigned long long wait_ns) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full[kEmuStages], consumed[kEmuStages], dready, dfree, done;
   __shared__ uint32_t tmem_slot;
@@ -250,21 +250,21 @@ __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask*
         for (int c = 0; c < 16; ++c) {
           const int v = __float2int_rn(__uint_as_float(r[c]));
           if (o < 4) hi[c] += static_cast<long long>(v) * (1 << (24 - 8 * o));
-          else lo[c] += static_cast<long long>(v) * (1 << (8 * (6 - o)));
+          else lo[c] += static_cast<long long>(v) * (1 << (8 * (kDigits - 1 - o)));
         }
       }
     }
     chain_trigger();
     const int row = (warp & 3) * 32 + lane;
     if (ok && row < tk.m && col0 < tk.n) {
+      const int* exps = reinterpret_cast<const int*>(scratch);
       const int ea = exps[tk.ea + row];
       double* dst = Cb + tk.c + int64_t(row) * tk.ldc + col0;
 #pragma unroll
       for (int c = 0; c < 16; ++c) {
         if (col0 + c >= tk.n) break;
         const int eb = exps[tk.eb + col0 + c];
-        // hi holds units of 2^-38, lo of 2^-62 (14 + 8 o for o = 3 and 6)
-        double v = emu_value(hi[c], lo[c], ea + eb - 62);
+        double v = emu_value(hi[c], lo[c], ea + eb - 38 - kLoBits);
         if (ea == kNotFinite || eb == kNotFinite) v = __longlong_as_double(0x7FF8000000000000ll);
         if (MODE == kSub) dst[c] -= v;
         else if (MODE == kStore) dst[c] = v;
@@ -280,14 +280,14 @@ __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask*
         const int s = t % kEmuStages;
         if (t >= kEmuStages && !wait(&consumed[s], uint32_t(((t - kEmuStages) / kEmuStages) & 1), true, wait_ns)) break;
         const uint32_t d0 = smem_u32(smem + s * kStageBytes), fb = smem_u32(&full[s]);
-        const uint8_t* a = planes + tk.a + int64_t(tk.k0 + t) * kChunkBytes;
+        const uint8_t* a = scratch + tk.a + int64_t(tk.k0 + t) * kChunkBytes;
         mbar_expect_tx(fb, kStageBytes);
 #pragma unroll
         for (int p = 0; p < kDigits; ++p) {
           bulk_load(d0 + p * 2 * kBlkBytes, a + p * kBlkBytes, kBlkBytes, fb);
           bulk_load(d0 + p * 2 * kBlkBytes + kBlkBytes, a + tk.a_step + p * kBlkBytes, kBlkBytes, fb);
         }
-        bulk_load(d0 + kStageA, planes + tk.b + int64_t(tk.k0 + t) * kChunkBytes, kChunkBytes, fb);
+        bulk_load(d0 + kStageA, scratch + tk.b + int64_t(tk.k0 + t) * kChunkBytes, kChunkBytes, fb);
         issued = t + 1;
       }
       // copies still in flight (a failed wait ended the loop early) must land first
@@ -329,28 +329,28 @@ __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask*
 }
 
 template <int MODE>
-void launch_emu(const EmuTask* t, int n, const uint8_t* planes, const int* exps, double* C, int* err, cudaStream_t st,
+void launch_emu(const EmuTask* t, int n, const uint8_t* scratch, double* C, int* err, cudaStream_t st,
                 unsigned long long wait_ns) {
   static const bool attr = [] {  // once per instantiation, thread-safely
     cudaFuncSetAttribute(emu_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kEmuSmem);
     return true;
   }();
   (void)attr;
-  launch_chained(emu_gemm_kernel<MODE>, n, kEmuThreads, kEmuSmem, st, t, planes, exps, C, err, wait_ns);
+  launch_chained(emu_gemm_kernel<MODE>, n, kEmuThreads, kEmuSmem, st, t, scratch, C, err, wait_ns);
 }
 
 }  // namespace
 
 void launch_emu_gemm(const EmuSplit* splits, int nsplits, const EmuTask* tasks, int ntasks, const double* A,
-                     const double* B, double* C, int mode, uint8_t* planes, int* exps, int* err, cudaStream_t st,
+                     const double* B, double* C, int mode, uint8_t* scratch, int* err, cudaStream_t st,
                      unsigned long long wait_ns) {
   if (ntasks <= 0) return;
-  launch_chained(emu_split_kernel, 8 * nsplits, 256, 0, st, splits, A, B, planes, exps);
+  launch_chained(emu_split_kernel, 8 * nsplits, 256, 0, st, splits, A, B, scratch);
   switch (mode) {
-    case kSub: launch_emu<kSub>(tasks, ntasks, planes, exps, C, err, st, wait_ns); break;
-    case kStore: launch_emu<kStore>(tasks, ntasks, planes, exps, C, err, st, wait_ns); break;
-    case kNegStore: launch_emu<kNegStore>(tasks, ntasks, planes, exps, C, err, st, wait_ns); break;
-    default: launch_emu<kAdd>(tasks, ntasks, planes, exps, C, err, st, wait_ns); break;
+    case kSub: launch_emu<kSub>(tasks, ntasks, scratch, C, err, st, wait_ns); break;
+    case kStore: launch_emu<kStore>(tasks, ntasks, scratch, C, err, st, wait_ns); break;
+    case kNegStore: launch_emu<kNegStore>(tasks, ntasks, scratch, C, err, st, wait_ns); break;
+    default: launch_emu<kAdd>(tasks, ntasks, scratch, C, err, st, wait_ns); break;
   }
 }
 

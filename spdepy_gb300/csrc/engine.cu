@@ -82,70 +82,112 @@ struct Builder {
   explicit Builder(Schedule& sc, int tm, int tn, bool pairs = false, bool emu = false)
       : s(sc), TM(tm), TN(tn), pair_ok(pairs), emu_ok(emu) {}
 
-  // operands split by the op being built: (buffer, offset, ld, k) -> rows, digits, row exponents
-  struct EmuOperand { int rows; int64_t dst; int exp; };
+  // Where the op being built may put digits and row exponents: memory of the arenas that the
+  // op does not use (buffer, first byte, bytes).  The tensor cores take a product
+  // whenever it fits there, whole or in slices of its rows, so that the path depends on
+  // the lattice alone and takes no memory of its own.
+  struct EmuSpace { int buf = B_NONE; int64_t base = 0, bytes = 0; } emu_space;
+  // operands already split: (buffer, offset, ld, k) -> rows, digits, row exponents
+  struct EmuOperand { int rows; int64_t dst, exp; };
   std::map<std::tuple<int, int64_t, int, int>, EmuOperand> emu_operands;
+  // split and product launches of the op being built: more than one where its operands do not fit together
+  struct EmuBatch { size_t task, split; double flops; };
+  std::vector<EmuBatch> emu_batches;
   int64_t emu_cursor = 0;
-  int emu_row_cursor = 0;
-  double emu_flops = 0.0;
-  size_t emu_first = 0, esplit_first = 0;
 
+  static int64_t emu_bytes(int rows, int k) {
+    return int64_t((rows + 63) / 64) * (int64_t((k + 31) / 32) * kEmuChunkBytes + kEmuExpBytes);
+  }
+  const EmuOperand* emu_known(int buf, int64_t off, int ld, int rows, int k) const {
+    auto it = emu_operands.find(std::make_tuple(buf, off, ld, k));
+    return it != emu_operands.end() && it->second.rows >= rows ? &it->second : nullptr;
+  }
+  void emu_new_batch() {
+    emu_operands.clear();
+    emu_cursor = 0;
+    emu_batches.push_back({s.emu.size(), s.esplit.size(), 0.0});
+  }
   EmuOperand emu_operand(int buf, int which, int64_t off, int ld, int rows, int k) {
-    const auto key = std::make_tuple(buf, off, ld, k);
-    auto it = emu_operands.find(key);
-    if (it != emu_operands.end() && it->second.rows >= rows) return it->second;
-    const int nch = (k + 31) / 32;
-    EmuOperand o{rows, emu_cursor, emu_row_cursor};
-    for (int r = 0; r < rows; r += 64) {
-      s.esplit.push_back({off + int64_t(r) * ld, emu_cursor, ld, std::min(64, rows - r), k, nch, o.exp + r, which});
-      emu_cursor += nch * kEmuChunkBytes;
-    }
-    emu_row_cursor += (rows + 63) / 64 * 64;
-    emu_operands[key] = o;
+    if (const EmuOperand* known = emu_known(buf, off, ld, rows, k)) return *known;
+    const int nch = (k + 31) / 32, tiles = (rows + 63) / 64;
+    const int64_t dst = emu_space.base + emu_cursor, exp = dst + tiles * nch * kEmuChunkBytes;
+    const EmuOperand o{rows, dst, exp / 4};
+    for (int r = 0; r < rows; r += 64)
+      s.esplit.push_back({off + int64_t(r) * ld, dst + r / 64 * (nch * kEmuChunkBytes), o.exp + r, ld,
+                          std::min(64, rows - r), k, nch, which});
+    emu_cursor += emu_bytes(rows, k);
+    emu_operands[std::make_tuple(buf, off, ld, k)] = o;
     return o;
   }
-  // C (op)= A B' in 128 x 64 tiles of OP_EMU; arguments as gemm_tiles
-  void emu_tiles(int64_t a, int lda, int64_t b, int ldb, int64_t c, int ldc, int m, int n, int k, bool lower, int kt) {
+  // C (op)= A B' as products of OP_EMU (arguments as gemm_tiles); false: no space for one tile
+  bool emu_tiles(int64_t a, int lda, int64_t b, int ldb, int64_t c, int ldc, int m, int n, int k, bool lower, int kt) {
     const Op& op = s.ops.back();
-    const EmuOperand x = emu_operand(op.abuf, 0, a, lda, m, k), y = emu_operand(op.bbuf, 1, b, ldb, n, k);
-    const int64_t step = int64_t((k + 31) / 32) * kEmuChunkBytes;  // a 64-row tile
-    for (int j0 = 0; j0 < n; j0 += 64)
-      for (int i0 = lower ? j0 : 0; i0 < m; i0 += 128) {
-        int klo = 0, khi = k;
-        if (kt == KT_A_UPPER) klo = std::min(i0, k);
-        else if (kt == KT_B_LOWER) khi = std::min(k, j0 + 64);
-        else if (kt == KT_BOTH_UPPER) klo = std::min(std::max(i0, j0), k);
-        if (khi <= klo) { klo = 0; khi = std::min(k, 1); }
-        EmuTask t;
-        t.a = x.dst + i0 / 64 * step;
-        t.b = y.dst + j0 / 64 * step;
-        t.c = c + int64_t(i0) * ldc + j0;
-        t.a_step = m - i0 > 64 ? step : 0;
-        t.ldc = ldc;
-        t.m = std::min(128, m - i0);
-        t.n = std::min(64, n - j0);
-        t.k0 = klo / 32;
-        t.k1 = (khi + 31) / 32;
-        t.ea = x.exp + i0;
-        t.eb = y.exp + j0;
-        s.emu.push_back(t);
-        emu_flops += 2.0 * t.m * t.n * (khi - klo);
+    auto need = [&](int64_t oa, int ra, int64_t ob, int rb) {
+      int64_t bytes = emu_known(op.abuf, oa, lda, ra, k) ? 0 : emu_bytes(ra, k);
+      const bool same = op.abuf == op.bbuf && oa == ob && lda == ldb && rb <= ra;
+      if (!same && !emu_known(op.bbuf, ob, ldb, rb, k)) bytes += emu_bytes(rb, k);
+      return bytes;
+    };
+    // slices of A's and B's rows: all of them, or what half the space holds
+    int ra = m, rb = n;
+    if (emu_bytes(m, k) + (op.abuf == op.bbuf && a == b && lda == ldb && n <= m ? 0 : emu_bytes(n, k)) > emu_space.bytes) {
+      const int half = int(std::min<int64_t>(1 << 20, emu_space.bytes / 2 / emu_bytes(64, k))) * 64;
+      ra = std::min(m, half / 128 * 128);
+      rb = std::min(n, half);
+      if (ra < std::min(m, 128) || rb < std::min(n, 64)) return false;
+    }
+    for (int js = 0; js < n; js += rb)
+      for (int is = 0; is < m; is += ra) {
+        const int ms = std::min(ra, m - is), ns = std::min(rb, n - js);
+        if (lower && is + ms <= js) continue;  // above the diagonal
+        const int64_t as = a + int64_t(is) * lda, bs = b + int64_t(js) * ldb;
+        if (emu_batches.empty() || emu_cursor + need(as, ms, bs, ns) > emu_space.bytes) emu_new_batch();
+        const EmuOperand x = emu_operand(op.abuf, 0, as, lda, ms, k), y = emu_operand(op.bbuf, 1, bs, ldb, ns, k);
+        const int64_t step = int64_t((k + 31) / 32) * kEmuChunkBytes;  // a 64-row tile
+        for (int j0 = 0; j0 < ns; j0 += 64)
+          for (int i0 = lower && js + j0 > is ? (js + j0 - is) / 64 * 64 : 0; i0 < ms; i0 += 128) {
+            const int i = is + i0, j = js + j0;
+            int klo = 0, khi = k;
+            if (kt == KT_A_UPPER) klo = std::min(i, k);
+            else if (kt == KT_B_LOWER) khi = std::min(k, j + 64);
+            else if (kt == KT_BOTH_UPPER) klo = std::min(std::max(i, j), k);
+            if (khi <= klo) { klo = 0; khi = std::min(k, 1); }
+            EmuTask t;
+            t.a = x.dst + i0 / 64 * step;
+            t.b = y.dst + j0 / 64 * step;
+            t.c = c + int64_t(i) * ldc + j;
+            t.a_step = ms - i0 > 64 ? step : 0;
+            t.ldc = ldc;
+            t.m = std::min(128, ms - i0);
+            t.n = std::min(64, ns - j0);
+            t.k0 = klo / 32;
+            t.k1 = (khi + 31) / 32;
+            t.ea = x.exp + i0;
+            t.eb = y.exp + j0;
+            s.emu.push_back(t);
+            emu_batches.back().flops += 2.0 * t.m * t.n * (khi - klo);
+          }
       }
+    return true;
   }
-  // an OP_EMU with the tiles collected since begin(), like the op `proto`
-  void emu_op(const Op& proto) {
-    Op o = proto;
-    o.kind = OP_EMU;
-    o.tc = kPathSimt;
-    o.off = int64_t(emu_first);
-    o.count = int(s.emu.size() - emu_first);
-    o.soff = int64_t(esplit_first);
-    o.scount = int(s.esplit.size() - esplit_first);
-    o.flops = emu_flops;
-    s.ops.push_back(o);
-    s.launches += 2;
-    s.emu_bytes = std::max(s.emu_bytes, emu_cursor);
-    s.emu_rows = std::max<int64_t>(s.emu_rows, emu_row_cursor);
+  // the OP_EMUs with the tiles collected since begin(), like the op `proto`
+  void emu_ops(const Op& proto) {
+    for (size_t q = 0; q < emu_batches.size(); ++q) {
+      const EmuBatch& x = emu_batches[q];
+      const bool last = q + 1 == emu_batches.size();
+      Op o = proto;
+      o.kind = OP_EMU;
+      o.tc = kPathSimt;
+      o.sbuf = emu_space.buf;
+      o.off = int64_t(x.task);
+      o.count = int((last ? s.emu.size() : emu_batches[q + 1].task) - x.task);
+      o.soff = int64_t(x.split);
+      o.scount = int((last ? s.esplit.size() : emu_batches[q + 1].split) - x.split);
+      o.flops = x.flops;
+      s.ops.push_back(o);
+      s.launches += 2;
+    }
+    emu_batches.clear();
   }
 
   // TMA source of a row-major operand starting at element `off` of buffer `buf`,
@@ -175,12 +217,7 @@ struct Builder {
     Op& o = s.ops.back();
     o.kind = kind;
     o.depth = depth;
-    emu_operands.clear();
-    emu_cursor = 0;
-    emu_row_cursor = 0;
-    emu_flops = 0.0;
-    emu_first = s.emu.size();
-    esplit_first = s.esplit.size();
+    emu_batches.clear();
     switch (kind) {
       case OP_GEMM: o.off = int64_t(s.gemm.size()); break;
       case OP_DIAG: o.off = int64_t(s.diag.size()); break;
@@ -194,7 +231,7 @@ struct Builder {
     const Op proto = s.ops.back();
     if (proto.kind == OP_GEMM) split_by_k();
     finish(s.ops.back());
-    if (s.emu.size() > emu_first) emu_op(proto);
+    emu_ops(proto);
   }
   // Tiles with a short K (panel solves, rank-64 updates) run on the SIMT kernel,
   // the others on the tensor-core kernel: split one GEMM launch into two, the
@@ -283,10 +320,8 @@ struct Builder {
     if (m <= 0 || n <= 0 || k <= 0) return;
     const Op& op = s.ops.back();
     if (emu_ok && arow == lda && brow == ldb && op.al == kRow && op.bl == kRow && m >= kEmuMin && n >= kEmuMin &&
-        k >= kEmuMinK && i_start == 0) {
-      emu_tiles(a, lda, b, ldb, c, ldc, m, n, k, lower, kt);
+        k >= kEmuMinK && i_start == 0 && emu_tiles(a, lda, b, ldb, c, ldc, m, n, k, lower, kt))
       return;
-    }
     const bool pair = pair_ok && abase >= 0 && bbase >= 0 && arow == lda && brow == ldb && op.al == kRow &&
                       op.bl == kRow && m >= 128 && n >= 128 && k >= kPairMinK && i_start == 0;
     const int tm = pair ? kPairTile : TM, tn = pair ? kPairTile : TN;
@@ -334,9 +369,11 @@ struct Builder {
 
 static inline int nblocks(int ns) { return (ns + kNbk - 1) / kNbk; }
 
-static void build_factor_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, bool pairs, bool emu) {
+static void build_factor_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, bool pairs, bool emu,
+                                  int64_t sx_elems) {
   Builder b(sc, TM, TN, pairs, emu);
   const auto& F = S.fronts;
+  b.emu_space = {B_SX, 0, sx_elems * int64_t(sizeof(double))};  // the selected inversion's scratch
   for (int d = S.max_depth; d >= 0; --d) {
     const auto& fr = S.by_depth[d];
     b.depth = d;
@@ -621,58 +658,76 @@ static void build_bwd_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, 
 // reads its operands row by row (K contiguous).  W and W^T are both kept
 // (row-major); for a node [a, b) of the halving tree with children [a, m), [m, b):
 //   TT = W_11^T L_21^T,  (W^T)_12 = -TT W_22^T,  W_21 = ((W^T)_12)^T.
-static void build_selinv_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, int64_t* scratch_elems,
-                                  bool pairs, bool emu) {
+// Scratch layout of one depth: W, W^T, X^T, TT per front, and the front's halving tree
+struct Sx { int64_t w, wt, xt, tt; int ldw, ldx; std::vector<std::vector<std::array<int, 3>>> levels; };
+static int64_t selinv_layout(const Symbolic& S, int d, std::vector<Sx>* out) {
+  const auto& fr = S.by_depth[d];
+  auto r4 = [](int64_t v) { return (v + 3) / 4 * 4; };
+  std::vector<Sx> sx(fr.size());
+  int64_t off = 0;
+  for (size_t q = 0; q < fr.size(); ++q) {
+    const Front& x = S.fronts[fr[q]];
+    Sx& z = sx[q];
+    z.ldw = int(r4(x.ns));
+    z.ldx = int(r4(std::max(x.nb, 1)));
+    z.w = off; off += int64_t(x.ns) * z.ldw;
+    z.wt = off; off += int64_t(x.ns) * z.ldw;
+    z.xt = off; off += int64_t(x.ns) * z.ldx;
+    // halving tree over the 64-blocks; levels[L] = nodes (a, m, b) at recursion depth L
+    const int nblk = nblocks(x.ns);
+    std::vector<std::array<int, 4>> stack{{0, nblk, 0, 0}};
+    while (!stack.empty()) {
+      auto nd = stack.back();
+      stack.pop_back();
+      const int a = nd[0], e = nd[1], L = nd[2];
+      if (e - a < 2) continue;
+      const int m = a + (e - a) / 2;
+      if (int(z.levels.size()) <= L) z.levels.resize(L + 1);
+      z.levels[L].push_back({a, m, e});
+      stack.push_back({a, m, L + 1, 0});
+      stack.push_back({m, e, L + 1, 0});
+    }
+    int64_t tt_need = 0;
+    for (auto& lv : z.levels) {
+      int64_t sum = 0;
+      for (auto& nd : lv) {
+        const int64_t r0 = int64_t(nd[0]) * kNbk, r1 = int64_t(nd[1]) * kNbk;
+        const int64_t c0 = r1, c1 = std::min<int64_t>(int64_t(nd[2]) * kNbk, x.ns);
+        sum += (r1 - r0) * r4(c1 - c0);
+      }
+      tt_need = std::max(tt_need, sum);
+    }
+    z.tt = off; off += tt_need;
+    off = (off + 31) / 32 * 32;
+  }
+  if (out) *out = std::move(sx);
+  return off;
+}
+// Elements of the scratch: the largest depth's, and (FP64 plan) at least 4 MB, so that small
+// lattices, whose pools are small too, have space for the digits of a few tiles.
+static int64_t selinv_scratch(const Symbolic& S, bool emu) {
+  int64_t n = emu ? (4 << 20) / 8 : 32;
+  for (int d = 0; d <= S.max_depth; ++d) n = std::max(n, selinv_layout(S, d, nullptr));
+  return n;
+}
+
+static void build_selinv_schedule(const Symbolic& S, Schedule& sc, int TM, int TN, int64_t sx_elems,
+                                  const int64_t* pool_elems, bool pairs, bool emu) {
   Builder b(sc, TM, TN, pairs, emu);
   const auto& F = S.fronts;
   auto r4 = [](int64_t v) { return (v + 3) / 4 * 4; };
-  int64_t scratch = 32;
   for (int d = 0; d <= S.max_depth; ++d) {
     const auto& fr = S.by_depth[d];
     b.depth = d;
     const int pz = (d & 1) ? B_P1 : B_P0;
-    // scratch layout of this depth: W, W^T, X^T, TT per front
-    struct Sx { int64_t w, wt, xt, tt; int ldw, ldx; std::vector<std::vector<std::array<int, 3>>> levels; };
-    std::vector<Sx> sx(fr.size());
-    int64_t off = 0;
+    std::vector<Sx> sx;
+    const int64_t off = selinv_layout(S, d, &sx);
     int maxlev = 0;
-    for (size_t q = 0; q < fr.size(); ++q) {
-      const Front& x = F[fr[q]];
-      Sx& z = sx[q];
-      z.ldw = int(r4(x.ns));
-      z.ldx = int(r4(std::max(x.nb, 1)));
-      z.w = off; off += int64_t(x.ns) * z.ldw;
-      z.wt = off; off += int64_t(x.ns) * z.ldw;
-      z.xt = off; off += int64_t(x.ns) * z.ldx;
-      // halving tree over the 64-blocks; levels[L] = nodes (a, m, b) at recursion depth L
-      const int nblk = nblocks(x.ns);
-      std::vector<std::array<int, 4>> stack{{0, nblk, 0, 0}};
-      while (!stack.empty()) {
-        auto nd = stack.back();
-        stack.pop_back();
-        const int a = nd[0], e = nd[1], L = nd[2];
-        if (e - a < 2) continue;
-        const int m = a + (e - a) / 2;
-        if (int(z.levels.size()) <= L) z.levels.resize(L + 1);
-        z.levels[L].push_back({a, m, e});
-        stack.push_back({a, m, L + 1, 0});
-        stack.push_back({m, e, L + 1, 0});
-      }
-      maxlev = std::max(maxlev, int(z.levels.size()));
-      int64_t tt_need = 0;
-      for (auto& lv : z.levels) {
-        int64_t sum = 0;
-        for (auto& nd : lv) {
-          const int64_t r0 = int64_t(nd[0]) * kNbk, r1 = int64_t(nd[1]) * kNbk;
-          const int64_t c0 = r1, c1 = std::min<int64_t>(int64_t(nd[2]) * kNbk, x.ns);
-          sum += (r1 - r0) * r4(c1 - c0);
-        }
-        tt_need = std::max(tt_need, sum);
-      }
-      z.tt = off; off += tt_need;
-      off = (off + 31) / 32 * 32;
-    }
-    scratch = std::max(scratch, off);
+    for (const Sx& z : sx) maxlev = std::max(maxlev, int(z.levels.size()));
+    // digits go to the parents' pool, dead once OP_ZGATHER has read it, or to the end of the scratch
+    const int64_t other = pool_elems[(d + 1) & 1], tail = sx_elems - off;
+    if (other >= tail) b.emu_space = {(d & 1) ? B_P0 : B_P1, 0, other * int64_t(sizeof(double))};
+    else b.emu_space = {B_SX, off * int64_t(sizeof(double)), tail * int64_t(sizeof(double))};
     {
       Op& o = b.begin(OP_ZGATHER);
       o.depth = d;
@@ -821,7 +876,6 @@ static void build_selinv_schedule(const Symbolic& S, Schedule& sc, int TM, int T
       b.end();
     }
   }
-  *scratch_elems = scratch;
 }
 
 // ------------------------------------------------------ one-column sweeps
@@ -1350,7 +1404,8 @@ struct Exec {
         case OP_EMU:
           if constexpr (sizeof(T) == sizeof(double))
             launch_emu_gemm(s.d_esplit + o.soff, o.scount, s.d_emu + o.off, o.count, buf(o.abuf), buf(o.bbuf),
-                            buf(o.cbuf), o.mode, p->d_emu, p->d_emu_exp, p->d_emu_err, st, p->tc_wait_ns);
+                            buf(o.cbuf), o.mode, reinterpret_cast<uint8_t*>(buf(o.sbuf)), p->d_emu_err, st,
+                            p->tc_wait_ns);
           break;
         case OP_SGATHER_FWD: {
           int pd = o.depth & 1;
@@ -1598,35 +1653,14 @@ int plan_build(Plan* p) {
     CUDA_TRY(cudaMalloc(&p->d_pool[k], size_t(p->pool_elems[k]) * es));
   }
   const bool pairs = p->precision == 1 && tc_gemm_enabled();
-  bool emu = p->precision == 0 && tc_gemm_enabled();
-  int64_t sx_elems = 0;
-  build_factor_schedule(S, p->sched_factor, TM, TM, pairs, emu);
-  build_selinv_schedule(S, p->sched_selinv, TM, TM, &sx_elems, pairs, emu);
+  const bool emu = p->precision == 0 && tc_gemm_enabled();
+  const int64_t sx_elems = selinv_scratch(S, emu);
+  build_factor_schedule(S, p->sched_factor, TM, TM, pairs, emu, sx_elems);
+  build_selinv_schedule(S, p->sched_selinv, TM, TM, sx_elems, p->pool_elems, pairs, emu);
   CUDA_TRY(cudaMalloc(&p->d_sx, size_t(sx_elems) * es));
   if (emu) {
-    // digits and row exponents of the largest launch.  They are taken only if that leaves as
-    // much memory free as the arenas hold (a second pipeline, the solves' vectors), so
-    // that they never make a call fail; without them the products stay on the CUDA cores
-    const int64_t bytes = std::max(p->sched_factor.emu_bytes, p->sched_selinv.emu_bytes);
-    const int64_t rows = std::max(p->sched_factor.emu_rows, p->sched_selinv.emu_rows);
-    const size_t arenas = size_t(S.l_size + S.dinv_size + p->pool_elems[0] + p->pool_elems[1] + sx_elems) * es;
-    size_t room = 0, total = 0;
-    if (bytes > 0 && (cudaMemGetInfo(&room, &total) != cudaSuccess ||
-                      room < size_t(bytes) + size_t(rows) * sizeof(int) + arenas ||
-                      cudaMalloc(&p->d_emu, size_t(bytes)) != cudaSuccess ||
-                      cudaMalloc(&p->d_emu_exp, size_t(rows) * sizeof(int)) != cudaSuccess ||
-                      cudaMalloc(&p->d_emu_err, sizeof(int)) != cudaSuccess)) {
-      cudaGetLastError();
-      cudaFree(p->d_emu); cudaFree(p->d_emu_exp);
-      p->d_emu = nullptr;
-      p->d_emu_exp = nullptr;
-      p->sched_factor = Schedule();
-      p->sched_selinv = Schedule();
-      build_factor_schedule(S, p->sched_factor, TM, TM, pairs, false);
-      build_selinv_schedule(S, p->sched_selinv, TM, TM, &sx_elems, pairs, false);
-    } else if (bytes > 0) {
-      CUDA_TRY(cudaMemset(p->d_emu_err, 0, sizeof(int)));
-    }
+    CUDA_TRY(cudaMalloc(&p->d_emu_err, sizeof(int)));
+    CUDA_TRY(cudaMemset(p->d_emu_err, 0, sizeof(int)));
   }
   if (pairs) {
     const int64_t sizes[] = {S.l_size, p->pool_elems[0], p->pool_elems[1], sx_elems};

@@ -48,8 +48,8 @@ struct Op {
   int abuf = B_NONE, bbuf = B_NONE, cbuf = B_NONE;
   int64_t elems = 0;  // memset length
   int depth = 0;
-  int64_t soff = 0;   // OP_EMU: first split task and their number
-  int scount = 0;
+  int64_t soff = 0;   // OP_EMU: first split task and their number, buffer that takes the digits
+  int scount = 0, sbuf = B_NONE;
 };
 
 // 32 x 32 block copy, rows x cols of src: dst[j*ldd + i] = src[i*lds + j] when
@@ -83,7 +83,6 @@ struct Schedule {
   std::map<std::tuple<int, int64_t, int>, int> map_index;
   std::vector<EmuSplit> esplit;
   std::vector<EmuTask> emu;
-  int64_t emu_bytes = 0, emu_rows = 0;  // digit scratch and row exponents of the largest launch
   // device copies
   GemmTask* d_gemm = nullptr;
   DiagTask* d_diag = nullptr;
@@ -158,11 +157,7 @@ struct Plan {
   void* d_pool[2] = {nullptr, nullptr};
   void* d_sx = nullptr;  // selected-inversion scratch (triangular inverse, X^T)
   int64_t pool_elems[2] = {0, 0};
-  // FP64 plan: split operands of one launch of OP_EMU (digits, row exponents) and
-  // the flag its kernel sets when a wait gives up
-  uint8_t* d_emu = nullptr;
-  int* d_emu_exp = nullptr;
-  int* d_emu_err = nullptr;
+  int* d_emu_err = nullptr;  // FP64 plan: set when a wait of a tensor-core product gives up
   double* d_logpiv = nullptr;
   int* d_err = nullptr;
   // one-column triangular sweeps (engine.cu, fwd_chain_kernel / bwd_chain_kernel):

@@ -113,22 +113,23 @@ void launch_gemm_pair(const GemmTask* tasks, int ntasks, const CUtensorMap* maps
                       float* C, int mode, cudaStream_t st, unsigned long long wait_ns = kTcWaitNs);
 // FP64 products on the tensor cores (emu_gemm.cu).  Split task: 64 rows (the last
 // tile of an operand fewer) of a row-major operand in buffer A (buf 0) or B (1),
-// k values each, into nch = ceil(k / 32) chunks of digits at byte dst of the digit
-// scratch and row exponents at exp.  Product task: one 128 x 64 tile over the
+// k values each, into nch = ceil(k / 32) chunks of digits at byte dst of the
+// scratch and row exponents at its int exp.  Product task: one 128 x 64 tile over the
 // chunks [k0, k1); a / b: byte offsets of the operand tiles' digits, a_step: bytes
 // from A's first 64-row tile to its second, ea / eb: their row exponents.
 constexpr int kEmuDigits = 7;
 constexpr int64_t kEmuChunkBytes = kEmuDigits * 4096;  // 64 rows x 32 values, all digits
+constexpr int64_t kEmuExpBytes = 64 * 4;               // row exponents of 64 rows
 struct EmuSplit {
-  int64_t src, dst;
-  int ld, rows, k, nch, exp, buf;
+  int64_t src, dst, exp;
+  int ld, rows, k, nch, buf;
 };
 struct EmuTask {
-  int64_t a, b, c, a_step;
-  int ldc, m, n, k0, k1, ea, eb;
+  int64_t a, b, c, a_step, ea, eb;
+  int ldc, m, n, k0, k1;
 };
 void launch_emu_gemm(const EmuSplit* splits, int nsplits, const EmuTask* tasks, int ntasks, const double* A,
-                     const double* B, double* C, int mode, uint8_t* planes, int* exps, int* err, cudaStream_t st,
+                     const double* B, double* C, int mode, uint8_t* scratch, int* err, cudaStream_t st,
                      unsigned long long wait_ns = kTcWaitNs);
 int tc_gemm_take_error(cudaStream_t st, int* pinned);
 bool tc_gemm_enabled();
