@@ -29,7 +29,7 @@ extern "C" {
 #define SPDE_ERR_STATE 5
 #define SPDE_ERR_NOT_CONVERGED 6
 
-#define SPDE_PRECISION_FP64 0 /* factor, solves and inverse in FP64 (products from exact digit products, rounded to FP64) */
+#define SPDE_PRECISION_FP64 0 /* factor, solves and inverse in FP64; products of operands kept to 2^-64 of a row's largest entry */
 #define SPDE_PRECISION_MIXED 1 /* FP32 factor, FP64 pivots / log-det / refinement */
 #define SPDE_PRECISION_ITERATIVE 2 /* no factorisation: assembly, products, PCG */
 

@@ -4,25 +4,35 @@
 // matrix multiplication and its applications", Numer. Algorithms 59, 2012).
 //
 // Split: every operand row is scaled by a power of two (the row's largest magnitude
-// below 1) and written as seven signed base-256 digits,
+// below 1) and written as eight signed base-256 digits,
 //   x = 2^e sum_s d_s 2^(-7 - 8 s),  |d_s| <= 128,
-// rounded to nearest at 2^-56 of the row's scale.  Digits are exact in bf16.
-// Product: digits i of A and j of B with i + j = o <= 6 (28 products) accumulate in
+// rounded to nearest at 2^-64 of the row's scale: entries down to 2^-10 of the row's
+// largest keep all 53 bits, smaller ones lose their last.  Digits are exact in bf16.
+// Product: digits i of A and j of B with i + j = o <= 7 (36 products) accumulate in
 // the tensor core's FP32 accumulator o: all terms are integers, and over 128 values
-// of k their sum stays below 7 * 128 * 2^14 < 2^24, so every accumulator is exact.
-// After each 128 values of k the seven accumulators are added into two 64-bit
+// of k their sum does not pass 8 * 128 * 2^14 = 2^24, so every accumulator is exact.
+// After each 128 values of k the eight accumulators are added into two 64-bit
 // integers per output entry, and at the end one conversion rounds
-// 2^(ea + eb) sum_o acc_o 2^(-14 - 8 o) to FP64.  The pairs left out (i + j > 6) and the
-// rounding of the digits are below 2^-53 of (row scale of A) (row scale of B) k.
+// 2^(ea + eb) sum_o acc_o 2^(-14 - 8 o) to FP64.
+// Error of an entry, besides that rounding: 2 * 2^-64 for the operands' digits and
+// 7.1 * 2^-64 for the pairs left out (i + j > 7), per value of k and relative to
+// (row scale of A) (row scale of B).  FP64 FMAs round each partial sum at 2^-53 of
+// itself, so theirs is larger unless the sums stay 2^10 below the scales' product.
+// In a factor they do not matter there (|L_i| |L_j| <= sqrt(Q_ii Q_jj), Cholesky's own
+// bound); an inverse, whose rows follow the variances along k, was measured: with standard
+// deviations over 2^28 its entries' errors, relative to sqrt(Z_ii Z_jj), are 0.5 to 1.1
+// times those of FP64 FMAs (seven digits, 2^-56: up to 11 times).
 //
 // Why: FP64 is a narrow pipe on this part (two FMAs per clock and SM, 1.26 TFLOP/s),
-// while 28 bf16 products cost 28 / 2250 of it.
+// while 36 bf16 products cost 36 / 2250 of it.  The eighth digit: fit of 30 x 30 x 24
+// 15.6 ms (14.8 with seven), 48 x 48 x 24 53.0 ms (49.6).
 //
-// Split operands lie in memory that the plan's arenas do not use at the time, as the shared-memory images the tensor core reads:
+// Split operands lie in memory that the plan's arenas do not use at the time, as the
+// shared-memory images the tensor core reads:
 // [64-row tile][32-wide k chunk][digit][8-row group][8-wide k core][row][8 x bf16], 4 KB
 // per digit, so that a stage is filled by a few bulk copies.  A CTA computes a
-// 128 x 64 tile: the seven accumulators take 448 of 512 TMEM columns, and a stage (seven
-// digits of 128 x 32 and 64 x 32) 84 KB, two of which fit in shared memory.
+// 128 x 64 tile: the eight accumulators take all 512 TMEM columns, and a stage (eight
+// digits of 128 x 32 and 64 x 32) 96 KB, two of which fit in shared memory.
 // Bound: the tensor core's shared-memory reads (128 + 64 rows per 128 x 64 product).
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -50,10 +60,10 @@ constexpr int kNotFinite = 1 << 20;                   // row exponent of a row t
 
 // ------------------------------------------------------------------ split
 // Eight CTAs per 64-row tile, a warp per row: the row's exponent from its largest
-// magnitude, then eight values per lane into their seven digits (16-byte stores).
+// magnitude, then eight values per lane into their digits (16-byte stores).
 // Rows of up to 512 values are held in registers between the two steps, longer ones
 // read again (from L1 / L2).  Bound: latency for the short rows, memory (8 bytes read,
-// 14 written per value) for large operands.
+// 16 written per value) for large operands.
 __device__ __forceinline__ void split_load(const double* x, int k0, int k, bool vec, double (&v)[8]) {
   if (vec && k0 + 8 <= k) {
 #pragma unroll

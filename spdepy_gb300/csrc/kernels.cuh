@@ -117,7 +117,7 @@ void launch_gemm_pair(const GemmTask* tasks, int ntasks, const CUtensorMap* maps
 // scratch and row exponents at its int exp.  Product task: one 128 x 64 tile over the
 // chunks [k0, k1); a / b: byte offsets of the operand tiles' digits, a_step: bytes
 // from A's first 64-row tile to its second, ea / eb: their row exponents.
-constexpr int kEmuDigits = 7;
+constexpr int kEmuDigits = 8;
 constexpr int64_t kEmuChunkBytes = kEmuDigits * 4096;  // 64 rows x 32 values, all digits
 constexpr int64_t kEmuExpBytes = 64 * 4;               // row exponents of 64 rows
 struct EmuSplit {
