@@ -765,7 +765,7 @@ template <typename T>
 constexpr int potrf_smem() { return (2 * kMaxNbk * kDfLd + 3 * kDfSub * kDfSub) * int(sizeof(T)); }
 
 // The elimination's arithmetic by storage type: numbers, their shared-memory form,
-// products, reciprocal and reciprocal square root of a pivot.
+// products, reciprocal and square root of a pivot.
 template <typename T>
 struct Elim;
 template <>
@@ -791,9 +791,12 @@ struct Elim<float> {
     x1 = DF{h.y, l.y};
   }
   static __device__ __forceinline__ DF rcp(DF d) { return df_rcp(d); }
-  static __device__ __forceinline__ float rsqrt_of(DF d) { return df_rsqrt(d); }
+  // of a pivot: what `root` holds, and from it 1 / sqrt(d), sqrt(d) and an entry of L
+  static __device__ __forceinline__ float root(DF d) { return df_rsqrt(d); }
+  static __device__ __forceinline__ float inv(float r) { return r; }
+  static __device__ __forceinline__ float diag(float r) { return 1.0f / r; }
+  static __device__ __forceinline__ float entry(DF v, float r) { return (v.hi + v.lo) * r; }
   static __device__ __forceinline__ bool bad(DF d) { return !(d.hi > 0.0f) || !isfinite(d.hi); }
-  static __device__ __forceinline__ float value(DF v) { return v.hi + v.lo; }
   static __device__ __forceinline__ double wide(DF v) { return double(v.hi) + double(v.lo); }
 };
 template <>
@@ -813,7 +816,9 @@ struct Elim<double> {
   }
   // 1 / d for d > 0: the FP32 reciprocal of the significand and two Newton steps
   // (four FP64 operations instead of a full division on the narrow pipe); pivots
-  // outside the normal range of d and 1 / d take the division
+  // outside the normal range of d and 1 / d take the division.  The steps leave 2^-88 before the
+  // last rounding: 4 10^8 random significands, with estimates up to two units off, all gave the
+  // division's result
   static __device__ __forceinline__ double rcp(double d) {
     const long long b = __double_as_longlong(d);
     const int f = int(b >> 52);
@@ -824,9 +829,13 @@ struct Elim<double> {
     y = fma(y, fma(-m, y, 1.0), y);
     return __longlong_as_double(__double_as_longlong(y) - (static_cast<long long>(f - 1023) << 52));
   }
-  static __device__ __forceinline__ double rsqrt_of(double d) { return rsqrt(d); }
+  // the root itself, so that L takes one division (rsqrt is not correctly rounded, and a
+  // product with it rounds again)
+  static __device__ __forceinline__ double root(double d) { return sqrt(d); }
+  static __device__ __forceinline__ double inv(double r) { return 1.0 / r; }
+  static __device__ __forceinline__ double diag(double r) { return r; }
+  static __device__ __forceinline__ double entry(double v, double r) { return v / r; }
   static __device__ __forceinline__ bool bad(double d) { return !(d > 0.0) || !isfinite(d); }
-  static __device__ __forceinline__ double value(double v) { return v; }
   static __device__ __forceinline__ double wide(double v) { return v; }
 };
 
@@ -848,7 +857,7 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
   // L and L^-1; before that, two panel buffers and the panel's multipliers
   extern __shared__ __align__(16) uint8_t potrf_sm[];
   __shared__ Pair dp[kMaxNbk];
-  __shared__ T rsq[kMaxNbk];
+  __shared__ T root[kMaxNbk], rinv[kMaxNbk];
   __shared__ int bad;
   static_assert(2 * kMaxNbk * kDfLd * sizeof(T) >= 3 * kMaxNbk * kDfPan * sizeof(Pair), "panel buffers fit");
   T (*Ls)[kDfLd] = reinterpret_cast<T (*)[kDfLd]>(potrf_sm);
@@ -956,7 +965,10 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
     }
   }
   __syncthreads();
-  if (tid < w) rsq[tid] = E::rsqrt_of(E::load(dp[tid]));
+  if (tid < w) {
+    root[tid] = E::root(E::load(dp[tid]));
+    rinv[tid] = E::inv(root[tid]);
+  }
   __syncthreads();
   // L = a_ik / sqrt(d_k), zero above the diagonal
 #pragma unroll
@@ -967,8 +979,8 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
       if (i < w && k < w) {
         T v = T(0);
         if (n <= m) {
-          if (k < i) v = E::value(r[m][n]) * rsq[k];
-          else if (k == i) v = T(1) / rsq[k];
+          if (k < i) v = E::entry(r[m][n], root[k]);
+          else if (k == i) v = E::diag(root[k]);
         }
         Ls[i][k] = v;
         blk[int64_t(i) * tk.lda + k] = v;
@@ -987,8 +999,8 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
       for (int k = 0; k < kDfSub; ++k) {
         if (k >= cw) break;
         T x = T(0);
-        if (k == c) x = rsq[c0 + k];
-        else if (k > c) x = -sum[k] * rsq[c0 + k];
+        if (k == c) x = rinv[c0 + k];
+        else if (k > c) x = -sum[k] * rinv[c0 + k];
         Xs[c0 + k][c0 + c] = x;
 #pragma unroll
         for (int ii = k + 1; ii < kDfSub; ++ii)

@@ -45,3 +45,18 @@ def test_factor_and_inverse(lib, w, up):
     inv = np.linalg.inv(ref)
     assert np.abs(X[:w, :w] - inv).max() <= tol * np.abs(inv).max()
     assert abs(lp[0] - np.log(np.diag(ref)).sum()) <= tol * w
+
+
+def test_first_column_is_rounded_once(lib):
+    """The FP64 factor's first column, which no update reaches, is sqrt(a) and a_i / sqrt(a)."""
+    rng = np.random.default_rng(9)
+    for _ in range(40):
+        w = 24
+        A = np.diag(rng.uniform(0.5, 8.0, w)) + 0.0
+        A[:, 0] += 1e-3 * rng.uniform(-1, 1, w)
+        L, X = np.tril(A), np.zeros((64, 64))
+        lp, err = np.zeros(1), np.full(1, -1, np.int32)
+        lib.potrf_host(w, w, *[v.ctypes.data_as(ctypes.c_void_p) for v in (L, X, lp, err)], 1)
+        root = np.sqrt(A[0, 0])
+        assert L[0, 0] == root and X[0, 0] == 1 / root
+        assert np.array_equal(L[1:, 0], A[1:, 0] / root)
