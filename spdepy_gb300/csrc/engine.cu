@@ -1375,8 +1375,8 @@ struct Exec {
     };
     for (const Op& o : s.ops) {
       if (depth_log && (dmarks.empty() || dmarks.back().first != o.depth)) dmark(o.depth);
-      const bool on_tc = o.kind == OP_GEMM && sizeof(T) == sizeof(float) &&
-                         ((o.tc == kPathTensor && tc_gemm_enabled()) || o.tc == kPathPair);
+      const bool on_tc = o.kind == OP_EMU || (o.kind == OP_GEMM && sizeof(T) == sizeof(float) &&
+                                              ((o.tc == kPathTensor && tc_gemm_enabled()) || o.tc == kPathPair));
       const bool timed = p->profile && o.kind != OP_MEMSET && (on_tc || !p->profile_tc_only);
       if (timed) prof_begin(p, st);
       switch (o.kind) {
@@ -1451,7 +1451,7 @@ struct Exec {
       }
       if (timed)
         prof_end(p, st, on_tc ? kProfTensorCore : (o.kind >= OP_FWD_CHAIN ? int(OP_GEMM) : o.kind), o.flops, o.site,
-                 o.kind == OP_GEMM ? o.count : 0);
+                 o.kind == OP_GEMM || o.kind == OP_EMU ? o.count : 0);
     }
     if (depth_log && !dmarks.empty()) {
       dmark(-1);
@@ -1715,7 +1715,9 @@ static int factor_t(Plan* p, int with_obs, double tau) {
   CUDA_TRY(cudaGetLastError());
   const double sum = p->h_pin[1024];
   const int err = p->pin_int()[0];
-  if (tc_gemm_take_error(p->stream, p->pin_int() + 1) || emu_take_error(p, p->stream, p->pin_int() + 3)) {
+  // both flags, so that neither is left for the next call
+  const int tc_err = tc_gemm_take_error(p->stream, p->pin_int() + 1);
+  if (emu_take_error(p, p->stream, p->pin_int() + 3) || tc_err) {
     p->last_error = "tensor-core product timed out";
     p->factored = 0;
     return 2;
@@ -1902,7 +1904,8 @@ static int selinv_t(Plan* p, double* zq, cudaStream_t st, std::string* error) {
     *error = std::string("selected inversion: ") + cudaGetErrorString(e);
     return 2;
   }
-  if (tc_gemm_take_error(st, p->pin_int() + 5) || emu_take_error(p, st, p->pin_int() + 6)) {
+  const int tc_err = tc_gemm_take_error(st, p->pin_int() + 5);
+  if (emu_take_error(p, st, p->pin_int() + 6) || tc_err) {
     *error = "tensor-core product timed out";
     return 2;
   }
