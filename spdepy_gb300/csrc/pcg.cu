@@ -1043,7 +1043,7 @@ struct GWeights {
   int nob, Ns, T, compact;
   // with mask: the nodes p whose row of G^T gathers from an observed node (bit p of
   // near, number of bits before each word in nrank) have that row written out,
-  // near_w[o ncap + index]
+  // near_w[o ncap + index]; without memory for it (near null) every weight is looked up
   const uint32_t* near;
   const int* nrank;
   const float* near_w;
@@ -1096,6 +1096,13 @@ __global__ void __launch_bounds__(1024) bit_rank_kernel(const uint32_t* __restri
 
 __device__ __forceinline__ int time_class(int t, int T) { return t == 0 ? 0 : (t == T - 1 ? 2 : 1); }
 
+// G(q, q + d_o) from the compact weights, q the node of cell cq at time tq
+__device__ __forceinline__ float compact_weight(const GWeights& gw, int o, int cq, int tq, int q) {
+  const uint32_t m = gw.mask[q >> 5], b = 1u << (q & 31);
+  if (m & b) return gw.w[int64_t(3 * kOff) * gw.Ns + o * gw.nob + gw.rank[q >> 5] + __popc(m & (b - 1u))];
+  return gw.w[int64_t(time_class(tq, gw.T) * kOff + o) * gw.Ns + cq];
+}
+
 // The rows of G^T next to observed nodes: near_w[o ncap + i] = weight with which
 // node p gathers from q = p - d_o, 0 outside the grid
 __global__ void near_rows_kernel(int Mx, int Ny, int T, GWeights gw, float* __restrict__ near_w) {
@@ -1111,10 +1118,8 @@ __global__ void near_rows_kernel(int Mx, int Ny, int T, GWeights gw, float* __re
     const int xq = x - dx, yq = y - dy, tq = t - dt;
     float v = 0.f;
     if (xq >= 0 && xq < Mx && yq >= 0 && yq < Ny && tq >= 0 && tq < T) {
-      const int cq = yq * Mx + xq, q = tq * Ns + cq;
-      const uint32_t m = gw.mask[q >> 5], b = 1u << (q & 31);
-      if (m & b) v = gw.w[int64_t(3 * kOff) * Ns + o * gw.nob + gw.rank[q >> 5] + __popc(m & (b - 1u))];
-      else v = gw.w[int64_t(time_class(tq, T) * kOff + o) * Ns + cq];
+      const int cq = yq * Mx + xq;
+      v = compact_weight(gw, o, cq, tq, tq * Ns + cq);
     }
     near_w[int64_t(o) * gw.ncap + i] = v;
   }
@@ -1122,7 +1127,7 @@ __global__ void near_rows_kernel(int Mx, int Ny, int T, GWeights gw, float* __re
 
 // u = G r (TRANS 0) or z = G^T u with the warp groups' sums of r . z (TRANS 1) for
 // the columns [lead + V y, + V), one thread per node and V columns; the rows of G
-// come from the compact (COMPACT 1) or per-node weights through L1 / L2.  Every
+// come from the compact (COMPACT 1; 2: G^T without near_w) or per-node weights through L1 / L2.  Every
 // row is one base, stride and neighbour shift per time offset, so that observed
 // nodes, their neighbours and the boundary differ from the interior by a
 // predicate per offset and not by another path (a warp holds several kinds).
@@ -1158,14 +1163,14 @@ __global__ void __launch_bounds__(256, V == 1 ? 4 : 3) g32_kernel(int Mx, int Ny
       const uint32_t bx = bits(xx, Mx, sg), by = bits(y, Ny, sg), bt = bits(t, T, sg);
       // weight of offset o: row[dt + 1][o stride - dy shift_y - dx shift_x]
       const float* row[3];
-      int stride, shift_y = 0, shift_x = 0;
-      if (!COMPACT) {
+      int stride = 0, shift_y = 0, shift_x = 0;
+      if (COMPACT == 0) {
         stride = n;
         shift_y = TRANS ? Mx : 0;
         shift_x = TRANS ? 1 : 0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) row[d] = gw.w + p - (TRANS ? (d - 1) * Ns : 0);
-      } else {
+      } else if (COMPACT == 1) {
         const uint32_t* own = TRANS ? gw.near : gw.mask;  // nodes with a row of their own
         const uint32_t word = own ? own[p >> 5] : 0u, bit = 1u << (p & 31);
         if (word & bit) {
@@ -1188,8 +1193,13 @@ __global__ void __launch_bounds__(256, V == 1 ? 4 : 3) g32_kernel(int Mx, int Ny
         const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dt = o / 9 - 1;
         // a neighbour outside the grid counts with weight zero (on the node's own value)
         const bool in = (bx >> (dx + 1)) & (by >> (dy + 1)) & (bt >> (dt + 1)) & 1u;
-        const float wv = in ? row[dt + 1][o * stride - dy * shift_y - dx * shift_x] : 0.f;
         const int d = in ? dt * Ns + dy * Mx + dx : 0;
+        float wv = 0.f;
+        if (COMPACT == 2) {
+          if (in) wv = compact_weight(gw, o, c - dy * Mx - dx, t - dt, p - d);
+        } else if (in) {
+          wv = row[dt + 1][o * stride - dy * shift_y - dx * shift_x];
+        }
         const Cols<V> xq = x[TRANS ? p - d : p + d];
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v] = fmaf(wv, xq.v[v], acc[v]);
@@ -1643,9 +1653,16 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   auto pad4 = [](size_t e) { return (e + 3) & ~size_t(3); };  // 16-byte sections
   const size_t vlen = pad4(size_t(len));  // a group of columns then starts at a multiple of its width
   const size_t need32 = 6 * vlen + size_t(nrhs) * gpad + pad4(size_t(kCoef32) * Ns) + pad4(size_t(n)) +
-                        pad4(size_t(2 * nrhs)) + (kind == 4 ? pad4(size_t(kIcRow) * n) : 0) +
-                        (near_bits ? 2 * pad4(nwords) + size_t(kOff) * ncap : 0);
-  float* b32 = scratch32(p, need32);
+                        pad4(size_t(2 * nrhs)) + (kind == 4 ? pad4(size_t(kIcRow) * n) : 0);
+  // the rows of G^T next to observed nodes (27 floats for up to every node): a solve that has no
+  // memory for them looks the weights up, with the same result
+  bool near_table = near_bits;
+  float* b32 = scratch32(p, need32 + (near_table ? 2 * pad4(nwords) + size_t(kOff) * ncap : 0));
+  if (!b32 && near_table) {
+    cudaGetLastError();
+    near_table = false;
+    b32 = scratch32(p, need32);
+  }
   if (!base || !b32) return 4;
   double* r64 = base;
   double* partA = r64 + len;
@@ -1664,8 +1681,8 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   float* beta = alpha + nrhs;
   float* Lic = alpha + pad4(size_t(2 * nrhs));  // IC(0) factor (kind 4)
   uint32_t* near = reinterpret_cast<uint32_t*>(Lic + (kind == 4 ? pad4(size_t(kIcRow) * n) : 0));
-  int* nrank = reinterpret_cast<int*>(near + (near_bits ? pad4(nwords) : 0));
-  float* near_w = reinterpret_cast<float*>(nrank + (near_bits ? pad4(nwords) : 0));
+  int* nrank = reinterpret_cast<int*>(near + (near_table ? pad4(nwords) : 0));
+  float* near_w = reinterpret_cast<float*>(nrank + (near_table ? pad4(nwords) : 0));
   const QStencil q = p->qstencil();
   const double* obs = with_obs ? p->d_obs_cnt : nullptr;
   const int sep = q.sep;
@@ -1685,8 +1702,8 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
     w += kCompactHeader;
   }
   GWeights gw{w, near_bits ? p->d_obs_mask : nullptr, p->d_obs_rank, p->nob, Ns, T, kind == 3 ? 1 : 0,
-              near_bits ? near : nullptr, nrank, near_w, int(ncap)};
-  if (near_bits) {
+              near_table ? near : nullptr, nrank, near_w, int(ncap)};
+  if (near_table) {
     cudaMemsetAsync(near, 0, nwords * sizeof(uint32_t), st);
     if (p->nob > 0) near_obs_kernel<<<nblk(p->nob), 256, 0, st>>>(p->d_obs_nodes, p->nob, Mx, Ny, T, near);
     bit_rank_kernel<<<1, 1024, 0, st>>>(near, int(nwords), nrank);
@@ -1754,7 +1771,10 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
       const Walk wk = walk(groups, &grid);
       if (kind == 3) {
         g32_kernel<V, 0, 1><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, r32, u32, nullptr, nullptr);
-        g32_kernel<V, 1, 1><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, u32, z32, r32, gsum);
+        if (near_bits && !near_table)
+          g32_kernel<V, 1, 2><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, u32, z32, r32, gsum);
+        else
+          g32_kernel<V, 1, 1><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, u32, z32, r32, gsum);
       } else {
         g32_kernel<V, 0, 0><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, r32, u32, nullptr, nullptr);
         g32_kernel<V, 1, 0><<<grid, 256, 0, st>>>(Mx, Ny, T, wk, lead, gpad, gw, u32, z32, r32, gsum);
