@@ -223,11 +223,7 @@ __global__ void __launch_bounds__(256, 2) gemm32_kernel(const GemmTask* __restri
 template <typename T, int MODE, int AL, int BL>
 static void gemm_layout(const GemmTask* t, int n, const T* A, const T* B, T* C, cudaStream_t st) {
   if constexpr (sizeof(T) == sizeof(float)) {
-    static const bool attr = [] {  // once, thread-safely
-      cudaFuncSetAttribute(gemm32_kernel<MODE, AL, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgSmem);
-      return true;
-    }();
-    (void)attr;
+    allow_smem<gemm32_kernel<MODE, AL, BL>>(kSgSmem);
     launch_chained(gemm32_kernel<MODE, AL, BL>, n, 256, kSgSmem, st, t, A, B, C);
   } else {
     launch_chained(gemm64_kernel<MODE, AL, BL>, n, 256, 0, st, t, A, B, C);
@@ -535,11 +531,7 @@ __global__ void __launch_bounds__(256) panel64_kernel(const GemmTask* __restrict
 // Fewer rows per CTA while the launch leaves SMs idle: 32 rows up to 152 tasks, 64 up to 304.
 template <int MODE, int ROWS>
 static void panel64_rows(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st) {
-  static const bool attr = [] {  // once, thread-safely (two pipelines launch from two host threads)
-    cudaFuncSetAttribute(panel64_kernel<MODE, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem(ROWS));
-    return true;
-  }();
-  (void)attr;
+  allow_smem<panel64_kernel<MODE, ROWS>>(panel_smem(ROWS));
   launch_chained(panel64_kernel<MODE, ROWS>, n * (128 / ROWS), 256, panel_smem(ROWS), st, t, A, B, C);
 }
 template <int MODE>
@@ -1067,11 +1059,7 @@ __global__ void __launch_bounds__(256, Elim<T>::kMinCtas)
 template <typename T>
 void launch_potrf(const DiagTask* tasks, int ntasks, T* L, T* dinv, double* logpiv, int* err, cudaStream_t st) {
   if (ntasks <= 0) return;
-  static const bool attr = [] {  // once, thread-safely
-    cudaFuncSetAttribute(potrf_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, potrf_smem<T>());
-    return true;
-  }();
-  (void)attr;
+  allow_smem<potrf_kernel<T>>(potrf_smem<T>());
   launch_chained(potrf_kernel<T>, ntasks, 256, potrf_smem<T>(), st, tasks, L, dinv, logpiv, err);
 }
 template void launch_potrf<double>(const DiagTask*, int, double*, double*, double*, int*, cudaStream_t);

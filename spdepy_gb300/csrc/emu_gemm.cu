@@ -341,11 +341,7 @@ __global__ void __launch_bounds__(kEmuThreads, 1) emu_gemm_kernel(const EmuTask*
 template <int MODE>
 void launch_emu(const EmuTask* t, int n, const uint8_t* scratch, double* C, int* err, cudaStream_t st,
                 unsigned long long wait_ns) {
-  static const bool attr = [] {  // once per instantiation, thread-safely
-    cudaFuncSetAttribute(emu_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kEmuSmem);
-    return true;
-  }();
-  (void)attr;
+  allow_smem<emu_gemm_kernel<MODE>>(kEmuSmem);
   launch_chained(emu_gemm_kernel<MODE>, n, kEmuThreads, kEmuSmem, st, t, scratch, C, err, wait_ns);
 }
 

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 
 namespace spde {
@@ -53,6 +54,19 @@ inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Dynamic shared memory above 48 KB is granted per kernel and device: on its first launch on
+// each (plans may live on several devices and launch from several threads)
+template <auto Kernel>
+inline void allow_smem(int bytes) {
+  static std::atomic<uint64_t> granted{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+  if (granted.load(std::memory_order_acquire) & bit) return;
+  cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  granted.fetch_or(bit, std::memory_order_release);
 }
 
 // an integer constant as a type (selects a kernel's template argument in a lambda)

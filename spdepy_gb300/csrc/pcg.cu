@@ -1493,11 +1493,7 @@ int qsqrt_apply(Plan* p, int transpose, const double* x, double* y, int nrhs) {
 int pc_weights(Plan* p, int with_obs, double tau, const float* prm, float* w, float* act) {
   const int64_t n = p->sym.n;
   constexpr int kActSmem = (kNP + 128 * kAct) * int(sizeof(float));
-  static const bool attr = [] {  // once, thread-safely
-    cudaFuncSetAttribute(pc_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kActSmem);
-    return true;
-  }();
-  (void)attr;
+  allow_smem<pc_forward_kernel>(kActSmem);
   pc_forward_kernel<<<nblk(n, 128), 128, act ? kActSmem : kNP * int(sizeof(float)), p->stream>>>(
       p->qstencil(), with_obs ? p->d_obs_cnt : nullptr, tau, prm, w, act);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
@@ -1535,11 +1531,7 @@ int pc_grad(Plan* p, int with_obs, double tau, const float* prm, const float* w,
   if (k == 4) pc_wgrad_kernel<4><<<nblk(n, 128), 128, 0, st>>>(q, z, e, u, g2, k, scale, act, dout);
   else pc_wgrad_kernel<0><<<nblk(n, 128), 128, 0, st>>>(q, z, e, u, g2, k, scale, act, dout);
   const size_t smem = sizeof(float) * (kHid * kHid + kOff * kHid + kBwNodes * (kFeat + 4 * kHid + kOff));
-  static const bool attr = [smem] {  // once, thread-safely
-    cudaFuncSetAttribute(pc_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    return true;
-  }();
-  (void)attr;
+  allow_smem<pc_backward_kernel>(int(smem));
   pc_backward_kernel<<<nbw, kBwThreads, smem, st>>>(n, prm, act, dout, bpart);
   cudaMemsetAsync(arrived, 0, 32 * sizeof(double), st);
   pc_colsum_kernel<<<dim3(nblk(kNP, 128), kColParts), 128, 0, st>>>(bpart, nbw, colsums, arrived, grad);

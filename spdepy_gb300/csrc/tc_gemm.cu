@@ -644,25 +644,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 template <int MODE>
 void launch_pair(const GemmTask* t, int n, const CUtensorMap* maps, const float* A, const float* B, float* C,
                  cudaStream_t st, unsigned long long wait_ns) {
-  static const bool attr = [] {  // once per instantiation, thread-safely
-    cudaFuncSetAttribute(tc_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    return true;
-  }();
-  (void)attr;
+  allow_smem<tc_pair_kernel<MODE>>(kSmem);
   launch_chained(tc_pair_kernel<MODE>, 2 * n, kPairThreads, kSmem, st, t, maps, A, B, C, wait_ns);
 }
 
 template <int MODE, int AL, int BL, int ST>
 void launch_stages(const GemmTask* t, int n, const float* A, const float* B, float* C, cudaStream_t st,
                    unsigned long long wait_ns) {
-  // once per instantiation; a function-local static is initialised thread-safely
-  // (the second log-likelihood pipeline launches from its own host thread)
   constexpr int smem = ST * kStageBytes + 1024;
-  static const bool attr = [] {
-    cudaFuncSetAttribute(tc_gemm_kernel<MODE, AL, BL, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return true;
-  }();
-  (void)attr;
+  allow_smem<tc_gemm_kernel<MODE, AL, BL, ST>>(smem);
   launch_chained(tc_gemm_kernel<MODE, AL, BL, ST>, n, kThreads, smem, st, t, A, B, C, wait_ns);
 }
 // Four stages while every tile has an SM to itself (a shorter wait per tile), two
