@@ -402,7 +402,11 @@ __global__ void __launch_bounds__(128) spmv_sep_kernel(QStencil q, const double*
 static dim3 spmv_grid(const QStencil& q, int nrhs, int* steps) {
   const int64_t tot = int64_t(q.Ns) * nrhs;
   *steps = q.T;
-  while (*steps > 1 && tot * ((q.T + *steps - 1) / *steps) < 152 * 1536) *steps = (*steps + 1) / 2;
+  while (*steps > 1 && tot * ((q.T + *steps - 1) / *steps) < 152 * 1536) {
+    const int half = (*steps + 1) / 2;
+    if ((q.T + half - 1) / half > 65535) break;  // grid limit, reached by a few cells and very many steps
+    *steps = half;
+  }
   return dim3(nblk(tot, 128), (q.T + *steps - 1) / *steps);
 }
 void launch_spmv(const QStencil& q, const double* obs, double tau, const double* x, double* y, int nrhs,
