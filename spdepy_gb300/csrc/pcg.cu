@@ -676,8 +676,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // ap = A p in FP32 for the columns [lead + V y, + V), one thread per node and V
 // columns, and the warp groups' sums of p . ap into part[col gpad + group].  Node
-// offsets fit in 32 bits (27 n does, checked by the caller), and so do those inside a group of
-// 25 coefficients; where a group starts (up to 68 Ns) they may not, with one or two time steps.
+// offsets fit in 32 bits (27 n < 2^31, checked by the caller), coefficient offsets in 32 bits
+// without sign: below 50 Ns with one time step, below 69 Ns with two or more.
 // Bound: L1 / L2 loads (43 coefficients and 43 V vector values per node).  Four
 // columns per thread share the coefficients' loads and the index arithmetic.
 // Measured at 200 x 200 x 24: 16 columns 155 us (417 with one column per thread), at
@@ -713,30 +713,28 @@ __global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, f
       float acc[V];
       // a neighbour outside the grid counts with coefficient zero (on the node's own
       // value): no branches, so that the loads of a node overlap
-      auto add = [&](const float* qs, int s, int dx, int dy, int dt, bool in) {
-        const float q = in ? qs[s * Ns] : 0.f;
+      auto add = [&](int slot, int dx, int dy, int dt, bool in) {
+        const float q = in ? cc[unsigned(slot) * unsigned(Ns)] : 0.f;
         const Cols<V> xv = xt[in ? dt * Ns + dy * Mx + dx : 0];
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v] = fmaf(q, xv.v[v], acc[v]);
       };
       auto block25 = [&](int sb, int dt) {
         const bool vd = (vt >> (dt + 1)) & 1u;
-        const float* qs = cc + int64_t(sb) * Ns;
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v] = 0.f;
 #pragma unroll
         for (int s = 0; s < 25; ++s) {
           const int dx = s % 5 - 2, dy = s / 5 - 2;
-          add(qs, s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
+          add(sb + s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
         }
       };
       auto block9 = [&](int s0, int dt) {
         const bool vd = (vt >> (dt + 1)) & 1u;
-        const float* qs = cc + int64_t(s0) * Ns;
 #pragma unroll
         for (int s = 0; s < 9; ++s) {
           const int dx = s % 3 - 1, dy = s / 3 - 1;
-          add(qs, s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
+          add(s0 + s, dx, dy, dt, vd && ((vx >> (dx + 2)) & (vy >> (dy + 2)) & 1u));
         }
       };
       if (SEP) {
@@ -755,7 +753,7 @@ __global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, f
         for (int v = 0; v < V; ++v) acc[v] = s[v];
       } else {
         block25(t == 0 && T > 1 ? 0 : 25, 0);
-        add(cc + int64_t(68) * Ns, 0, 0, 0, 0, T > 1 && t < T - 1);
+        add(68, 0, 0, 0, T > 1 && t < T - 1);
         if (T > 1) {
           block9(50, 1);
           block9(59, -1);
@@ -1131,8 +1129,8 @@ __global__ void near_rows_kernel(int Mx, int Ny, int T, GWeights gw, float* __re
 // row is one base, stride and neighbour shift per time offset, so that observed
 // nodes, their neighbours and the boundary differ from the interior by a
 // predicate per offset and not by another path (a warp holds several kinds).
-// Offsets inside a class of rows fit in 32 bits (27 n does, checked by the caller); a class starts at
-// up to 81 Ns, which may not.  Bound: L1 / L2 loads.
+// Offsets of the classes' rows fit in 32 bits (27 n < 2^31, checked by the caller; 54 Ns needs two
+// time steps), the observed rows' start, 81 Ns, does not.  Bound: L1 / L2 loads.
 // Measured at 200 x 200 x 24 with 1 % observed, 16 columns: G 101 us (413 with one
 // column per thread), G^T 150 us (1,026: near an observed node, which is in nearly
 // every warp, each of 27 weights was looked up through bitmask and rank).
@@ -1182,7 +1180,7 @@ __global__ void __launch_bounds__(256, V == 1 ? 4 : 3) g32_kernel(int Mx, int Ny
           shift_y = TRANS ? Mx : 0;
           shift_x = TRANS ? 1 : 0;
 #pragma unroll
-          for (int d = 0; d < 3; ++d) row[d] = gw.w + int64_t(time_class(TRANS ? t - (d - 1) : t, T) * kOff) * Ns + c;
+          for (int d = 0; d < 3; ++d) row[d] = gw.w + time_class(TRANS ? t - (d - 1) : t, T) * kOff * Ns + c;
         }
       }
       float acc[V];
