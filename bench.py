@@ -404,6 +404,40 @@ def run_reference(args, rank, world):
     print(json.dumps(line))
 
 
+def fp64_leg(w, steps):
+    """Seconds, objective and gradient of one evaluation with the FP64 plan."""
+    import torch
+    from spdepy_gb300.workloads import build_model
+    mod = build_model(w, "fp64")
+    mod.initFit(w.y, idx=w.idx)
+    mod._ensure_model()
+    mod.plan.set_obs(w.grid.obs_nodes(w.idx))
+    canon = mod.canonical(w.par)
+    y = torch.as_tensor(w.y).cuda()
+    mod.plan.loglike(canon, y, 0)  # warm-up: both factorisations and the solve, no inversion
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    for _ in range(steps):
+        f, jac = mod.plan.loglike(canon, y, 1)
+    torch.cuda.synchronize()
+    return (time.perf_counter() - t0) / steps, f, jac
+
+
+def fp64_plain_leg(args, w):
+    """The FP64 plan with FP64 FMAs on the CUDA cores throughout, the plain side of the
+    metric: SPDE_TC=0 in a process of its own (the switch is read once per process)."""
+    import tempfile
+    with tempfile.TemporaryDirectory() as d:
+        y = os.path.join(d, "y.npy")
+        np.save(y, w.y)
+        cmd = [sys.executable, os.path.abspath(__file__), "--size", args.size, "--fp64-steps", str(args.fp64_steps),
+               "--fp64-plain", y]
+        r = subprocess.run(cmd, capture_output=True, text=True, env=dict(os.environ, SPDE_TC="0"))
+    if r.returncode != 0:
+        return {"failed": (r.stderr.strip().splitlines() or ["no message"])[-1][:300]}
+    return json.loads(r.stdout.strip().splitlines()[-1])
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -413,7 +447,9 @@ def main():
     ap.add_argument("--precision", default="mixed")
     ap.add_argument("--size", default="200,200,24")
     ap.add_argument("--fp64-steps", type=int, default=1,
-                    help="timed evaluations of the plain FP64 plan (the metric's denominator); 0 skips it")
+                    help="timed evaluations of the FP64 plan, as it runs and with plain FP64 products "
+                         "(the metric's denominator); 0 skips both")
+    ap.add_argument("--fp64-plain", metavar="Y.npy", help="run only the FP64 plan on these observations and print its time")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-pcg", action="store_true")
     ap.add_argument("--pcg-only", action="store_true", help="run only the learned-PCG leg and print its record")
@@ -436,6 +472,13 @@ def main():
         b.build()
         size = tuple(int(v) for v in args.pcg_size.split(","))
         print(json.dumps({"learned_pcg": learned_pcg_leg(args.pcg_train_steps, size)}))
+        return
+    if args.fp64_plain:
+        from spdepy_gb300.workloads import nonstationary_advection_diffusion
+        w = nonstationary_advection_diffusion(*(int(v) for v in args.size.split(",")))
+        w.y = np.load(args.fp64_plain)
+        t64, f64, _ = fp64_leg(w, args.fp64_steps)
+        print(json.dumps({"evals_per_s": 1.0 / t64, "s_per_eval": t64, "steps": args.fp64_steps, "f": f64}))
         return
     dist = None
     if world > 1:
@@ -527,34 +570,27 @@ def main():
     samples_per_s = 256.0 / (time.perf_counter() - s0)
 
     nobs_total = float(w.idx.size)  # m r, the objective's normalisation (r = 1)
-    fp64 = None
+    fp64 = fp64_plain = None
     dgemm = _dgemm_tflops(torch)
     if args.fp64_steps > 0:
-        # the plain FP64 plan on the same workload: the metric's denominator
-        m64 = build_model(w, "fp64")
-        m64.initFit(w.y, idx=w.idx)
-        m64._ensure_model()
-        m64.plan.set_obs(w.grid.obs_nodes(w.idx))
-        c64 = m64.canonical(w.par)
-        m64.plan.loglike(c64, y_dev, 0)  # warm-up: both factorisations and the solve, no inversion
-        torch.cuda.synchronize()
-        t0 = time.perf_counter()
-        for _ in range(args.fp64_steps):
-            f64, j64 = m64.plan.loglike(c64, y_dev, 1)
-        torch.cuda.synchronize()
-        t64 = (time.perf_counter() - t0) / args.fp64_steps
         dense_flops = 2.0 * (info.factor_flops + info.selinv_flops)
+        t64, f64, j64 = fp64_leg(w, args.fp64_steps)
         fp64 = {"evals_per_s": 1.0 / t64, "s_per_eval": t64, "steps": args.fp64_steps, "f": f64,
                 "mixed_speedup": evals_per_s * t64,
                 "rel_dlogL_mixed_vs_fp64": abs(f - f64) / abs(f64),
                 "abs_dlogL_mixed_vs_fp64": abs(f - f64) * nobs_total,
                 "rel_dgrad_mixed_vs_fp64": float(np.abs(jac - j64).max() / np.abs(j64).max()),
                 "dense_tflops": dense_flops / t64 / 1e12, "dgemm_cublas_tflops": dgemm,
-                "frac_of_dgemm": (dense_flops / t64 / 1e12) / dgemm if dgemm else None,
-                "note": "one FP64-plan evaluation after a warm-up without inversion; abs_dlogL is |f - f64| "
+                "note": "the FP64 plan as it runs, its products from base-256 digits on the tensor cores; one "
+                        "evaluation after a warm-up without inversion; abs_dlogL is |f - f64| "
                         "times m r, the difference in the log-likelihood itself; dense_tflops counts the two "
                         "factorisations' and two inversions' algorithmic flops"}
-        del m64
+        if rank == 0 and world == 1:
+            fp64_plain = fp64_plain_leg(args, w)
+            if "s_per_eval" in fp64_plain:
+                t = fp64_plain["s_per_eval"]
+                fp64_plain.update({"mixed_speedup": evals_per_s * t, "dense_tflops": dense_flops / t / 1e12,
+                                   "frac_of_dgemm": (dense_flops / t / 1e12) / dgemm if dgemm else None})
 
     peaks, peak_src = _peaks()
     # dominant kernel: the tensor-core tiled product (profile class 9), timed
@@ -610,7 +646,7 @@ def main():
         "algorithmic": {"factor_tflop": info.factor_flops / 1e12, "selinv_tflop": info.selinv_flops / 1e12,
                         "nnz_L": info.nnz_l},
         "gemm_sites": sites,
-        "objective": f, "clocks": clk, "cpu_baseline": cb, "fp64_plain": fp64, "learned_pcg": pcg, "lbfgs_fit": fit, "stationary_100x100x24": c2,
+        "objective": f, "clocks": clk, "cpu_baseline": cb, "fp64_plan": fp64, "fp64_plain": fp64_plain, "learned_pcg": pcg, "lbfgs_fit": fit, "stationary_100x100x24": c2,
     }
     print(json.dumps(line))
 
