@@ -1375,8 +1375,8 @@ struct Exec {
     };
     for (const Op& o : s.ops) {
       if (depth_log && (dmarks.empty() || dmarks.back().first != o.depth)) dmark(o.depth);
-      const bool on_tc = o.kind == OP_EMU || (o.kind == OP_GEMM && sizeof(T) == sizeof(float) &&
-                                              ((o.tc == kPathTensor && tc_gemm_enabled()) || o.tc == kPathPair));
+      const bool on_tc = o.kind == OP_GEMM && sizeof(T) == sizeof(float) &&
+                         ((o.tc == kPathTensor && tc_gemm_enabled()) || o.tc == kPathPair);
       const bool timed = p->profile && o.kind != OP_MEMSET && (on_tc || !p->profile_tc_only);
       if (timed) prof_begin(p, st);
       switch (o.kind) {

@@ -20,7 +20,8 @@ enum OpKind {
   OP_FWD_CHAIN, OP_BWD_CHAIN,
   OP_EMU  // FP64 products on the tensor cores (split, then product)
 };
-// profile class of a tiled product that ran on the tensor cores (the others count as OP_GEMM)
+// profile class of an FP32 tiled product that ran on the tensor cores (the others, the FP64
+// plan's digit products among them, count as OP_GEMM)
 constexpr int kProfTensorCore = 9;
 constexpr int kProfClasses = 10;
 

@@ -33,7 +33,7 @@ def test_fp64_products():
     z0 = plan.selinv().cpu().numpy()
     prof = np.zeros(10, dtype=np.int64)
     L.spde_plan_read_profile(plan.h, None, None, None, 1)
-    nat.check(L.spde_plan_set_profiling(plan.h, 2), plan.h)
+    nat.check(L.spde_plan_set_profiling(plan.h, 1), plan.h)
     ld = ctypes.c_double()
     try:
         with Limit(plan):
@@ -41,7 +41,7 @@ def test_fp64_products():
     finally:
         L.spde_plan_read_profile(plan.h, None, None, prof.ctypes.data, 1)
         L.spde_plan_set_profiling(plan.h, 0)
-    assert prof[9] > 0  # tensor-core products ran (and gave up)
+    assert prof[3] > 0  # products ran (and gave up)
     assert rc == 2 and b"timed out" in L.spde_last_error(plan.h)
     with pytest.raises(nat.SpdeError):
         plan.solve(torch.zeros(w.grid.n, dtype=torch.float64))  # no valid factor
