@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(256) gemm64_kernel(const GemmTask* __restrict_
 // layout, read two k values at a time) or, per k, rows side by side (column layout);
 // a warp computes 32 x 64 entries, warps outside the task's rows or columns skip the
 // arithmetic.  Every entry adds its products in the order of k.  Same aliasing rule
-// as above.  Bound: the FP32 pipe for many tiles, latency for few.
+// as above.  Bound: the FP32 pipe for many tiles, latency for few.  Two CTAs per SM leave
+// 128 registers, of which the forms with A in rows spill 20 to 72 bytes.
 constexpr int kSgBk = 32, kSgRow = kSgBk + 4, kSgCol = 128 + 4;  // row strides: 16-byte rows, 4 banks apart
 constexpr int kSgOp = 128 * kSgRow;                              // floats of one operand's buffer (either layout)
 static_assert(kSgBk * kSgCol <= kSgOp && 128 * kSgCol <= 4 * kSgOp, "column layout and the output tile fit");

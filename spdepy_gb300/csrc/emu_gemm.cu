@@ -33,7 +33,8 @@
 // per digit, so that a stage is filled by a few bulk copies.  A CTA computes a
 // 128 x 64 tile: the eight accumulators take all 512 TMEM columns, and a stage (eight
 // digits of 128 x 32 and 64 x 32) 96 KB, two of which fit in shared memory.
-// Bound: the tensor core's shared-memory reads (128 + 64 rows per 128 x 64 product).
+// Bound: the tensor core's shared-memory reads (128 + 64 rows per 128 x 64 product); the
+// epilogue's 64 bits x 32 sums leave 24 bytes of spills (96 registers, 576 threads).
 #include <cuda_runtime.h>
 #include <cstdint>
 

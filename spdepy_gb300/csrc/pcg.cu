@@ -790,7 +790,8 @@ __global__ void __launch_bounds__(256, 4) spmv32_kernel(int Mx, int Ny, int T, f
 // group_dot_kernel forms them.
 // Bound: latency, the loads in flight of 24 warps per SM (three CTAs; at two 175 us
 // without spills, at four 152); the values two steps ahead are fetched to L2
-// (130 us without).  Measured at 400 x 400 x 48: 124 us, spmv32_kernel 177.
+// (130 us without).  At three CTAs its 80 registers spill 80 to 92 bytes (none separable).
+// Measured at 400 x 400 x 48: 124 us, spmv32_kernel 177.
 // Warps take runs of 32 cells as in Walk, with P runs per time step (the last one ragged).
 struct CellWalk {
   int R, P, bx, steps;  // runs per grid row and per time step, CTAs per time step, time steps per CTA
@@ -968,6 +969,10 @@ __device__ __forceinline__ float diag32(const float* __restrict__ cf, int Ns, in
 // r . r into partB[col G + b].
 // The sums are those of kElemBlocks blocks per column; the launch leaves out the blocks
 // past the last node (G = gridDim.x of them run).
+// Bound: memory (32 bytes per node and column with Jacobi and observations: x, r, p, Ap
+// and the observation term read, x, r and z written, less z without a preconditioner) and, for one
+// column, registers: at eight CTAs per SM its 32 spill 600 bytes of stores and 720 of loads a
+// thread (60 us at 400 x 400 x 48, whose bytes need 36).
 constexpr int kElemBlocks = 1216;  // 8 per SM
 template <int V>
 __global__ void __launch_bounds__(256, V == 1 ? 8 : 4) update32_kernel(int Ns, int T, int sep, float qe, float qm, int mode, int lead,

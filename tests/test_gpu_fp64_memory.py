@@ -33,8 +33,10 @@ def test_same_bits_with_little_memory():
     gc.collect()
     torch.cuda.empty_cache()
     hold = torch.empty(int(torch.cuda.mem_get_info()[0] - taken - (64 << 20)), dtype=torch.uint8, device="cuda")
-    f2, jac2, _, mod = _evaluate()
-    del hold, mod
-    gc.collect()
-    torch.cuda.empty_cache()
+    try:
+        f2, jac2, _, _ = _evaluate()
+    finally:
+        del hold
+        gc.collect()
+        torch.cuda.empty_cache()
     assert f2 == f and np.array_equal(jac2, jac)

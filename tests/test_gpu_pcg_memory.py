@@ -39,10 +39,13 @@ def test_same_solution_with_little_memory():
     mod, solve = _solver(M, N, T)
     # 26 floats a node and 69 a cell for the solve and its results, a third of it to spare; the rows take 27 a node
     keep = int(4 / 3 * 4 * (6 * n + n + 69 * M * N) + 4 * 8 * n)
-    hold = torch.empty(torch.cuda.mem_get_info()[0] - keep, dtype=torch.uint8, device="cuda")
     assert keep < 4 * 27 * n + 4 * 7 * n
-    x2, it2, _ = solve()
-    assert it2 == it and torch.equal(x2.cpu(), x)
-    del hold, mod, solve
-    gc.collect()
-    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - keep, dtype=torch.uint8, device="cuda")
+    try:
+        x2, it2, _ = solve()
+        x2 = x2.cpu()
+    finally:
+        del hold, mod, solve
+        gc.collect()
+        torch.cuda.empty_cache()
+    assert it2 == it and torch.equal(x2, x)
