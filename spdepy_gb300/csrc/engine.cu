@@ -41,7 +41,7 @@ constexpr int kPairMinK = 256;
 // per k value (the FP64 pipe), a tensor-core tile a fixed 10 us with its share of the
 // split and 2.3 us per 32 values.  Measured with the limit at 32 (all sizes), 16 and
 // (8, k 4): 17.5, 17.0 and 16.6 ms per FP64 evaluation at 30 x 30 x 24, 55.8, 51.1
-// and 51.0 ms at 48 x 48 x 24 (the leaf fronts' narrow products).
+// and 51.0 ms at 48 x 48 x 24 (the leaf fronts' narrow products; all with seven digits).
 constexpr int kEmuMin = 8, kEmuMinK = 4;
 enum { KT_NONE = 0, KT_A_UPPER, KT_B_LOWER, KT_BOTH_UPPER };
 constexpr int kPanel = 512;   // panel width of the two-level blocked factorisation
