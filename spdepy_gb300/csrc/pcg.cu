@@ -1393,6 +1393,12 @@ __global__ void __launch_bounds__(256) scal32_kernel(const float* __restrict__ g
   const int nblocks = groupsA ? (ngroups + 7) / 8 : na;
   const float4* ga = reinterpret_cast<const float4*>(groupsA + int64_t(col) * gpad);  // zero past the last group
   double s1 = 0.0, s2 = 0.0;
+  // every CTA reads B's sums and the column's state (the last one's count), so that they do not
+  // wait for the arrivals
+  const bool over = mode != 2 && done[col];
+  const double rz0 = mode != 2 ? rz[col] : 0.0;
+  if (mode != 0)
+    for (int i = tid; i < nb; i += 256) s2 += partB[int64_t(col) * nb + i];
   for (int j0 = 0; int(blockIdx.x) * W + 256 * j0 < nblocks; j0 += Q) {
     const int b = first + 256 * (j0 + lane);
     double s = 0.0;
@@ -1424,8 +1430,6 @@ __global__ void __launch_bounds__(256) scal32_kernel(const float* __restrict__ g
     s1 = __ldcg(chains + int64_t(col) * 256 + tid);
     if (tid == 0) arrived[col] = 0u;
   }
-  if (mode != 0)
-    for (int i = tid; i < nb; i += 256) s2 += partB[int64_t(col) * nb + i];
   sh[0][tid] = s1;
   sh[1][tid] = s2;
   __syncthreads();
@@ -1440,9 +1444,9 @@ __global__ void __launch_bounds__(256) scal32_kernel(const float* __restrict__ g
   const double a = sh[0][0], b = sh[1][0];
   if (mode == 0) {
     pap[col] = a;
-    alpha[col] = (!done[col] && a > 0.0) ? float(rz[col] / a) : 0.f;
+    alpha[col] = (!over && a > 0.0) ? float(rz0 / a) : 0.f;
   } else if (mode == 1) {
-    beta[col] = (!done[col] && rz[col] != 0.0) ? float(a / rz[col]) : 0.f;
+    beta[col] = (!over && rz0 != 0.0) ? float(a / rz0) : 0.f;
     rz[col] = a;
     rr[col] = b;
   } else {
@@ -1786,10 +1790,12 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   // r . z: block sums of the update (none, Jacobi) or of IC(0)'s dot product, else G^T's group sums
   const int na = mode == 2 ? nsp : nel;
   const float* gz = mode == 2 && kind != 4 ? gsum : nullptr;
-  // CTAs per column of the scalar kernel: one per two blocks of each chain, up to 64
+  // CTAs per column of the scalar kernel: one per block of each chain, up to 64.  Measured with Jacobi,
+  // one column, at one CTA per 2 / 1 / 0.5 blocks: 130 x 120 x 16 3,881 / 3,604 / 3,606 us a solve,
+  // 200 x 200 x 16 4,648 / 4,506 / 4,573, 400 x 400 x 48 25.4 / 25.4 / 25.4 ms.
   auto scalars = [&](const float* groups, int na_, int nb_, int what) {
     int Q = 1;
-    while (Q < 64 && (groups ? nsp : na_) > 512 * Q) Q *= 2;
+    while (Q < 64 && (groups ? nsp : na_) > 256 * Q) Q *= 2;
     scal32_kernel<<<dim3(Q, nrhs), 256, 0, st>>>(groups, ngroups, gpad, partA, na_, partB, nb_, what, done, chains,
                                                  arrived, rz, rr, pap, alpha, beta);
   };
