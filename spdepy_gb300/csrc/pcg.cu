@@ -1628,6 +1628,19 @@ int pc_weights_compact(Plan* p, int with_obs, double tau, const float* prm, floa
 constexpr double kReplaceDrop = 0.1;
 constexpr int kReplaceEvery = 64;
 
+// Whether a solve's columns go in groups of 4, 2 and 1 or each by itself (a column's bits are the
+// same).  Every width is a launch of its own in each step, and widths follow one another: with two
+// or three of them a small solve is faster by single columns, in one launch.  Measured (Jacobi,
+// groups / single columns, us a solve): 3 columns at 40 x 30 x 8 3,754 / 2,448, at 200 x 200 x 24
+// 11,155 / 10,381; 6 at 90 x 70 x 12 4,663 / 3,913, at 160 x 150 x 16 7,943 / 8,332; 7 at 110 x 100 x 16
+// 8,285 / 6,644; 17 at 90 x 70 x 12 5,940 / 6,163.
+bool columns_grouped(int64_t n, int nrhs) {
+  const int widths = (nrhs >= 4) + ((nrhs & 2) != 0) + (nrhs & 1);
+  if (widths == 1) return true;
+  if (nrhs == 3) return false;
+  return n * nrhs > int64_t(1) << (widths == 2 ? 19 : 21);
+}
+
 int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const double* b, double* x, int nrhs,
               double tol, int maxit, int check_every, int* iters, double* relres) {
   const int64_t n = p->sym.n, len = n * nrhs;
@@ -1639,7 +1652,7 @@ int pcg_solve(Plan* p, int with_obs, double tau, int kind, const float* w, const
   const int ngroups = nblk(n, 32), gpad = 8 * nsp;
   const int nel = std::min(int(kElemBlocks), nsp);  // elementwise blocks with nodes
   const int na_max = std::max(nsp, int(kElemBlocks));
-  const int packed = kind == 4 ? 0 : 1;
+  const int packed = kind != 4 && columns_grouped(n, nrhs) ? 1 : 0;
   // FP64: true residual (row-major), block partials, per-column scalars
   const size_t need64 = size_t(len) + size_t(nrhs) * (na_max + kElemBlocks) + size_t(kDotBlocks) * nrhs +
                         size_t(8 * nrhs) + size_t(nrhs) + size_t(257) * nrhs;
