@@ -1563,7 +1563,7 @@ int jacobi_smooth(Plan* p, int with_obs, double tau, double omega, int sweeps, d
   double *az = base, *part = az + len, *ss = part + size_t(kDotBlocks) * nrhs, *wd = ss + nrhs;
   const QStencil q = p->qstencil();
   const double* obs = with_obs ? p->d_obs_cnt : nullptr;
-  if (q.sep) {
+  if (q.sep || sweeps == 1) {  // a single sweep: one launch fewer than with weights and a copy back
     for (int it = 0; it < sweeps; ++it) {
       launch_spmv(q, obs, tau, z, az, nrhs, p->stream);
       jacobi_sweep_kernel<<<nblk(len), 256, 0, p->stream>>>(q, obs, tau, omega, az, z, nrhs);
